@@ -223,9 +223,9 @@ __global__ void k_emit(int N, Nodes t, int node_off, int slot_off, DNode* __rest
     bh = th;
   }
   DNode n;
-  n.a = make_float4(al.x, al.y, al.z, ah.x);
-  n.b = make_float4(ah.y, ah.z, bl.x, bl.y);
-  n.c = make_float4(bl.z, bh.x, bh.y, bh.z);
+  n.a = make_float4(al.x, bl.x, ah.x, bh.x);
+  n.b = make_float4(al.y, bl.y, ah.y, bh.y);
+  n.c = make_float4(al.z, bl.z, ah.z, bh.z);
   const bool la = t.leaf[a], lb = t.leaf[b];
   const int aref = la ? slot_off + t.off[a] : node_off + (a - N), bref = lb ? slot_off + t.off[b] : node_off + (b - N);
   const unsigned int acnt = la ? (unsigned int)t.cnt[a] : 0u, bcnt = lb ? (unsigned int)t.cnt[b] : 0u;
@@ -276,7 +276,7 @@ tr_status upload_device_built(tr_ctx* ctx) {
       std::memcpy(&fneg, &neg, 4);
       src[3 * p] = float4{A.x, A.y, A.z, fid};
       src[3 * p + 1] = float4{AB.x, AB.y, AB.z, fneg};
-      src[3 * p + 2] = float4{AC.x, AC.y, AC.z, 0.0f};
+      src[3 * p + 2] = float4{AC.x, AC.y, AC.z, tri_margin(AB, AC)};
     } else {
       int idv = (int)p, sv = pr.shape;
       float fid, fs;
@@ -465,6 +465,9 @@ tr_status upload_device_built(tr_ctx* ctx) {
   sc.nodes4 = nullptr;
   sc.treelet = nullptr;  // no host copy of the device-built tree to stage from
   sc.treelet_n = 0;
+  sc.box_order = 1;  // unions of the primitive boxes keep their order
+  for (size_t i = 0; i < hs.blo.size(); ++i)
+    if (!(hs.blo[i] <= hs.bhi[i])) sc.box_order = 0;
   sc.slot_leaf = nullptr;  // nor the leaf of every slot: no occluder cache
   hs.dnodes.clear();
   hs.root0 = -1;

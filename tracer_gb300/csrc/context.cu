@@ -57,8 +57,8 @@ struct Child4 {
 
 void node_children(const DNode& n, Child4& l, Child4& r) {
   const uint32_t cc = (uint32_t)n.d.z;
-  l = Child4{{n.a.x, n.a.y, n.a.z}, {n.a.w, n.b.x, n.b.y}, n.d.x, (int)(cc & 0xffffu)};
-  r = Child4{{n.b.z, n.b.w, n.c.x}, {n.c.y, n.c.z, n.c.w}, n.d.y, (int)(cc >> 16)};
+  l = Child4{{n.a.x, n.b.x, n.c.x}, {n.a.z, n.b.z, n.c.z}, n.d.x, (int)(cc & 0xffffu)};
+  r = Child4{{n.a.y, n.b.y, n.c.y}, {n.a.w, n.b.w, n.c.w}, n.d.y, (int)(cc >> 16)};
 }
 
 float half_area(const Child4& c) {
@@ -140,9 +140,10 @@ tr_status upload_device_tables(tr_ctx* ctx) {
   }
   for (uint32_t p : hs.order)
     if (p >= hs.prims.size()) return set_err(ctx, TR_ERR_ARG, "bvh primitive order entry out of range");
-  int maxd = 0;
+  int maxd = 0, box_order = 1;
   for (size_t i = 0; i < nn; ++i) {
     const tr_bvh_node32& n = hs.nodes[i];
+    for (int c = 0; c < 3; ++c) box_order &= n.lo[c] <= n.hi[c];
     if (n.count == 0) {
       depth[i + 1] = std::max(depth[i + 1], depth[i] + 1);
       depth[n.offset] = std::max(depth[n.offset], depth[i] + 1);
@@ -162,9 +163,9 @@ tr_status upload_device_tables(tr_ctx* ctx) {
     const tr_bvh_node32& L = hs.nodes[i + 1];
     const tr_bvh_node32& R = hs.nodes[n.offset];
     DNode& d = dn[dix[i]];
-    d.a = float4{L.lo[0], L.lo[1], L.lo[2], L.hi[0]};
-    d.b = float4{L.hi[1], L.hi[2], R.lo[0], R.lo[1]};
-    d.c = float4{R.lo[2], R.hi[0], R.hi[1], R.hi[2]};
+    d.a = float4{L.lo[0], R.lo[0], L.hi[0], R.hi[0]};
+    d.b = float4{L.lo[1], R.lo[1], L.hi[1], R.hi[1]};
+    d.c = float4{L.lo[2], R.lo[2], L.hi[2], R.hi[2]};
     const int lref = L.count > 0 ? L.offset : dix[i + 1];
     const int rref = R.count > 0 ? R.offset : dix[n.offset];
     d.d = int4{lref, rref, (int)((uint32_t)L.count | ((uint32_t)R.count << 16)), (int)n.axis};
@@ -177,7 +178,7 @@ tr_status upload_device_tables(tr_ctx* ctx) {
       const f3 A = hs.A[p.shape], AB = hs.AB[p.shape], AC = hs.AC[p.shape];
       slots[3 * s] = float4{A.x, A.y, A.z, as_float((int)pid)};
       slots[3 * s + 1] = float4{AB.x, AB.y, AB.z, as_float(-1)};
-      slots[3 * s + 2] = float4{AC.x, AC.y, AC.z, 0.0f};
+      slots[3 * s + 2] = float4{AC.x, AC.y, AC.z, tri_margin(AB, AC)};
     } else {
       slots[3 * s] = float4{0.0f, 0.0f, 0.0f, as_float((int)pid)};
       slots[3 * s + 1] = float4{0.0f, 0.0f, 0.0f, as_float(p.shape)};
@@ -261,6 +262,7 @@ tr_status upload_device_tables(tr_ctx* ctx) {
   DScene& sc = ctx->dsc;
   sc.nodes = ctx->d_nodes.as<DNode>();
   sc.nodes4 = wide ? ctx->d_nodes4.as<DNode4>() : nullptr;
+  sc.box_order = box_order;
   sc.treelet = nullptr;
   sc.treelet_n = 0;
   sc.slots = ctx->d_slots.as<float4>();

@@ -10,8 +10,9 @@
 //  * DNode4: the same tree collapsed to four-wide nodes for any-hit rays,
 //    whose result does not depend on the visiting order.
 //  * Slots: primitives in BVH leaf order, three float4 (48 bytes) each.
-//    Triangle: (A, id) (B-A, -1) (C-A, 0) -- B-A and C-A are the float
-//    differences the reference computes on every test. Sphere: (0, id)
+//    Triangle: (A, id) (B-A, -1) (C-A, margin) -- B-A and C-A are the float
+//    differences the reference computes on every test, the margin is that of
+//    the quick rejection before it (tri_surely_missed). Sphere: (0, id)
 //    (0, sphere index) (0).
 //  * Per-primitive, per-triangle, per-sphere, per-material and per-light
 //    tables indexed by the scene description's ids, holding only values
@@ -45,9 +46,9 @@ constexpr int kTreeletMax = 1024;
 constexpr int kTreeletRef = 1 << 25;
 
 struct alignas(16) DNode {
-  float4 a;  // L.lo.x L.lo.y L.lo.z L.hi.x
-  float4 b;  // L.hi.y L.hi.z R.lo.x R.lo.y
-  float4 c;  // R.lo.z R.hi.x R.hi.y R.hi.z
+  float4 a;  // L.lo.x R.lo.x L.hi.x R.hi.x: an axis's planes side by side,
+  float4 b;  // L.lo.y R.lo.y L.hi.y R.hi.y  for both boxes in one packed
+  float4 c;  // L.lo.z R.lo.z L.hi.z R.hi.z  operation (pair_boxes)
   int4 d;    // L.ref, R.ref, L.count | R.count << 16, axis. count > 0: ref is a
              // leaf's first slot; count == 0: ref is the child's DNode index.
 };
@@ -232,6 +233,7 @@ struct DScene {
   // The materials' factory arguments and maps, by material index (only for
   // sets with image maps; null otherwise)
   const tr_material* msrc;
+  int box_order;  // every box has lo <= hi (pair_boxes' condition; 0: some uploaded box does not)
   // Binary any-hit walks: the child entered first when both pass
   // (tr_tuning.any_hit_order: 0 near, 1 far, 2 larger box surface).
   int any_order;
