@@ -9,10 +9,10 @@
 //     sums, one Newton step on rsqrt),
 //  2. rounds that to float and checks, with a rigorous error bound that also
 //     covers the reference's intermediate double roundings (at most a few
-//     2^-53 relative), that the true value lies strictly inside the rounding
-//     interval of that float -- then the reference's float(double(...)) is
-//     the same float,
-//  3. otherwise evaluates the reference's double expression directly.
+//     2^-53 relative), that every real within the bound rounds to that float
+//     (ziv) -- then the reference's float(double(...)) is the same float,
+//  3. otherwise evaluates the reference's double expression directly, out of
+//     line: its code is long (double divide and square root) and rarely runs.
 // Step 3 is needed only when the value lies within ~2^-40 relative of a
 // float rounding boundary or outside a safe exponent range (rare), so
 // results equal the reference bit for bit while the common case uses the
@@ -65,16 +65,27 @@ TR_HD bool in_range(float x) {
   return e >= 67u && e <= 187u;
 }
 
-// True when every real within err of (y + r) rounds to y, where y is a
-// normal float and r the exact residual of the approximation (|r| at most
-// half a spacing). Both neighbouring half-spacings are checked.
-TR_HD bool rounds_to(float y, float r, float err) {
-  const uint32_t b = fbits(y) & 0x7fffffffu;
-  if (b < 0x01000000u || b >= 0x7e800000u) return false;  // tiny, huge, inf, nan
-  const float ulp = bitsf(b & 0x7f800000u) * 1.1920928955078125e-07f;  // 2^(e-23)
-  float half = 0.5f * ulp;
-  if ((b & 0x007fffffu) == 0u) half *= 0.5f;  // power of two: smaller spacing below
-  return fabsf(r) + err < half;
+// The value a + b rounded to float, when every real within err of a + b
+// rounds the same way (Ziv's rounding test: rounding is monotone, so if the
+// two ends of the interval round alike, all of it does). a is a float near
+// the result, b the small rest; the ends' own sums b +- err are rounded too,
+// by at most 2^-24 (|b| + err), which the callers' err includes. Five
+// operations instead of the seventeen of comparing the rest with half a
+// spacing taken from the result's exponent.
+TR_HD bool ziv(float a, float b, float err, float& y) {
+  y = a + (b + err);
+  return y == a + (b - err);
+}
+
+// 2 |x| as an integer, less one: zero is the largest value, so the smallest
+// of several tells whether each is zero or at least as large as a bound.
+TR_HD uint32_t zero_or_at_least(float x) { return 2u * fbits(x) - 1u; }
+TR_HD uint32_t umin3(uint32_t a, uint32_t b, uint32_t c) {
+  const uint32_t m = a < b ? a : b;
+  return m < c ? m : c;
+}
+TR_HD float csign(float x, float s) {  // |x| with the sign of s
+  return bitsf((fbits(x) & 0x7fffffffu) | (fbits(s) & 0x80000000u));
 }
 
 // (s, e) with s = RN(a + b) and s + e = a + b exactly.
@@ -101,22 +112,22 @@ TR_HD_COLD float cross1_d(float a, float b, float c, float d) {
 }
 
 // float(double(a) * b - double(c) * d): one component of the reference's cross().
+// The exact difference is s + e + pl - ql; w is within
+// 2^-24 (|pl| + |ql|) + 2^-24 |w| <= 2^-46 (|p| + |q|) of its rest, the
+// reference's double rounding within 2^-53 of the result, ziv's sums within
+// 2^-47 (|p| + |q|): 1.6 x 2^-46 covers them. Below 2^-90 the error terms
+// could underflow; products there (zeros above all) take the double
+// expression unless both are exactly zero. (err > 0, so y is never zero.)
 TR_HD float cross1(float a, float b, float c, float d) {
   const float ph = a * b, qh = c * d;
-  const bool pz = (a == 0.0f) | (b == 0.0f), qz = (c == 0.0f) | (d == 0.0f);
-  if (pz | qz) {
-    if (pz & qz) return ph - qh;  // exact zeros, with the double result's sign
-    return pz ? -qh : ph;         // the other product, exactly rounded once
-  }
-  if (in_range(ph) & in_range(qh)) {
+  const float sum = fabsf(ph) + fabsf(qh);
+  if (sum >= 8.0779357e-28f && sum <= 1.2676506e+30f) {  // 2^-90, 2^100
     const float pl = ffma(a, b, -ph), ql = ffma(c, d, -qh);
-    float e;
+    float e, y;
     const float s = two_sum(ph, -qh, e);
-    const float w = e + (pl - ql);
-    float r;
-    const float y = two_sum(s, w, r);
-    const float err = 1.4210855e-14f * (fabsf(ph) + fabsf(qh)) + 8.8817842e-16f * fabsf(y);  // 2^-46, 2^-50
-    if (rounds_to(y, r, err)) return y;
+    if (ziv(s, e + (pl - ql), 2.28e-14f * sum, y)) return y;
+  } else if (((a == 0.0f) | (b == 0.0f)) & ((c == 0.0f) | (d == 0.0f)) & (sum == 0.0f)) {
+    return ph - qh;  // exact zeros, with the double result's sign
   }
   return cross1_d(a, b, c, d);
 }
@@ -126,43 +137,29 @@ TR_HD f3 cross_x(f3 a, f3 b) {
 }
 
 // The reference's normalize(v): float(x * (1.0 / sqrt(double(|v|^2_float)))).
-TR_HD f3 normalize_x(f3 v) {
+// r0 + c is 1/sqrt(L) within 2^-43, x (r0 + c) = ph + zl within 2^-42.8
+// (zl's rounding and the reference's double roundings included): 2^-41.
+TR_HD_MATH f3 normalize_x(f3 v) {
   const float L = len2f(v);
-  if (L >= 8.6736174e-19f && L <= 1.1529215e+18f) {  // [2^-60, 2^60]
+  // L in [2^-60, 2^60]; components zero or at least 2^-75 (the error terms do not underflow)
+  if (L >= 8.6736174e-19f && L <= 1.1529215e+18f &&
+      umin3(zero_or_at_least(v.x), zero_or_at_least(v.y), zero_or_at_least(v.z)) >= 2u * 0x1a000000u - 1u) {
     float r0, c;
     rsqrt_ff(L, r0, c);
-    float o[3];
-    const float in[3] = {v.x, v.y, v.z};
-    bool ok = true;
-    for (int k = 0; k < 3; ++k) {
-      const float x = in[k];
-      if (x == 0.0f) {
-        o[k] = x;  // +-0 * positive finite
-        continue;
-      }
-      if (!in_range(x)) {
-        ok = false;
-        break;
-      }
-      const float ph = x * r0;
-      const float pl = ffma(x, r0, -ph);
-      const float zl = pl + x * c;
-      float r;
-      const float y = two_sum(ph, zl, r);
-      if (!rounds_to(y, r, 9.094947e-13f * fabsf(y))) {  // 2^-40
-        ok = false;
-        break;
-      }
-      o[k] = y;
-    }
-    if (ok) return mk3(o[0], o[1], o[2]);
+    const float px = v.x * r0, py = v.y * r0, pz = v.z * r0;
+    const float zx = ffma(v.x, c, ffma(v.x, r0, -px)), zy = ffma(v.y, c, ffma(v.y, r0, -py)),
+                zz = ffma(v.z, c, ffma(v.z, r0, -pz));
+    float x, y, z;
+    const bool ox = ziv(px, zx, 4.5474735e-13f * px, x), oy = ziv(py, zy, 4.5474735e-13f * py, y),
+               oz = ziv(pz, zz, 4.5474735e-13f * pz, z);
+    if (ox & oy & oz) return mk3(csign(x, v.x), csign(y, v.y), csign(z, v.z));  // zeros keep their sign
   }
   return normalize_d(v);
 }
 
 // float(double(dot32(a, b)) / (sqrt(double(La)) * sqrt(double(Lb)))), the
 // reference's cos(w1, w2).
-TR_HD float cos_x(f3 a, f3 b) {
+TR_HD_MATH float cos_x(f3 a, f3 b) {
   const float d = dot(a, b);
   const float La = len2f(a), Lb = len2f(b);
   if (d == 0.0f && La > 0.0f && Lb > 0.0f && La <= 1e30f && Lb <= 1e30f) return d;
@@ -174,11 +171,10 @@ TR_HD float cos_x(f3 a, f3 b) {
     const float Rh = ra * rb;
     const float Rl = ffma(ra, rb, -Rh) + (ra * cb + rb * ca);
     const float ph = d * Rh;
-    if (in_range(ph)) {
-      const float zl = ffma(d, Rh, -ph) + d * Rl;
-      float r;
-      const float y = two_sum(ph, zl, r);
-      if (rounds_to(y, r, 1.8189894e-12f * fabsf(y))) return y;  // 2^-39
+    if (fabsf(ph) >= 8.6736174e-19f) {  // 2^-60
+      const float zl = ffma(d, Rl, ffma(d, Rh, -ph));
+      float y;
+      if (ziv(ph, zl, 1.8189894e-12f * ph, y)) return y;  // 2^-39
     }
   }
   return cosv_d(a, b);
@@ -203,11 +199,10 @@ TR_HD float dist_minus_eps(float L, bool& le_eps) {
     float e1;
     const float t = two_sum(sh, -kEps, e1);
     const float w = e1 + sl;
-    float r;
-    const float y = two_sum(t, w, r);
+    float y;
     // error: 2^-43 |sqrt L| from r, plus the reference's two double roundings
     const float err = 2.2737368e-13f * sh;  // 2^-42
-    if (rounds_to(y, r, err)) {
+    if (ziv(t, w, 1.25f * err, y)) {
       const float margin = 2.0f * err + 1.1920929e-07f * kEps;
       if (y > kEps + margin) {
         le_eps = false;
@@ -240,47 +235,26 @@ TR_HD float area_to_solid_pdf(float A, float d, float L) {
     const float y0 = A / qh;
     const float res = ffma(-y0, qh, A) - y0 * ql;
     const float corr = res / qh;
-    float r;
-    const float y = two_sum(y0, corr, r);
-    if (rounds_to(y, r, 1.8189894e-12f * fabsf(y))) return y;  // 2^-39
+    float y;
+    if (ziv(y0, corr, 1.8189894e-12f * y0, y)) return y;  // 2^-39
   }
   return area_to_solid_pdf_d(A, d, L);
 }
 
 // Vector3 / f for a float f (src/utility/geometry.hpp:429-433):
-// float(x * (1.0 / double(f))) per component.
-TR_HD f3 div_x(f3 v, float f) {
-  if (in_range(f)) {
+// float(x * (1.0 / double(f))) per component. i0 + i1 is 1/f within 2^-46.
+TR_HD_MATH f3 div_x(f3 v, float f) {
+  if (in_range(f) && fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fabsf(v.z)) <= 1.1529215e+18f &&  // 2^60
+      umin3(zero_or_at_least(v.x), zero_or_at_least(v.y), zero_or_at_least(v.z)) >= 2u * 0x2b800000u - 1u) {  // 2^-40
     const float i0 = 1.0f / f;
-    const float i1 = i0 * ffma(-i0, f, 1.0f);  // 1/f ~ i0 + i1
-    float o[3];
-    const float in[3] = {v.x, v.y, v.z};
-    bool ok = true;
-    for (int k = 0; k < 3; ++k) {
-      const float x = in[k];
-      if (x == 0.0f) {
-        o[k] = (f > 0.0f) ? x : -x;
-        continue;
-      }
-      if (!in_range(x)) {
-        ok = false;
-        break;
-      }
-      const float ph = x * i0;
-      if (!in_range(ph)) {
-        ok = false;
-        break;
-      }
-      const float zl = ffma(x, i0, -ph) + x * i1;
-      float r;
-      const float y = two_sum(ph, zl, r);
-      if (!rounds_to(y, r, 9.094947e-13f * fabsf(y))) {  // 2^-40
-        ok = false;
-        break;
-      }
-      o[k] = y;
-    }
-    if (ok) return mk3(o[0], o[1], o[2]);
+    const float i1 = i0 * ffma(-i0, f, 1.0f);
+    const float px = v.x * i0, py = v.y * i0, pz = v.z * i0;
+    const float zx = ffma(v.x, i1, ffma(v.x, i0, -px)), zy = ffma(v.y, i1, ffma(v.y, i0, -py)),
+                zz = ffma(v.z, i1, ffma(v.z, i0, -pz));
+    float x, y, z;
+    const bool ox = ziv(px, zx, 4.5474735e-13f * px, x), oy = ziv(py, zy, 4.5474735e-13f * py, y),
+               oz = ziv(pz, zz, 4.5474735e-13f * pz, z);  // 2^-41
+    if (ox & oy & oz) return mk3(csign(x, px), csign(y, py), csign(z, pz));
   }
   return divd(v, (double)f);
 }

@@ -25,6 +25,8 @@
 // Guided rendering and instrumented renders (stage times, visit counts) use
 // the wavefront.
 
+#define TRG_MATH_OUT_OF_LINE  // tr_math.cuh: this kernel holds every material's code
+
 #include <cuda_runtime.h>
 
 #include "mega.h"

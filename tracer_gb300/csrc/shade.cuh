@@ -406,9 +406,8 @@ __device__ __forceinline__ float disney_fd90(float L, float r) {
       float e;
       const float s0 = two_sum(0.5f, 2.0f * a, e);
       const float w = e + 2.0f * al;
-      float res;
-      const float y = two_sum(s0, w, res);
-      if (rounds_to(y, res, 5.6843419e-14f * (2.0f * fabsf(a) + 1.0f))) return y;  // 2^-44
+      float y;
+      if (ziv(s0, w, 7.2e-14f * (2.0f * fabsf(a) + 1.0f), y)) return y;  // 1.25 x 2^-44
     }
   }
   return disney_fd90_d(L, r);
@@ -429,10 +428,9 @@ __device__ __forceinline__ float disney_ss(float Fss, float S) {
     const float ql = e2 + pl;
     const float qh2 = q * 1.25f;
     const float ql2 = ffma(q, 1.25f, -qh2) + ql * 1.25f;
-    float res;
-    const float y = two_sum(qh2, ql2, res);
-    const float err = 2.2737368e-13f * (1.0f + fabsf(Fss) * (fabsf(i0) + 1.0f));  // 2^-42
-    if (rounds_to(y, res, err)) return y;
+    float y;
+    const float err = 2.6e-13f * (1.0f + fabsf(Fss) * (fabsf(i0) + 1.0f));  // 1.125 x 2^-42
+    if (ziv(qh2, ql2, err, y)) return y;
   }
   return disney_ss_d(Fss, S);
 }
