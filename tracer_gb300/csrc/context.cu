@@ -763,9 +763,9 @@ static tr_status build_host_scene(tr_ctx* ctx, const tr_scene_desc* d, HostScene
     ts.gy = g.y;
     ts.gz = g.z;
     const f3 nA = normalize(N[i0]), nB = normalize(N[i1]), nC = normalize(N[i2]);
-    ts.nA = nA;
-    ts.dn1 = nB - nA;
-    ts.dn2 = nC - nA;
+    ts.a = nA;
+    ts.b = nB - nA;
+    ts.c = nC - nA;
     ts.uvA[0] = uA[0];
     ts.uvA[1] = uA[1];
     ts.duv1[0] = m00;
@@ -773,11 +773,26 @@ static tr_status build_host_scene(tr_ctx* ctx, const tr_scene_desc* d, HostScene
     ts.duv2[0] = m10;
     ts.duv2[1] = m11;
     const float det = m00 * m11 - m01 * m10;
-    ts.det_nonzero = det ? 1 : 0;
+    ts.form = det ? TRI_SMOOTH_UV : TRI_SMOOTH;
     if (det) {
       const float inv_det = 1.0f / det;
-      ts.dndu0 = scale(ts.dn1, m11 * inv_det) - scale(ts.dn2, m01 * inv_det);
-      ts.dndv0 = scale(ts.dn1, m10 * inv_det) - scale(ts.dn2, m00 * inv_det);
+      ts.dndu0 = scale(ts.b, m11 * inv_det) - scale(ts.c, m01 * inv_det);
+      ts.dndv0 = scale(ts.b, m10 * inv_det) - scale(ts.c, m00 * inv_det);
+    }
+    // equal normals: the interpolated one is A's bit for bit (A + 0 alpha + 0
+    // beta; a -0 would become +0, so such a normal stays smooth), and
+    // triangle_isect's frame from it is the same at every hit
+    const bool minus0 = fbits(nA.x) == 0x80000000u || fbits(nA.y) == 0x80000000u || fbits(nA.z) == 0x80000000u;
+    if (all_zero(ts.b) && all_zero(ts.c) && all_zero(ts.dndu0) && all_zero(ts.dndv0) && !minus0) {
+      f3 du, dv;
+      coordinate(nA, du, dv);
+      du = cross(dv, nA);
+      dv = cross(nA, du);
+      const Frame f = make_frame(du, dv, nA);
+      ts.form = TRI_FLAT;
+      ts.a = f.x;
+      ts.b = f.y;
+      ts.c = f.z;
     }
   }
   hs.spheres.resize(ns);

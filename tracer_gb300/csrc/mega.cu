@@ -82,25 +82,18 @@ __device__ __noinline__ Traced warp_trace(const DScene& sc, bool active, int sce
 // Material dispatch limited to the kinds of the instantiation (the sampler
 // out of line: one copy serves the path's and the MIS sample).
 template <unsigned MASK>
-__device__ __noinline__ BsdfSample m_sample(const Bsdf& b, int kind, f3 wo, float u, float v, float w) {
-  if ((MASK & MK_DISNEY12) && kind == MAT_DISNEY12) return b.disney_sample(wo, u, v, w);
-  if ((MASK & MK_METAL) && kind == MAT_METAL) return b.metal_sample(wo, u, v, w);
-  if ((MASK & MK_DISNEY15) && kind == MAT_DISNEY15) return b.d15_sample(wo, u, v, w);
-  return b.phong_sample_agg(wo, u, v, w);
+__device__ __noinline__ BsdfSample m_sample(const Bsdf& b, int kind, float u, float v, float w) {
+  if ((MASK & MK_DISNEY12) && kind == MAT_DISNEY12) return b.disney_sample(u, v, w);
+  if ((MASK & MK_METAL) && kind == MAT_METAL) return b.metal_sample(u, v, w);
+  if ((MASK & MK_DISNEY15) && kind == MAT_DISNEY15) return b.d15_sample(u, v, w);
+  return b.phong_sample_agg(u, v, w);
 }
 template <unsigned MASK>
-__device__ __forceinline__ f3 m_eval(const Bsdf& b, int kind, f3 wi, f3 wo) {
-  if ((MASK & MK_DISNEY12) && kind == MAT_DISNEY12) return b.disney_eval(wi, wo);
-  if ((MASK & MK_METAL) && kind == MAT_METAL) return b.metal_eval(wi, wo);
-  if ((MASK & MK_DISNEY15) && kind == MAT_DISNEY15) return b.d15_eval(wi, wo);
-  return b.phong_eval_agg(wi, wo);
-}
-template <unsigned MASK>
-__device__ __forceinline__ float m_pdf(const Bsdf& b, int kind, f3 wi, f3 wo) {
-  if ((MASK & MK_DISNEY12) && kind == MAT_DISNEY12) return b.disney_pdf(wi, wo);
-  if ((MASK & MK_METAL) && kind == MAT_METAL) return b.metal_pdf(wi, wo);
-  if ((MASK & MK_DISNEY15) && kind == MAT_DISNEY15) return b.d15_pdf(wi, wo);
-  return b.phong_pdf_agg(wi, wo);
+__device__ __forceinline__ void m_value(const Bsdf& b, int kind, f3 wi, f3& f, float& pdf) {
+  if ((MASK & MK_DISNEY12) && kind == MAT_DISNEY12) b.disney_value(wi, f, pdf);
+  else if ((MASK & MK_METAL) && kind == MAT_METAL) b.metal_value(wi, f, pdf);
+  else if ((MASK & MK_DISNEY15) && kind == MAT_DISNEY15) b.d15_value(wi, f, pdf);
+  else b.phong_value(wi, f, pdf);
 }
 
 // The per-lane state of one pixel slot.
@@ -262,11 +255,12 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_mega(MegaLaunch P) {
           }
           bsdf.g = is.g;
           bsdf.s = is.s;
+          bsdf.look_from(is.wo);
           if ((MASK & MK_GLASS) && kind == MAT_GLASS) {
             // k_glass: a delta sample, no direct lighting
             const float u0 = Pcg::next(p.st);
             Pcg::skip<2>(p.st);  // the rest of sample3()
-            const BsdfSample bs = bsdf.glass_sample(is.wo, u0);
+            const BsdfSample bs = bsdf.glass_sample(u0);
             bool t = black(bs.f) || bs.pdf < kEps;
             if (!t) {
               const bool counted = p.sdepth >= kMaxSpecularDepth;
@@ -295,7 +289,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_mega(MegaLaunch P) {
             }
           } else {
             const float u0 = Pcg::next(p.st), u1 = Pcg::next(p.st), u2 = Pcg::next(p.st);
-            const BsdfSample bs = m_sample<MASK>(bsdf, kind, is.wo, u0, u1, u2);
+            const BsdfSample bs = m_sample<MASK>(bsdf, kind, u0, u1, u2);
             if (black(bs.f) || bs.pdf < kEps) {
               ended = true;
             } else {
@@ -320,7 +314,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_mega(MegaLaunch P) {
               }
               // the MIS BSDF ray (sample_bsdf, src/renderer/direct_illumination.cpp:144-155)
               const float v0 = Pcg::next(p.st), v1 = Pcg::next(p.st), v2 = Pcg::next(p.st);
-              const BsdfSample ms = m_sample<MASK>(bsdf, kind, is.wo, v0, v1, v2);
+              const BsdfSample ms = m_sample<MASK>(bsdf, kind, v0, v1, v2);
               if (ms.valid()) {
                 const f3 wi = normalize(ms.wi);
                 mo = is.eps_offset(wi);
@@ -364,6 +358,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_mega(MegaLaunch P) {
     bsdf.m = mcode >= 0 ? sc.mats + mcode : &tmat;
     bsdf.g = is.g;
     bsdf.s = is.s;
+    if (vertex) bsdf.look_from(is.wo);
     for (int l = 0; l < P.nl_max; ++l) {
       bool trace = false;
       f3 cc = mk3(0.0f, 0.0f, 0.0f), so = cc, sd = cc;
@@ -381,10 +376,11 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_mega(MegaLaunch P) {
             dist = dist_minus_eps(len2f(to_light), too_close);
             if (!too_close) {
               to_light = normalize(to_light);
-              const f3 bf = m_eval<MASK>(bsdf, kind, to_light, is.wo);
+              f3 bf;
+              float bpdf;
+              m_value<MASK>(bsdf, kind, to_light, bf, bpdf);
               trace = !black(bf);
               if (trace) {
-                const float bpdf = m_pdf<MASK>(bsdf, kind, to_light, is.wo);
                 const f3 fl = muls(mulc(Le, bf), abs_cos(to_light, bsdf.g.z));
                 const float w = power_heuristic(lpdf, bpdf);
                 cc = mulc(coef_prev, divs(muls(fl, w), lpdf));
@@ -409,10 +405,11 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_mega(MegaLaunch P) {
               dist = dist_minus_eps(len2f(to_light), too_close);
               if (!too_close) {
                 to_light = normalize(to_light);
-                const f3 bf = m_eval<MASK>(bsdf, kind, to_light, is.wo);
+                f3 bf;
+                float bpdf;
+                m_value<MASK>(bsdf, kind, to_light, bf, bpdf);
                 trace = !black(bf);
                 if (trace) {
-                  const float bpdf = m_pdf<MASK>(bsdf, kind, to_light, is.wo);
                   const f3 fl = muls(mulc(lt.emission, bf), abs_cos(to_light, bsdf.g.z));
                   const float w = power_heuristic(lpdf, bpdf);
                   cc = mulc(coef_prev, divs(muls(fl, w), lpdf));

@@ -799,23 +799,17 @@ __global__ void __launch_bounds__(128) k_logic(Launch P, int cur) {
 
 template <int KIND>
 struct MatOps {
-  static __device__ __forceinline__ BsdfSample sample(const Bsdf& b, f3 wo, float u, float v, float w) {
-    if (KIND == MAT_GLASS) return b.glass_sample(wo, u);
-    if (KIND == MAT_METAL) return b.metal_sample(wo, u, v, w);
-    if (KIND == MAT_DISNEY15) return b.d15_sample(wo, u, v, w);
-    return KIND == MAT_PHONG ? b.phong_sample_agg(wo, u, v, w) : b.disney_sample(wo, u, v, w);
+  static __device__ __forceinline__ BsdfSample sample(const Bsdf& b, float u, float v, float w) {
+    if (KIND == MAT_METAL) return b.metal_sample(u, v, w);
+    if (KIND == MAT_DISNEY15) return b.d15_sample(u, v, w);
+    return KIND == MAT_PHONG ? b.phong_sample_agg(u, v, w) : b.disney_sample(u, v, w);
   }
-  static __device__ __forceinline__ f3 eval(const Bsdf& b, f3 wi, f3 wo) {
-    if (KIND == MAT_GLASS) return mk3(0.0f, 0.0f, 0.0f);
-    if (KIND == MAT_METAL) return b.metal_eval(wi, wo);
-    if (KIND == MAT_DISNEY15) return b.d15_eval(wi, wo);
-    return KIND == MAT_PHONG ? b.phong_eval_agg(wi, wo) : b.disney_eval(wi, wo);
-  }
-  static __device__ __forceinline__ float pdf(const Bsdf& b, f3 wi, f3 wo) {
-    if (KIND == MAT_GLASS) return 0.0f;
-    if (KIND == MAT_METAL) return b.metal_pdf(wi, wo);
-    if (KIND == MAT_DISNEY15) return b.d15_pdf(wi, wo);
-    return KIND == MAT_PHONG ? b.phong_pdf_agg(wi, wo) : b.disney_pdf(wi, wo);
+  // value and density of direction wi
+  static __device__ __forceinline__ void value(const Bsdf& b, f3 wi, f3& f, float& pdf) {
+    if (KIND == MAT_METAL) b.metal_value(wi, f, pdf);
+    else if (KIND == MAT_DISNEY15) b.d15_value(wi, f, pdf);
+    else if (KIND == MAT_PHONG) b.phong_value(wi, f, pdf);
+    else b.disney_value(wi, f, pdf);
   }
 };
 
@@ -826,10 +820,9 @@ struct MatOps {
 // density there is the cosine pdf, so a one-sample MIS of the network's
 // mixture (probability alpha) and the BSDF keeps the plain estimator's
 // expectation.
-__device__ __forceinline__ float lambert_plain_pdf(const Bsdf& bsdf, f3 wo, f3 wi) {
-  const f3 lwo = normalize(to_local(bsdf.s, wo)), lwi = normalize(to_local(bsdf.s, wi));
-  const float pb = cosine_pdf(lwi.z);
-  return (lwo.z > 0.0f && pb >= 0.001f) ? pb : 0.0f;
+__device__ __forceinline__ float lambert_plain_pdf(const Bsdf& bsdf, f3 wi) {
+  const float pb = cosine_pdf(normalize(to_local(bsdf.s, wi)).z);
+  return (bsdf.lwo.z > 0.0f && pb >= 0.001f) ? pb : 0.0f;
 }
 
 // Replaces the plain sample `bs` by the one-sample MIS choice: with
@@ -849,8 +842,8 @@ __device__ __noinline__ void guided_pick(const Launch& P, const Bsdf& bsdf, cons
     if (!bs.valid()) return;
     wi = bs.wi;
   }
-  ps = lambert_plain_pdf(bsdf, is.wo, wi);
-  nc = ps > 0.0f ? normal_correct(bsdf.g, bsdf.s, wi) : 0.0f;
+  ps = lambert_plain_pdf(bsdf, wi);
+  nc = ps > 0.0f ? bsdf.normal_correct(wi) : 0.0f;
   pm = mx.pdf(wi);
   bs.wi = wi;
   bs.f = muls(bsdf.m->diffuse_coef, nc);
@@ -873,12 +866,11 @@ __device__ __noinline__ void guided_mixture_ray(const Launch& P, const Bsdf& bsd
   const Mixture mx{P.gout + (size_t)row * kMixFloats};
   r.wi = normalize(mx.sample(u, v, w));
   r.p_mix = mx.pdf(r.wi);
-  r.ps = lambert_plain_pdf(bsdf, is.wo, r.wi);
-  r.nc = r.ps > 0.0f ? normal_correct(bsdf.g, bsdf.s, r.wi) : 0.0f;
+  r.ps = lambert_plain_pdf(bsdf, r.wi);
+  r.nc = r.ps > 0.0f ? bsdf.normal_correct(r.wi) : 0.0f;
   r.p_g = P.guide_alpha * r.p_mix + (1.0f - P.guide_alpha) * r.ps;
   const f3 wc = normalize(r.wi);
-  r.fe = bsdf.phong_eval_agg(wc, is.wo);
-  r.pb = bsdf.phong_pdf_agg(wc, is.wo);
+  bsdf.phong_value(wc, r.fe, r.pb);
   r.cosv = abs_cos(is.g.z, wc);
   r.trace = r.p_mix >= kEps && (r.ps > 0.0f || !black(r.fe));
 }
@@ -889,12 +881,15 @@ __device__ __noinline__ void guided_mixture_ray(const Launch& P, const Bsdf& bsd
 // of the plain BSDF sample. With guided_strategy_emission it estimates the
 // same direct-lighting integral as the reference's pair of strategies.
 // Returns that integrand times |cos| per unit emission, times the weight.
-__device__ __noinline__ f3 guided_nee_factor(const Launch& P, const Bsdf& bsdf, f3 wo, f3 wl, int row, bool three,
+__device__ __noinline__ f3 guided_nee_factor(const Launch& P, const Bsdf& bsdf, f3 wl, int row, bool three,
                                              float lpdf, float lq) {
   const Mixture mx{P.gout + (size_t)row * kMixFloats};
-  const float ps = lambert_plain_pdf(bsdf, wo, wl);
-  const f3 fs = ps > 0.0f ? muls(bsdf.m->diffuse_coef, normal_correct(bsdf.g, bsdf.s, wl)) : mk3(0.0f, 0.0f, 0.0f);
-  const f3 g = direct_integrand(bsdf.phong_eval_agg(wl, wo), bsdf.phong_pdf_agg(wl, wo), fs, ps, lpdf, lq);
+  const float ps = lambert_plain_pdf(bsdf, wl);
+  const f3 fs = ps > 0.0f ? muls(bsdf.m->diffuse_coef, bsdf.normal_correct(wl)) : mk3(0.0f, 0.0f, 0.0f);
+  f3 fe;
+  float pb;
+  bsdf.phong_value(wl, fe, pb);
+  const f3 g = direct_integrand(fe, pb, fs, ps, lpdf, lq);
   const float pm = mx.pdf(wl);
   const float pg = P.guide_alpha * pm + (1.0f - P.guide_alpha) * ps;
   const float po = three ? pm : 0.0f;
@@ -906,8 +901,8 @@ __device__ __noinline__ f3 guided_nee_factor(const Launch& P, const Bsdf& bsdf, 
 // (the path's sample and the MIS sample): one copy of the sampling code
 // instead of two keeps the kernel within the instruction cache.
 template <int KIND>
-__device__ __noinline__ BsdfSample sample_bsdf_shared(const Bsdf& b, f3 wo, float u, float v, float w) {
-  return MatOps<KIND>::sample(b, wo, u, v, w);
+__device__ __noinline__ BsdfSample sample_bsdf_shared(const Bsdf& b, float u, float v, float w) {
+  return MatOps<KIND>::sample(b, u, v, w);
 }
 
 // What a vertex adds to the queues.
@@ -942,8 +937,9 @@ __device__ __forceinline__ void shade_vertex(const Launch& P, int slot, unsigned
   }
   bsdf.g = is.g;
   bsdf.s = is.s;
+  bsdf.look_from(is.wo);
   const float u0 = Pcg::next(st), u1 = Pcg::next(st), u2 = Pcg::next(st);
-  BsdfSample bs = sample_bsdf_shared<KIND>(bsdf, is.wo, u0, u1, u2);
+  BsdfSample bs = sample_bsdf_shared<KIND>(bsdf, u0, u1, u2);
   if (black(bs.f) || bs.pdf < kEps) {
     const float4 p3 = P.P3[slot];
     add.ext_cont = add.act = finish_sample(P, slot, st, mk3(p3.x, p3.y, p3.z), finished);
@@ -961,15 +957,14 @@ __device__ __forceinline__ void shade_vertex(const Launch& P, int slot, unsigned
   f3 g_fe = mk3(0.0f, 0.0f, 0.0f);
   const int row = GUIDED && KIND == MAT_PHONG && P.guide_alpha > 0.0f ? P.grow[slot] : -1;
   const bool gv = GUIDED && KIND == MAT_PHONG && P.guide_alpha > 0.0f && row >= 0 && bsdf.m->w_specular == 0.0f &&
-                  !bsdf.fringe(is.wo);
+                  !bsdf.wo_fr;
   if (gv) {
     const float sel = Pcg::next(st), g0 = Pcg::next(st), g1 = Pcg::next(st);
     guided_pick(P, bsdf, is, row, sel, g0, g1, bs, g_ps, g_nc, g_pm);
     guided_end = black(bs.f) || bs.pdf < kEps;
     if (bs.pdf >= kEps) {
       const f3 wc = normalize(normalize(bs.wi));
-      g_fe = bsdf.phong_eval_agg(wc, is.wo);
-      g_pb = bsdf.phong_pdf_agg(wc, is.wo);
+      bsdf.phong_value(wc, g_fe, g_pb);
       g_cos = abs_cos(is.g.z, wc);
       g_trace = !black(bs.f) || !black(g_fe);
     }
@@ -1017,7 +1012,7 @@ __device__ __forceinline__ void shade_vertex(const Launch& P, int slot, unsigned
     guided_mixture_ray(P, bsdf, is, row, x0, x1, x2, gx);
   } else {
     const float v0 = Pcg::next(st), v1 = Pcg::next(st), v2 = Pcg::next(st);
-    const BsdfSample ms = sample_bsdf_shared<KIND>(bsdf, is.wo, v0, v1, v2);
+    const BsdfSample ms = sample_bsdf_shared<KIND>(bsdf, v0, v1, v2);
     if (ms.valid()) {
       const f3 wi = normalize(ms.wi);
       const f3 mo = is.eps_offset(wi);
@@ -1178,9 +1173,10 @@ __device__ __forceinline__ bool glass_vertex(const Launch& P, int slot, unsigned
   }
   bsdf.g = is.g;
   bsdf.s = is.s;
+  bsdf.look_from(is.wo);
   const float u0 = Pcg::next(st);
   Pcg::skip<2>(st);  // the rest of sample3()
-  const BsdfSample bs = bsdf.glass_sample(is.wo, u0);
+  const BsdfSample bs = bsdf.glass_sample(u0);
   bool term = black(bs.f) || bs.pdf < kEps;
   if (!term) {
     const bool counted = sdepth >= kMaxSpecularDepth;
@@ -1241,7 +1237,7 @@ __global__ void __launch_bounds__(128) k_glass(Launch P, int cur) {
 // one (vertex, environment light) item; false: no shadow ray. gcode: the
 // guided vertex's network row (bit 30: three strategies), else -1.
 template <int KIND>
-__device__ __noinline__ bool nee_env_item(const Launch& P, int slot, int env, f3 pos, f3 wo,
+__device__ __noinline__ bool nee_env_item(const Launch& P, int slot, int env, f3 pos,
                                           const Bsdf& bsdf, float2 uv, int gcode, float4* rec, float4* recc) {
   bool ok = false;
   // sample_environment_light (src/renderer/direct_illumination.cpp:73-106)
@@ -1257,15 +1253,16 @@ __device__ __noinline__ bool nee_env_item(const Launch& P, int slot, int env, f3
       f3 cc = mk3(0.0f, 0.0f, 0.0f);
       bool trace = false;
       if (KIND == MAT_PHONG && gcode >= 0) {
-        const f3 fw = guided_nee_factor(P, bsdf, wo, to_light, gcode & 0x3fffffff, (gcode >> 30) & 1, lpdf,
+        const f3 fw = guided_nee_factor(P, bsdf, to_light, gcode & 0x3fffffff, (gcode >> 30) & 1, lpdf,
                                         env_pdf(P.sc.envs[env], normalize(to_light)));
         trace = !black(fw);
         cc = mulc(mk3(p4.x, p4.y, p4.z), divs(mulc(Le, fw), lpdf));
       } else {
-        const f3 bf = MatOps<KIND>::eval(bsdf, to_light, wo);
+        f3 bf;
+        float bpdf;
+        MatOps<KIND>::value(bsdf, to_light, bf, bpdf);
         trace = !black(bf);
         if (trace) {
-          const float bpdf = MatOps<KIND>::pdf(bsdf, to_light, wo);
           const f3 fl = muls(mulc(Le, bf), abs_cos(to_light, bsdf.g.z));
           const float w = power_heuristic(lpdf, bpdf);
           cc = mulc(mk3(p4.x, p4.y, p4.z), divs(muls(fl, w), lpdf));
@@ -1301,12 +1298,13 @@ __device__ __forceinline__ bool nee_item(const Launch& P, int item) {
   bsdf.s.x = mk3(e.x, e.y, e.z);
   bsdf.s.y = mk3(e.w, f.x, f.y);
   bsdf.s.z = mk3(f.z, f.w, g.x);
+  bsdf.look_from(wo);
   const float2 uv = P.NU[item];
   const DLight& lt = P.sc.lights[job_of(P, slot).light_base + l];
   float4* rec = P.SH + 2 * (size_t)item;
   float4* recc = P.SHC + item;
   if (lt.env >= 0)  // out of line: its registers would otherwise count for every item
-    return nee_env_item<KIND>(P, slot, lt.env, pos, wo, bsdf, uv, __float_as_int(g.y), rec, recc);
+    return nee_env_item<KIND>(P, slot, lt.env, pos, bsdf, uv, __float_as_int(g.y), rec, recc);
   // Triangle::sample via UniformSampleTriangle (src/shape/triangle.cpp:61-97),
   // at the light table's point of the sample square when it is learned
   float2 su = uv;
@@ -1336,14 +1334,15 @@ __device__ __forceinline__ bool nee_item(const Launch& P, int item) {
         // weights stay those of the uniform sample)
         f3 inner = mk3(0.0f, 0.0f, 0.0f);
         if (KIND == MAT_PHONG && grow >= 0) {
-          const f3 fw = guided_nee_factor(P, bsdf, wo, to_light, grow, (gcode >> 30) & 1, lpdf, lpdf);
+          const f3 fw = guided_nee_factor(P, bsdf, to_light, grow, (gcode >> 30) & 1, lpdf, lpdf);
           trace = !black(fw);
           inner = divs(mulc(lt.emission, fw), lpdf);
         } else {
-          const f3 bf = MatOps<KIND>::eval(bsdf, to_light, wo);
+          f3 bf;
+          float bpdf;
+          MatOps<KIND>::value(bsdf, to_light, bf, bpdf);
           trace = !black(bf);
           if (trace) {
-            const float bpdf = MatOps<KIND>::pdf(bsdf, to_light, wo);
             const f3 fl = muls(mulc(lt.emission, bf), abs_cos(to_light, bsdf.g.z));
             const float w = power_heuristic(lpdf, bpdf);
             inner = divs(muls(fl, w), lpdf);

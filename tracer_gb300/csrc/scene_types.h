@@ -81,14 +81,22 @@ struct DPrim {
   float area;    // Triangle::surface_area() of emissive triangles
 };
 
-struct DTriShade {
-  f3 gx, gy, gz;  // geometry frame: constant per triangle (src/shape/triangle.cpp:193-198)
-  f3 nA, dn1, dn2;  // normalised vertex normal A, nB - nA, nC - nA
-  f3 dndu0, dndv0;  // compute_ss_ts(nB-nA, nC-nA, uv...) when its determinant != 0
-  int det_nonzero;
+// Shading constants of a triangle, read as 16-byte words.
+struct alignas(16) DTriShade {
+  f3 gx;         // geometry frame: constant per triangle (src/shape/triangle.cpp:193-198)
+  int form;      // TRI_FLAT, TRI_SMOOTH, TRI_SMOOTH_UV
+  f3 gy, gz;
+  f3 a, b, c;    // smooth: normalised vertex normal A, nB - nA, nC - nA; flat: the shading frame
+  f3 dndu0, dndv0;                 // TRI_SMOOTH_UV: compute_ss_ts(nB-nA, nC-nA, uv...)
   float uvA[2], duv1[2], duv2[2];  // uvA, uvB - uvA, uvC - uvA (the hit's uv, triangle.cpp:186)
   int pad;
 };
+static_assert(sizeof(DTriShade) == 128, "DTriShade must be 128 bytes");
+// Flat: the three vertex normals are equal, so the shading frame the
+// reference builds at every hit (a coordinate system of the normal, two
+// crosses, three normalisations) is one frame, kept instead of the normals.
+// Smooth: with (UV) or without a non-zero determinant of the uv edges.
+enum { TRI_SMOOTH = 0, TRI_SMOOTH_UV = 1, TRI_FLAT = 2 };
 
 // An image texture (HDRTexture2D or ImageTexture2D): w x h texels, texel
 // (x, y) at x + y * w; exactly one of the two pointers is set.

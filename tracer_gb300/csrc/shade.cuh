@@ -112,19 +112,31 @@ struct Isect {
 };
 
 // Triangle::intersect_p hit record (src/shape/triangle.cpp:175-213); the
-// geometry frame and compute_ss_ts of the normals are per-triangle constants.
+// geometry frame and compute_ss_ts of the normals are per-triangle constants,
+// and so is the whole shading frame of a flat triangle.
 __device__ __forceinline__ void triangle_isect(const DTriShade& ts, f3 o, f3 d, float t, float alpha, float beta,
                                                Isect& is) {
+  const float4* w = reinterpret_cast<const float4*>(&ts);
+  const float4 w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2), w3 = __ldg(w + 3), w4 = __ldg(w + 4);
   is.wo = -d;
   is.pos = o + scale(d, t);
-  is.g.x = ts.gx;
-  is.g.y = ts.gy;
-  is.g.z = ts.gz;
-  const f3 sn = ts.nA + scale(ts.dn1, alpha) + scale(ts.dn2, beta);
+  is.g.x = mk3(w0.x, w0.y, w0.z);
+  is.g.y = mk3(w1.x, w1.y, w1.z);
+  is.g.z = mk3(w1.w, w2.x, w2.y);
+  const f3 a = mk3(w2.z, w2.w, w3.x), b = mk3(w3.y, w3.z, w3.w), c = mk3(w4.x, w4.y, w4.z);
+  const int form = __float_as_int(w0.w);
+  if (form == TRI_FLAT) {
+    is.s.x = a;
+    is.s.y = b;
+    is.s.z = c;
+    return;
+  }
+  const f3 sn = a + scale(b, alpha) + scale(c, beta);
   f3 dndu, dndv;
-  if (ts.det_nonzero) {
-    dndu = ts.dndu0;
-    dndv = ts.dndv0;
+  if (form == TRI_SMOOTH_UV) {
+    const float4 w5 = __ldg(w + 5);
+    dndu = mk3(w4.w, w5.x, w5.y);
+    dndv = mk3(w5.z, w5.w, ts.dndv0.z);
   } else {
     coordinate(sn, dndu, dndv);
   }
@@ -435,71 +447,95 @@ __device__ __forceinline__ float disney_ss(float Fss, float S) {
   return disney_ss_d(Fss, S);
 }
 
-// normal_correct_factor (src/utility/coordinate.hpp:43-52)
-__device__ __forceinline__ float normal_correct(const Frame& g, const Frame& s, f3 wi) {
-  const float dem = fabsf(cosv(g.z, wi));
-  return dem < kEps ? 1.0f : fabsf(cosv(s.z, wi)) / dem;
+// Phong without a specular lobe: weight and colour zero, and an exponent for
+// which the lobe's value is finite, so that it adds exactly zero to the
+// diffuse lobe's value and density and need not be evaluated.
+__device__ __forceinline__ bool lambert(const DMat& m) {
+  return m.w_specular == 0.0f && black(m.specular) && m.ns >= 0.0f && m.ns <= 1e6f;
 }
 
+// A BSDF at a surface point seen from wo (LocalBSDF, src/core/bsdf.hpp).
+// The value and the density for one direction are needed together wherever
+// either is, and share the local directions, the half vector and the
+// distribution term: one function gives both. (Where a value is zero its
+// density is never read.) Sharing them, and skipping what is exactly zero
+// or one (lambert, the normal correction of equal normals), took a
+// 1024x768x16 room from 194 to 184 ms, the guided pass from 113 to 106, the
+// Disney grid from 60.9 to 56.9.
 struct Bsdf {
   const DMat* m;
   Frame g, s;
+  f3 lwo;       // wo in the shading frame, normalised
+  bool wo_g;    // wo on the geometry normal's side
+  bool wo_fr;   // wo in the fringe
+  bool same_n;  // geometry and shading normal are equal
+
+  __device__ __forceinline__ void look_from(f3 wo) {
+    wo_g = pos_hemi(g, wo);
+    wo_fr = wo_g ^ pos_hemi(s, wo);
+    lwo = normalize(to_local(s, wo));
+    same_n = g.z.x == s.z.x && g.z.y == s.z.y && g.z.z == s.z.z;
+  }
+  // normal_correct_factor (src/utility/coordinate.hpp:43-52)
+  __device__ __forceinline__ float normal_correct(f3 wi) const {
+    if (same_n) return 1.0f;  // x / x, or the 1 of a small cosine
+    const float dem = fabsf(cosv(g.z, wi));
+    return dem < kEps ? 1.0f : fabsf(cosv(s.z, wi)) / dem;
+  }
 
   // LocalBSDF black-fringe handling (src/core/bsdf.hpp:55-91)
   __device__ __forceinline__ bool fringe(f3 w) const { return pos_hemi(g, w) ^ pos_hemi(s, w); }
-  __device__ __forceinline__ f3 eval_fringe(f3 wi, f3 wo) const {
-    if (pos_hemi(g, wi) & pos_hemi(g, wo)) return muls(m->albedo, kInvPi);
-    return mk3(0.0f, 0.0f, 0.0f);
+  __device__ __forceinline__ void fringe_value(f3 wi, f3& f, float& pdf) const {
+    const bool wi_g = pos_hemi(g, wi);
+    f = mk3(0.0f, 0.0f, 0.0f);
+    pdf = 0.0f;
+    if (wi_g & wo_g) f = muls(m->albedo, kInvPi);
+    if (!(wi_g ^ wo_g)) pdf = cosine_pdf(normalize(to_local(g, wi)).z);
   }
-  __device__ __forceinline__ BsdfSample sample_fringe(f3 wo, float u, float v) const {
+  __device__ __forceinline__ BsdfSample sample_fringe(float u, float v) const {
     BsdfSample r;
     r.pdf = 0.0f;
     r.f = mk3(0.0f, 0.0f, 0.0f);
     r.wi = r.f;
-    if (!pos_hemi(g, wo)) return r;
+    if (!wo_g) return r;
     const f3 lwi = cosine_hemisphere(u, v);
     const float pdf = cosine_pdf(lwi.z);
     if (pdf < kEps) return r;
     const f3 wi = normalize(to_global(g, lwi));
-    const float nc = normal_correct(g, s, wi);
+    const float nc = normal_correct(wi);
     r.wi = wi;
     r.f = muls(muls(m->albedo, kInvPi), nc);
     r.pdf = pdf;
     return r;
   }
-  __device__ __forceinline__ float pdf_fringe(f3 wi, f3 wo) const {
-    if (pos_hemi(g, wi) ^ pos_hemi(g, wo)) return 0.0f;
-    return cosine_pdf(normalize(to_local(g, wi)).z);
-  }
 
   // ---- AggregateBSDF<2> of Phong (src/material/aggregate_bsdf.hpp:36-118)
-  __device__ f3 phong_eval_agg(f3 wi, f3 wo) const {
-    if (fringe(wi) | fringe(wo)) return eval_fringe(wi, wo);
-    const f3 lwi = normalize(to_local(s, wi)), lwo = normalize(to_local(s, wo));
-    if (!lwi.z || !lwo.z) return mk3(0.0f, 0.0f, 0.0f);
-    f3 r = mk3(0.0f, 0.0f, 0.0f);
-    r = r + diffuse_eval(*m, lwi, lwo);
-    r = r + phong_eval(*m, lwi, lwo);
-    return r;
-  }
-  __device__ float phong_pdf_agg(f3 wi, f3 wo) const {
-    if (fringe(wi) | fringe(wo)) return pdf_fringe(wi, wo);
-    const f3 lwi = normalize(to_local(s, wi)), lwo = normalize(to_local(s, wo));
-    if (!lwi.z || !lwo.z) return 0.0f;
-    float ws = 0.0f, pdf = 0.0f;
+  __device__ void phong_value(f3 wi, f3& f, float& pdf) const {
+    if (fringe(wi) | wo_fr) {
+      fringe_value(wi, f, pdf);
+      return;
+    }
+    const f3 lwi = normalize(to_local(s, wi));
+    f = mk3(0.0f, 0.0f, 0.0f);
+    pdf = 0.0f;
+    if (!lwi.z || !lwo.z) return;
+    float ws = 0.0f;
+    f = f + diffuse_eval(*m, lwi, lwo);
     ws += m->w_diffuse;
     pdf += m->w_diffuse * diffuse_pdf(lwi, lwo);
     ws += m->w_specular;
-    pdf += m->w_specular * phong_pdf(*m, lwi, lwo);
-    return ws > 0.0f ? pdf / ws : 0.0f;
+    if (!lambert(*m)) {
+      f = f + phong_eval(*m, lwi, lwo);
+      pdf += m->w_specular * phong_pdf(*m, lwi, lwo);
+    }
+    pdf = ws > 0.0f ? pdf / ws : 0.0f;
   }
-  __device__ BsdfSample phong_sample_agg(f3 wo, float u, float v, float w) const {
-    if (fringe(wo)) return sample_fringe(wo, u, v);
+  __device__ BsdfSample phong_sample_agg(float u, float v, float w) const {
+    if (wo_fr) return sample_fringe(u, v);
     BsdfSample out;
     out.pdf = 0.0f;
     out.f = mk3(0.0f, 0.0f, 0.0f);
     out.wi = out.f;
-    const f3 lwo = normalize(to_local(s, wo));
     if (!lwo.z) return out;
     float ws = 0.0f;
     ws += m->w_diffuse;
@@ -536,12 +572,12 @@ struct Bsdf {
       f = f + diffuse_eval(*m, lwi, lwo);
       pdf += diffuse_pdf(lwi, lwo) * w0;
     }
-    if (which != 1) {
+    if (which != 1 && !lambert(*m)) {
       f = f + phong_eval(*m, lwi, lwo);
       pdf += phong_pdf(*m, lwi, lwo) * w1;
     }
     const f3 wi = to_global(s, lwi);
-    const float nc = normal_correct(g, s, wi);
+    const float nc = normal_correct(wi);
     out.wi = wi;
     out.f = muls(f, nc);
     out.pdf = pdf;
@@ -553,15 +589,15 @@ struct Bsdf {
   // between sample and pdf, the pdf mixes with (1 - pdf_diffuse), clearcoat's
   // pdf passes (sin_phi, cos_phi, gloss) to gtr1, and the Smith term gets
   // (sin_phi, cos_phi) in its (cos_phi, sin_phi) slots.
-  __device__ __forceinline__ void alphas(float& ax, float& ay) const {
-    ax = m->ax;  // per-material constants computed at upload
-    ay = m->ay;
-  }
-  __device__ f3 disney_eval(f3 wi, f3 wo) const {
-    if (fringe(wi) | fringe(wo)) return eval_fringe(wi, wo);
+  __device__ void disney_value(f3 wi, f3& f, float& pdf) const {
+    if (fringe(wi) | wo_fr) {
+      fringe_value(wi, f, pdf);
+      return;
+    }
+    f = mk3(0.0f, 0.0f, 0.0f);
+    pdf = 0.0f;
     const f3 lwi = normalize(to_local(s, wi));
-    const f3 lwo = normalize(to_local(s, wo));
-    if (lwi.z < kEps || lwo.z < kEps) return mk3(0.0f, 0.0f, 0.0f);
+    if (lwi.z < kEps || lwo.z < kEps) return;
     const float NdotL = lwi.z, NdotV = lwo.z;
     const f3 H = normalize(lwi + lwo);
     const float LdotH = dot(lwi, H);
@@ -571,11 +607,9 @@ struct Bsdf {
     const f3 one = mk3(1.0f, 1.0f, 1.0f);
     const f3 Cspec0 = mix3(muls(mix3(one, Ctint, m->specular_tint), m->specular_s * 0.08f), bc, m->metallic);
     const f3 Csheen = mix3(one, Ctint, m->sheen_tint);
-    float ax, ay;
-    alphas(ax, ay);
-    const float phi_h = local_phi(H);
+    const float ax = m->ax, ay = m->ay;  // per-material constants computed at upload
     float sph, cph;
-    sincosf(phi_h, &sph, &cph);
+    sincosf(local_phi(H), &sph, &cph);
     const float Ds = anisotropic_gtr2(sph, cph, local_cos_to_sin(H.z), H.z, ax, ay);
     const float FH = one_minus_5(LdotH);
     const f3 Fs = mix3(Cspec0, one, FH);
@@ -599,44 +633,29 @@ struct Bsdf {
       const f3 Fsheen = muls(Csheen, FH * m->sheen);
       fd = fd + muls(muls(muls(bc, kInvPi), mixf(Fd, ss, m->subsurface)) + Fsheen, 1.0f - m->metallic);
     }
-    return muls(fd, normal_correct(g, s, wi));
-  }
-  __device__ float disney_pdf(f3 wi, f3 wo) const {
-    if (fringe(wi) | fringe(wo)) return pdf_fringe(wi, wo);
-    const float p_diffuse = m->p_diffuse;
-    const float p_specular = m->p_spec_pdf;
-    float ax, ay;
-    alphas(ax, ay);
-    const f3 lwi = normalize(to_local(s, wi));
-    const f3 lwo = normalize(to_local(s, wo));
-    if (lwi.z < kEps) return 0.0f;
-    const f3 H = normalize(lwi + lwo);
+    f = muls(fd, normal_correct(wi));
     const float pdf_diffuse = cosine_pdf(lwi.z);
-    float sph, cph;
-    sincosf(local_phi(H), &sph, &cph);
-    const float pdf_spec = anisotropic_gtr2(sph, cph, local_cos_to_sin(H.z), H.z, ax, ay) * H.z / (4.0f * dot(lwi, H));
-    const float pdf_cc = gtr1(sph, cph, m->clearcoat_gloss) * H.z / (4.0f * dot(lwi, H));
-    const float pdf = p_diffuse * pdf_diffuse + (1.0f - pdf_diffuse) * (p_specular * pdf_spec + (1.0f - p_specular) * pdf_cc);
-    if (!isfinite(pdf)) return 0.0f;
-    return pdf;
+    const float pdf_spec = Ds * H.z / (4.0f * LdotH);
+    const float pdf_cc = gtr1(sph, cph, m->clearcoat_gloss) * H.z / (4.0f * LdotH);
+    const float p_specular = m->p_spec_pdf;
+    pdf = m->p_diffuse * pdf_diffuse +
+          (1.0f - pdf_diffuse) * (p_specular * pdf_spec + (1.0f - p_specular) * pdf_cc);
+    if (!isfinite(pdf)) pdf = 0.0f;
   }
-  __device__ BsdfSample disney_sample(f3 wo, float u, float v, float w) const {
-    if (fringe(wo)) return sample_fringe(wo, u, v);
+  __device__ BsdfSample disney_sample(float u, float v, float w) const {
+    if (wo_fr) return sample_fringe(u, v);
     BsdfSample r;
     r.pdf = 0.0f;
     r.f = mk3(0.0f, 0.0f, 0.0f);
     r.wi = r.f;
     const float p_diffuse = m->p_diffuse;
     const float p_specular = m->p_spec_sample;
-    const f3 lwo = normalize(to_local(s, wo));
     f3 lwi = mk3(0.0f, 0.0f, 0.0f);
     float sel = u;
-    float ax, ay;
-    alphas(ax, ay);
     if (sel < p_diffuse) lwi = cosine_hemisphere(v, w);
     sel -= p_diffuse;
     if (sel < p_specular) {
-      const f3 lwh = sample_aniso_gtr2(ax, ay, v, w);
+      const f3 lwh = sample_aniso_gtr2(m->ax, m->ay, v, w);
       if (lwh.z > 0.0f) {
         lwi = normalize(scale(lwh, 2.0f * dot(lwo, lwh)) - lwo);
         if (lwi.z <= 0.0f) lwi = mk3(0.0f, 0.0f, 0.0f);
@@ -650,20 +669,18 @@ struct Bsdf {
     }
     if (all_zero(lwi)) return r;
     r.wi = to_global(s, lwi);
-    r.f = disney_eval(r.wi, wo);
-    r.pdf = disney_pdf(r.wi, wo);
+    disney_value(r.wi, r.f, r.pdf);
     return r;
   }
 
   // ---- GlassBSDF (src/material/glass.cpp:11-99) with DielectricFresnelPoint(ior, 1) and
   // TransportMode::Radiance: a delta BSDF (eval and pdf 0); u picks reflection with the
   // Fresnel probability, else refraction (refract_dir, src/utility/reflection.hpp:43-51)
-  __device__ BsdfSample glass_sample(f3 wo, float u) const {
+  __device__ BsdfSample glass_sample(float u) const {
     BsdfSample out;
     out.pdf = 0.0f;
     out.f = mk3(0.0f, 0.0f, 0.0f);
     out.wi = out.f;
-    const f3 lwo = normalize(to_local(s, wo));
     const f3 nor = lwo.z > 0.0f ? mk3(0.0f, 0.0f, 1.0f) : mk3(0.0f, 0.0f, -1.0f);
     const float fr = dielectric_fresnel(m->ior, 1.0f, lwo.z);
     if (u < fr) {
@@ -671,7 +688,7 @@ struct Bsdf {
       const f3 wi = to_global(s, lwi);
       const float q = fr / fabsf(lwi.z);
       out.wi = wi;
-      out.f = muls(mk3(m->kr.x * q, m->kr.y * q, m->kr.z * q), normal_correct(g, s, wi));
+      out.f = muls(mk3(m->kr.x * q, m->kr.y * q, m->kr.z * q), normal_correct(wi));
       out.pdf = fr;
       out.delta = true;
       return out;
@@ -689,7 +706,7 @@ struct Bsdf {
     const f3 f = mk3(((corr * m->kt_sqrt.x) * (1.0f - fr)) / az, ((corr * m->kt_sqrt.y) * (1.0f - fr)) / az,
                      ((corr * m->kt_sqrt.z) * (1.0f - fr)) / az);
     out.wi = wi;
-    out.f = muls(f, normal_correct(g, s, wi));
+    out.f = muls(f, normal_correct(wi));
     out.pdf = 1.0f - fr;
     out.delta = true;
     return out;
@@ -697,7 +714,7 @@ struct Bsdf {
 
   // ---- Metal: AggregateBSDF<1> (src/material/aggregate_bsdf.hpp:36-118) of one
   // GGXMicrofacetReflectionBXDF (src/material/bxdf/microfacet_refl_bxdf.cpp:13-78), weight 1
-  __device__ void ggx(f3 lwi, f3 lwo, f3* eval, float* pdf) const {
+  __device__ void ggx(f3 lwi, f3 lwo, f3& eval, float& pdf) const {
     const float cos_theta_i = lwi.z, cos_theta_o = lwo.z;
     const f3 lwh = normalize(lwi + lwo);
     const float cos_theta_d = dot(lwi, lwh);
@@ -711,15 +728,13 @@ struct Bsdf {
     sincosf(local_phi(lwo), &sin_phi_o, &cos_phi_o);
     const float Gi = smith_aniso_gtr2(cos_phi_i, sin_phi_i, m->ax, m->ay, local_tan_theta(lwi));
     const float Go = smith_aniso_gtr2(cos_phi_o, sin_phi_o, m->ax, m->ay, local_tan_theta(lwo));
-    if (eval) {
-      const float G = Gi * Go;
-      const float den = fabsf(4.0f * cos_theta_i * cos_theta_o);
-      const float Fr = m->f_paint.x * conductor_fresnel(m->f_eta2.x, m->f_etak2.x, cos_theta_d);
-      const float Fg = m->f_paint.y * conductor_fresnel(m->f_eta2.y, m->f_etak2.y, cos_theta_d);
-      const float Fb = m->f_paint.z * conductor_fresnel(m->f_eta2.z, m->f_etak2.z, cos_theta_d);
-      *eval = mk3(Fr * D * G / den, Fg * D * G / den, Fb * D * G / den);
-    }
-    if (pdf) *pdf = Go * D / (4.0f * cos_theta_o);
+    const float G = Gi * Go;
+    const float den = fabsf(4.0f * cos_theta_i * cos_theta_o);
+    const float Fr = m->f_paint.x * conductor_fresnel(m->f_eta2.x, m->f_etak2.x, cos_theta_d);
+    const float Fg = m->f_paint.y * conductor_fresnel(m->f_eta2.y, m->f_etak2.y, cos_theta_d);
+    const float Fb = m->f_paint.z * conductor_fresnel(m->f_eta2.z, m->f_etak2.z, cos_theta_d);
+    eval = mk3(Fr * D * G / den, Fg * D * G / den, Fb * D * G / den);
+    pdf = Go * D / (4.0f * cos_theta_o);
   }
   // microfacet::sample_anisotropic_gtr2_with_visible_normal (src/material/utility/microfacet.cpp:58-80)
   __device__ f3 sample_vndf(f3 ve, float u, float v) const { return sample_vndf_a(ve, u, v, m->ax, m->ay); }
@@ -739,33 +754,25 @@ struct Bsdf {
     const f3 nh = scale(t1, t_1) + scale(t2, t_2) + scale(vh, sqrtf(0.0f < q ? q : 0.0f));
     return normalize(mk3(ax * nh.x, ay * nh.y, 0.0f < nh.z ? nh.z : 0.0f));
   }
-  __device__ f3 metal_eval(f3 wi, f3 wo) const {
-    if (fringe(wi) | fringe(wo)) return eval_fringe(wi, wo);
-    const f3 lwi = normalize(to_local(s, wi)), lwo = normalize(to_local(s, wo));
-    if (!lwi.z || !lwo.z) return mk3(0.0f, 0.0f, 0.0f);
-    f3 r = mk3(0.0f, 0.0f, 0.0f);
-    if (!(lwi.z <= 0.0f || lwo.z <= 0.0f)) {
-      f3 e;
-      ggx(lwi, lwo, &e, nullptr);
-      r = r + e;
+  __device__ void metal_value(f3 wi, f3& f, float& pdf) const {
+    if (fringe(wi) | wo_fr) {
+      fringe_value(wi, f, pdf);
+      return;
     }
-    return r;
+    const f3 lwi = normalize(to_local(s, wi));
+    f = mk3(0.0f, 0.0f, 0.0f);
+    pdf = 0.0f;
+    if (!lwi.z || !lwo.z || lwi.z <= 0.0f || lwo.z <= 0.0f) return;
+    f3 e;
+    ggx(lwi, lwo, e, pdf);
+    f = f + e;
   }
-  __device__ float metal_pdf(f3 wi, f3 wo) const {
-    if (fringe(wi) | fringe(wo)) return pdf_fringe(wi, wo);
-    const f3 lwi = normalize(to_local(s, wi)), lwo = normalize(to_local(s, wo));
-    if (!lwi.z || !lwo.z) return 0.0f;
-    float p = 0.0f;
-    if (!(lwi.z <= 0.0f || lwo.z <= 0.0f)) ggx(lwi, lwo, nullptr, &p);
-    return (1.0f * p) / 1.0f;
-  }
-  __device__ BsdfSample metal_sample(f3 wo, float u, float v, float w) const {
-    if (fringe(wo)) return sample_fringe(wo, u, v);
+  __device__ BsdfSample metal_sample(float u, float v, float w) const {
+    if (wo_fr) return sample_fringe(u, v);
     BsdfSample out;
     out.pdf = 0.0f;
     out.f = mk3(0.0f, 0.0f, 0.0f);
     out.wi = out.f;
-    const f3 lwo = normalize(to_local(s, wo));
     if (!lwo.z) return out;
     if (!((u - 0.001f) * 1.0f <= 1.0f)) return out;
     if (lwo.z <= 0.0f) return out;
@@ -775,12 +782,12 @@ struct Bsdf {
     if (lwi0.z <= 0.0f) return out;
     f3 f;
     float pdf = 0.0f;
-    ggx(lwi0, lwo, &f, &pdf);
+    ggx(lwi0, lwo, f, pdf);
     if (!(pdf > 0.0f)) return out;  // BXDFSampleResult::is_valid
     const f3 lwi = normalize(lwi0);
     const f3 wi = to_global(s, lwi);
     out.wi = wi;
-    out.f = muls(f, normal_correct(g, s, wi));
+    out.f = muls(f, normal_correct(wi));
     out.pdf = pdf * 1.0f;
     return out;
   }
@@ -796,67 +803,64 @@ struct Bsdf {
     sincosf(local_phi(lw), &sp, &cp);
     return smith_aniso_gtr2(cp, sp, ax, ay, local_tan_theta(lw));
   }
-  __device__ f3 d15_f_transmission(f3 lwi, f3 lwo) const {
+  // transmission's value (disney.cpp f_transmission) and density, sharing the half vector and D
+  __device__ void d15_transmission(f3 lwi, f3& f, float& pdf) const {
     const float eta = lwo.z > 0.0f ? m->ior : 1.0f / m->ior;
     f3 lwh = normalize(lwo + scale(lwi, eta));
     if (lwh.z < 0.0f) lwh = -lwh;
-    const float cd = dot(lwo, lwh);
+    const float cd = dot(lwo, lwh), ci = dot(lwi, lwh);
     const float F = dielectric_fresnel(m->ior, 1.0f, cd);
     const float D = d15_D(lwh, m->trans_ax, m->trans_ay);
     const float G = d15_G1(lwi, m->trans_ax, m->trans_ay) * d15_G1(lwo, m->trans_ax, m->trans_ay);
-    const float sdem = cd + eta * dot(lwi, lwh);
+    const float sdem = cd + eta * ci;
     const float corr = 1.0f / eta;
-    const float val = (1.0f - F) * D * G * eta * eta * dot(lwi, lwh) * dot(lwo, lwh) * corr * corr /
-                      (lwi.z * lwo.z * sdem * sdem);
+    const float val = (1.0f - F) * D * G * eta * eta * ci * cd * corr * corr / (lwi.z * lwo.z * sdem * sdem);
     const float k = (1.0f - m->metallic) * (lwo.z > 0.0f ? m->transmission : 1.0f);
     const float av = fabsf(val);
-    return mk3(k * sqrtf(m->base.x) * av, k * sqrtf(m->base.y) * av, k * sqrtf(m->base.z) * av);
+    f = mk3(k * sqrtf(m->base.x) * av, k * sqrtf(m->base.y) * av, k * sqrtf(m->base.z) * av);
+    pdf = 0.0f;
+    if (((lwo.z > 0.0f) != (cd > 0.0f)) || ((lwi.z > 0.0f) != (ci > 0.0f))) return;
+    const float dwh_to_dwi = eta * eta * ci / (sdem * sdem);
+    pdf = fabsf(ci * D * dwh_to_dwi);
   }
-  __device__ f3 d15_f_inner_reflection(f3 lwi, f3 lwo) const {
+  __device__ void d15_inner_reflection(f3 lwi, f3& f, float& pdf) const {
     const f3 lwh = -normalize(lwi + lwo);
     const float F = dielectric_fresnel(m->ior, 1.0f, dot(lwo, lwh));
     const float D = d15_D(lwh, m->trans_ax, m->trans_ay);
     const float G = d15_G1(lwi, m->trans_ax, m->trans_ay) * d15_G1(lwo, m->trans_ax, m->trans_ay);
-    return muls(muls(m->base, m->transmission), fabsf(F * D * G / (4.0f * lwi.z * lwo.z)));
+    f = muls(muls(m->base, m->transmission), fabsf(F * D * G / (4.0f * lwi.z * lwo.z)));
+    pdf = fabsf(lwh.z * D / (4.0f * dot(lwi, lwh)));
   }
-  __device__ f3 d15_f_specular(f3 lwi, f3 lwo) const {
-    const f3 lwh = normalize(lwi + lwo);
-    const float cd = dot(lwi, lwh);
-    const f3 one = mk3(1.0f, 1.0f, 1.0f);
-    const f3 Cspec = mix3(mix3(one, m->c_tint, m->specular_tint), m->base, m->metallic);
-    const f3 diel = muls(Cspec, dielectric_fresnel(m->ior, 1.0f, cd));
-    const f3 cond = Cspec + muls(one - Cspec, one_minus_5(cd));
-    const f3 F = mix3(mulc(m->spec_scale, diel), cond, m->metallic);
-    const float D = d15_D(lwh, m->ax, m->ay);
-    const float G = d15_G1(lwi, m->ax, m->ay) * d15_G1(lwo, m->ax, m->ay);
-    return divs(muls(muls(F, D), G), fabsf(4.0f * lwi.z * lwo.z));
-  }
-  __device__ float d15_pdf_transmission(f3 lwi, f3 lwo) const {
-    const float eta = lwo.z > 0.0f ? m->ior : 1.0f / m->ior;
-    f3 lwh = normalize(lwo + scale(lwi, eta));
-    if (lwh.z < 0.0f) lwh = -lwh;
-    if (((lwo.z > 0.0f) != (dot(lwh, lwo) > 0.0f)) || ((lwi.z > 0.0f) != (dot(lwh, lwi) > 0.0f))) return 0.0f;
-    const float sdem = dot(lwo, lwh) + eta * dot(lwi, lwh);
-    const float dwh_to_dwi = eta * eta * dot(lwi, lwh) / (sdem * sdem);
-    const float D = d15_D(lwh, m->trans_ax, m->trans_ay);
-    return fabsf(dot(lwi, lwh) * D * dwh_to_dwi);
-  }
-  __device__ float d15_pdf_inner_reflection(f3 lwi, f3 lwo) const {
-    const f3 lwh = -normalize(lwi + lwo);
-    const float D = d15_D(lwh, m->trans_ax, m->trans_ay);
-    return fabsf(lwh.z * D / (4.0f * dot(lwi, lwh)));
-  }
-  __device__ f3 d15_eval(f3 wi, f3 wo) const {
-    if (fringe(wi) | fringe(wo)) return eval_fringe(wi, wo);
-    const f3 lwi = normalize(to_local(s, wi)), lwo = normalize(to_local(s, wo));
-    if (fabsf(lwi.z) < kEps || fabsf(lwo.z) < kEps) return mk3(0.0f, 0.0f, 0.0f);
+  __device__ void d15_value(f3 wi, f3& f, float& pdf) const {
+    if (fringe(wi) | wo_fr) {
+      fringe_value(wi, f, pdf);
+      return;
+    }
+    f = mk3(0.0f, 0.0f, 0.0f);
+    pdf = 0.0f;
+    const f3 lwi = normalize(to_local(s, wi));
+    if (fabsf(lwi.z) < kEps || fabsf(lwo.z) < kEps) return;
     if (lwi.z * lwo.z < 0.0f) {
-      if (m->transmission == 0.0f) return mk3(0.0f, 0.0f, 0.0f);
-      return muls(d15_f_transmission(lwi, lwo), normal_correct(g, s, wi));
+      if (m->transmission == 0.0f) return;
+      d15_transmission(lwi, f, pdf);
+      f = muls(f, normal_correct(wi));
+      if (lwo.z < 0.0f) {
+        float F = dielectric_fresnel(m->ior, 1.0f, lwo.z);
+        F = F < 0.1f ? 0.1f : (0.9f < F ? 0.9f : F);
+        pdf = (1.0f - F) * pdf;
+      } else {
+        pdf = m->w_trans * pdf;
+      }
+      return;
     }
     if (lwi.z < 0.0f && lwo.z < 0.0f) {
-      if (m->transmission == 0.0f) return mk3(0.0f, 0.0f, 0.0f);
-      return muls(d15_f_inner_reflection(lwi, lwo), normal_correct(g, s, wi));
+      if (m->transmission == 0.0f) return;
+      d15_inner_reflection(lwi, f, pdf);
+      f = muls(f, normal_correct(wi));
+      float F = dielectric_fresnel(m->ior, 1.0f, lwo.z);
+      F = F < 0.1f ? 0.1f : (0.9f < F ? 0.9f : F);
+      pdf = F * pdf;
+      return;
     }
     const f3 lwh = normalize(lwi + lwo);
     const float cd = dot(lwi, lwh);
@@ -871,48 +875,41 @@ struct Bsdf {
       if (m->sheen > 0.0f)
         sheen = muls(muls(mix3(mk3(1.0f, 1.0f, 1.0f), m->c_tint, m->sheen_tint), 4.0f * m->sheen), one_minus_5(cd));
     }
-    const f3 specular = d15_f_specular(lwi, lwo);
+    // f_specular
+    const f3 one = mk3(1.0f, 1.0f, 1.0f);
+    const f3 Cspec = mix3(mix3(one, m->c_tint, m->specular_tint), m->base, m->metallic);
+    const f3 diel = muls(Cspec, dielectric_fresnel(m->ior, 1.0f, cd));
+    const f3 cond = Cspec + muls(one - Cspec, one_minus_5(cd));
+    const f3 Fsp = mix3(mulc(m->spec_scale, diel), cond, m->metallic);
+    const float Dsp = d15_D(lwh, m->ax, m->ay);
+    const float phi_o = local_phi(lwo), tan_i = local_tan_theta(lwi), tan_o = local_tan_theta(lwo);
+    float spo, cpo;
+    sincosf(phi_o, &spo, &cpo);
+    const float Gsp = d15_G1(lwi, m->ax, m->ay) * smith_aniso_gtr2(cpo, spo, m->ax, m->ay, tan_o);
+    const f3 specular = divs(muls(muls(Fsp, Dsp), Gsp), fabsf(4.0f * lwi.z * lwo.z));
+    const float ch = lwh.z, sh = local_cos_to_sin(ch);
+    const float Dcc = gtr1(sh, ch, m->cc_rough);
     if (m->clearcoat > 0.0f) {
-      const float ch = lwh.z, sh = local_cos_to_sin(ch);
-      const float D = gtr1(sh, ch, m->cc_rough);
       const float F = 0.04f + (1.0f - 0.04f) * one_minus_5(cd);
-      const float G = smith_gtr2(local_tan_theta(lwi), 0.25f) * smith_gtr2(local_tan_theta(lwo), 0.25f);
-      const float c = m->clearcoat * D * F * G / fabsf(4.0f * lwi.z * lwo.z);
+      const float G = smith_gtr2(tan_i, 0.25f) * smith_gtr2(tan_o, 0.25f);
+      const float c = m->clearcoat * Dcc * F * G / fabsf(4.0f * lwi.z * lwo.z);
       clearcoat = mk3(c, c, c);
     }
     const f3 ret = muls(diffuse + sheen, (1.0f - m->metallic) * (1.0f - m->transmission)) + specular + clearcoat;
-    return muls(ret, normal_correct(g, s, wi));
-  }
-  __device__ float d15_pdf(f3 wi, f3 wo) const {
-    if (fringe(wi) | fringe(wo)) return pdf_fringe(wi, wo);
-    const f3 lwi = normalize(to_local(s, wi)), lwo = normalize(to_local(s, wo));
-    if (fabsf(lwi.z) < kEps || fabsf(lwo.z) < kEps) return 0.0f;
-    if (lwo.z < 0.0f) {
-      if (m->transmission == 0.0f) return 0.0f;
-      float F = dielectric_fresnel(m->ior, 1.0f, lwo.z);
-      F = F < 0.1f ? 0.1f : (0.9f < F ? 0.9f : F);
-      if (lwi.z > 0.0f) return (1.0f - F) * d15_pdf_transmission(lwi, lwo);
-      return F * d15_pdf_inner_reflection(lwi, lwo);
-    }
-    if (lwi.z < 0.0f) return m->w_trans * d15_pdf_transmission(lwi, lwo);
+    f = muls(ret, normal_correct(wi));
     // pdf_specular_clearcoat (disney.cpp:250-281): sin(phi_o) from cos(phi_o)
-    const f3 lwh = normalize(lwi + lwo);
-    const float ch = lwh.z, sh = local_cos_to_sin(ch);
-    const float cd = dot(lwi, lwh);
-    const float cos_phi_o = cosf(local_phi(lwo));
+    const float cos_phi_o = cosf(phi_o);
     const float sin_phi_o = local_cos_to_sin(cos_phi_o);
-    const float ps = smith_aniso_gtr2(cos_phi_o, sin_phi_o, m->ax, m->ay, local_tan_theta(lwo)) *
-                     d15_D(lwh, m->ax, m->ay) / (4.0f * lwo.z);
-    const float pc = ch * gtr1(sh, ch, m->cc_rough) / (4.0f * cd);
-    return m->w_diff15 * cosine_pdf(lwi.z) + m->w_spec15 * ps + m->w_cc * pc;
+    const float ps = smith_aniso_gtr2(cos_phi_o, sin_phi_o, m->ax, m->ay, tan_o) * Dsp / (4.0f * lwo.z);
+    const float pc = ch * Dcc / (4.0f * cd);
+    pdf = m->w_diff15 * cosine_pdf(lwi.z) + m->w_spec15 * ps + m->w_cc * pc;
   }
-  __device__ BsdfSample d15_sample(f3 wo, float u, float v, float w) const {
-    if (fringe(wo)) return sample_fringe(wo, u, v);
+  __device__ BsdfSample d15_sample(float u, float v, float w) const {
+    if (wo_fr) return sample_fringe(u, v);
     BsdfSample out;
     out.pdf = 0.0f;
     out.f = mk3(0.0f, 0.0f, 0.0f);
     out.wi = out.f;
-    const f3 lwo = normalize(to_local(s, wo));
     if (fabsf(lwo.z) < kEps) return out;
     if (lwo.z < 0.0f && m->transmission == 0.0f) return out;
     // the lobe choice (disney.cpp:471-488): the second test is not inside the
@@ -949,28 +946,8 @@ struct Bsdf {
     }
     if (lwi.x == 0.0f && lwi.y == 0.0f && lwi.z == 0.0f) return out;
     out.wi = to_global(s, lwi);
-    out.f = d15_eval(out.wi, wo);
-    out.pdf = d15_pdf(out.wi, wo);
+    d15_value(out.wi, out.f, out.pdf);
     return out;
-  }
-
-  __device__ __forceinline__ f3 eval(f3 wi, f3 wo) const {
-    if (m->kind == MAT_GLASS) return mk3(0.0f, 0.0f, 0.0f);
-    if (m->kind == MAT_METAL) return metal_eval(wi, wo);
-    if (m->kind == MAT_DISNEY15) return d15_eval(wi, wo);
-    return m->kind == MAT_PHONG ? phong_eval_agg(wi, wo) : disney_eval(wi, wo);
-  }
-  __device__ __forceinline__ float pdf(f3 wi, f3 wo) const {
-    if (m->kind == MAT_GLASS) return 0.0f;
-    if (m->kind == MAT_METAL) return metal_pdf(wi, wo);
-    if (m->kind == MAT_DISNEY15) return d15_pdf(wi, wo);
-    return m->kind == MAT_PHONG ? phong_pdf_agg(wi, wo) : disney_pdf(wi, wo);
-  }
-  __device__ __forceinline__ BsdfSample sample(f3 wo, float u, float v, float w) const {
-    if (m->kind == MAT_GLASS) return glass_sample(wo, u);
-    if (m->kind == MAT_METAL) return metal_sample(wo, u, v, w);
-    if (m->kind == MAT_DISNEY15) return d15_sample(wo, u, v, w);
-    return m->kind == MAT_PHONG ? phong_sample_agg(wo, u, v, w) : disney_sample(wo, u, v, w);
   }
 };
 
