@@ -4,24 +4,32 @@
 // PixelSamplerRenderer::render (src/renderer/pixel_sampler_renderer.cpp:24-109)
 // calls PathTraceRenderer::eval_pixel_li (src/renderer/path_trace_renderer.cpp:27-210)
 // once per camera sample, the samples of a pixel in order from one pcg32
-// stream. Here a thread owns a pixel (a path slot) at a time and runs its
-// samples one after another with the whole path state in registers; when the
+// stream. Here a lane owns a pixel (a path slot) at a time and runs its
+// samples one after another with the path state in registers; when the
 // pixel's samples are done it claims the next unrendered pixel of any job
 // (one atomic per warp). Each loop iteration processes one path vertex of
-// every lane of a warp, in phases the 32 lanes go through together:
+// every owning lane, in phases:
 //
-//   extend   closest hit of every lane's ray (warp-cooperative traversal)
-//   vertex   emission, escape to the environment light, BSDF sample, the
-//            light-sample draws, the MIS sample, throughput, Russian roulette
-//   lights   for each light index: the light sample and its shadow ray
-//   mis      closest hit of the MIS ray and its weighted emission
-//   finish   direct lighting added, the sample's film update, the next sample
+//   trace    every ray of the warp's pool: shadow rays, MIS rays and the
+//            continuation or camera rays of the owners' next vertices
+//   finish   the vertex's direct lighting, film updates of ended samples
+//   vertex   emission, escape to the environment light, BSDF sample, the MIS
+//            sample, throughput, Russian roulette, the next ray
+//   lights   light samples of the warp's vertices, dealt out over all lanes
+//
+// All random draws of a vertex happen in its vertex phase, so the rays of its
+// light samples and MIS sample and the path's next ray are independent, and
+// so is the next sample's camera ray when the path ends there: they are traced
+// together, any lane walking any ray, and the lights phase likewise takes
+// (vertex, light) pairs from a dense list. One walk and one light evaluation
+// per vertex are then on a path's serial chain instead of one per light, and
+// lanes whose vertex has fewer rays do not idle.
 //
 // The arithmetic, the order of random draws and the order of the sums are
 // those of the wavefront kernels of render.cu (k_logic, k_material, k_glass,
 // k_nee, mis_contribution), so a pixel gets the same film bit for bit either
 // way; only the work is arranged for small renders, where the wavefront's
-// ten launches per path vertex over a few thousand slots cannot fill the GPU.
+// launches per path vertex over a few thousand slots cannot fill the GPU.
 // Guided rendering and instrumented renders (stage times, visit counts) use
 // the wavefront.
 
@@ -38,45 +46,91 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 
-// What a trace gives back: the hit record (any hit: the occluding slot in
-// prim) and whether the ray is occluded.
-struct Traced {
-  Hit h;
-  bool occluded;
-};
+// A warp's ray pool in shared memory, three float4 per ray:
+//   a: origin, t_max
+//   b: direction, who (owner lane | kind << 5 | light << 7 | scene << 12)
+//   c: shadow rays: the light sample's contribution | the remembered occluder's
+//      slot (-1: none), after the walk kBlocked | the occluding slot if blocked;
+//      others, after the walk: t_attr, alpha, beta | primitive (-1: miss)
+// Continuation and MIS rays lie at the front and stay for the iteration;
+// shadow rays follow, walked in several rounds if they do not fit at once.
+constexpr int kPool = 128;
+constexpr size_t kPoolBytes = 3 * kPool * sizeof(float4);
+constexpr int kBlocked = 1 << 30;
+enum : int { RAY_NEXT = 0, RAY_MIS = 1, RAY_SHADOW = 2 };
+__device__ __forceinline__ int who_of(int owner, int kind, int light, int scene) {
+  return owner | kind << 5 | light << 7 | scene << 12;
+}
 
-// Closest hit (ANY = false) or occlusion (ANY = true) of every lane's ray,
-// the 32 lanes walking together: the speculative while-while of
-// persistent_traverse without its refill. Lanes with `active` false take no
-// part in the walk; every lane of the warp must call it. Out of line: one
-// copy serves the extension and the MIS ray; the walk's state is local to the
-// call (registers, its stack in local memory).
-template <bool ANY>
-__device__ __noinline__ Traced warp_trace(const DScene& sc, bool active, int scene, f3 o, f3 d, float tmin,
-                                          float tmax, int* err) {
-  TravLane<ANY, false> L;
+// Walks rays [from, n) of the pool: the speculative while-while of
+// persistent_traverse, closest-hit and any-hit rays side by side, finished
+// lanes taking the next ray once fewer than kPoolRefill walk. Every lane of
+// the warp calls it. Returns this lane's count of rays answered by their
+// remembered occluder.
+constexpr int kPoolRefill = 24;
+__device__ __noinline__ unsigned int pool_trace(const DScene& sc, float4* pool, int from, int n, int cache, int* err) {
+  float4 *pa = pool, *pb = pool + kPool, *pc = pool + 2 * kPool;
+  const unsigned int below = (1u << (threadIdx.x & 31u)) - 1u;
+  TravLane<false, false, false, true> L;
   VisitCount vc;
-  bool live = active && L.start(sc, scene, o, d, tmin, tmax, vc, false);
-  if (!active) {
-    L.h.prim = -1;
-    L.occluded = false;
-  }
+  bool live = false;
+  int ray = -1, next = from;
+  unsigned int hits = 0;
+  __syncwarp();
   for (;;) {
-    for (;;) {
-      if (live && L.cnt > 0 && L.pc == 0) L.postpone();
-      if (!__any_sync(kFull, live && L.pc == 0)) break;
-      if (live && L.cnt == 0) {
-        const bool more = L.interior(sc, err, vc);
-        if (!more) {
-          if (L.failed || L.pc == 0) live = false;
-          else L.cnt = -1;
+    const unsigned int idle = __ballot_sync(kFull, !live);
+    if (next < n) {
+      const int mine = next + __popc(idle & below);
+      next += __popc(idle);
+      if (!live && mine < n) {
+        ray = mine;
+        const float4 a = pa[ray], b = pb[ray];
+        const int who = __float_as_int(b.w), scene = who >> 12;
+        const f3 o = mk3(a.x, a.y, a.z), d = mk3(b.x, b.y, b.z);
+        L.any = ((who >> 5) & 3) == RAY_SHADOW;
+        const float t_min = L.any ? kEps : 0.0f;
+        const int oc = L.any && cache ? __float_as_int(pc[ray].w) : -1;
+        if (oc >= 0 && occluded_by_slot(sc, scene, oc, o, d, t_min, a.w)) {
+          pc[ray].w = __int_as_float(kBlocked | oc);
+          ++hits;
+        } else {
+          live = L.start(sc, scene, o, d, t_min, a.w, vc, false);
+          if (!live && !L.any) pc[ray] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(-1));
         }
       }
+    } else if (idle == kFull) {
+      break;
     }
-    if (live) live = L.postponed_leaf(sc, vc);
-    if (!__any_sync(kFull, live)) break;
+    if (!__any_sync(kFull, live)) continue;
+    for (;;) {
+      for (;;) {
+        if (live && L.cnt > 0 && L.pc == 0) L.postpone();
+        if (!__any_sync(kFull, live && L.pc == 0)) break;
+        bool ended = false;
+        if (live && L.cnt == 0) {
+          if (!L.interior(sc, err, vc)) {
+            if (L.failed || L.pc == 0) ended = true;
+            else L.cnt = -1;
+          }
+        }
+        if (ended) {
+          live = false;
+          if (!L.any) pc[ray] = make_float4(L.h.t_attr, L.h.alpha, L.h.beta, __int_as_float(L.h.prim));
+        }
+      }
+      if (live) {
+        live = L.postponed_leaf(sc, vc);
+        if (!live) {
+          if (!L.any) pc[ray] = make_float4(L.h.t_attr, L.h.alpha, L.h.beta, __int_as_float(L.h.prim));
+          else if (L.occluded) pc[ray].w = __int_as_float(kBlocked | L.h.prim);
+        }
+      }
+      const int walking = __popc(__ballot_sync(kFull, live));
+      if (walking == 0 || (walking < kPoolRefill && next < n)) break;
+    }
   }
-  return Traced{L.h, L.occluded};
+  __syncwarp();
+  return hits;
 }
 
 // Material dispatch limited to the kinds of the instantiation (the sampler
@@ -103,7 +157,7 @@ struct Path {
   unsigned long long st;
   int sample, depth, sdepth;
   bool spec;      // the ray continues a delta sample (emission it reaches counts)
-  bool has_ray;   // a ray to extend this iteration
+  bool has_ray;   // the path has a next ray
   f3 o, d, coef, L;
   float px, py;
   unsigned int finished;
@@ -148,34 +202,96 @@ __device__ __forceinline__ bool start_sample(Path& p) {
   return false;
 }
 
-// finish_sample of render.cu: the film update and the next sample.
-__device__ __forceinline__ void finish_sample(Path& p) {
-  f3 L = p.L;
-  if (!valid3(L)) L = mk3(0.0f, 0.0f, 0.0f);  // eval_pixel_li returns {} (path_trace_renderer.cpp:204-209)
-  film_add(*p.J, p.slot, p.px, p.py, L);
-  ++p.finished;
-  ++p.sample;
-  p.has_ray = start_sample(p);
+__device__ __forceinline__ f3 film_value(f3 L) {
+  return valid3(L) ? L : mk3(0.0f, 0.0f, 0.0f);  // eval_pixel_li returns {} (path_trace_renderer.cpp:204-209)
+}
+
+__device__ __forceinline__ f3 shfl3(f3 v, int src) {
+  return mk3(__shfl_sync(kFull, v.x, src), __shfl_sync(kFull, v.y, src), __shfl_sync(kFull, v.z, src));
+}
+__device__ __forceinline__ unsigned long long shfl64(unsigned long long v, int src) {
+  const unsigned int lo = __shfl_sync(kFull, (unsigned int)v, src), hi = __shfl_sync(kFull, (unsigned int)(v >> 32), src);
+  return (unsigned long long)hi << 32 | lo;
+}
+
+// One (vertex, light) pair (k_nee): the light sample of light `l` at pos, its
+// contribution cc and shadow ray sd, dist. Returns whether there is one.
+template <unsigned MASK>
+__device__ __forceinline__ bool light_item(const DScene& sc, const DLight& lt, const Bsdf& bsdf, int kind, f3 pos,
+                                           f3 coef, float2 uv, f3& cc, f3& sd, float& dist) {
+  f3 to_light, Le;
+  float lpdf;
+  if ((MASK & MK_ENV) && lt.env >= 0) {
+    // sample_environment_light (src/renderer/direct_illumination.cpp:73-106)
+    f3 lpos;
+    if (!env_sample(sc.envs[lt.env], pos, uv.x, uv.y, Le, lpdf, lpos) || black(Le)) return false;
+    to_light = lpos - pos;
+  } else {
+    // sample_area_light (src/renderer/direct_illumination.cpp:35-71) via
+    // UniformSampleTriangle (src/shape/triangle.cpp:61-97)
+    const float su0 = sqrtf(uv.x);
+    const float bx = 1.0f - su0, by = uv.y * su0;
+    const f3 lpos = scale(lt.A, bx) + scale(lt.B, by) + scale(lt.C, 1.0f - bx - by);
+    const f3 sp2ref = pos - lpos;
+    if (!(dot(lt.gz, sp2ref) > 0.0f)) return false;
+    const float dist2 = len2f(sp2ref);
+    lpdf = area_to_solid_pdf(lt.area_pdf * dist2, dot(lt.gz, sp2ref), dist2);
+    if (!lpdf) return false;
+    to_light = lpos - pos;
+    Le = lt.emission;
+  }
+  bool too_close;
+  dist = dist_minus_eps(len2f(to_light), too_close);
+  if (too_close) return false;
+  to_light = normalize(to_light);
+  f3 bf;
+  float bpdf;
+  m_value<MASK>(bsdf, kind, to_light, bf, bpdf);
+  if (black(bf)) return false;
+  const f3 fl = muls(mulc(Le, bf), abs_cos(to_light, bsdf.g.z));
+  const float w = power_heuristic(lpdf, bpdf);
+  cc = mulc(coef, divs(muls(fl, w), lpdf));
+  sd = normalize(to_light);
+  return true;
 }
 
 template <unsigned MASK>
 __global__ void __launch_bounds__(kMegaThreads, 1) k_mega(MegaLaunch P) {
+  extern __shared__ float4 pools[];
   const DScene& sc = P.sc;
   const int lane = (int)(threadIdx.x & 31u);
+  const unsigned int below = (1u << lane) - 1u;
+  float4* pool = pools + (threadIdx.x >> 5) * (3 * kPool);
+  float4 *pa = pool, *pb = pool + kPool, *pc = pool + 2 * kPool;
+  DMat* const tmat = (MASK & MK_MAPS) ? P.mt + (size_t)blockIdx.x * blockDim.x + threadIdx.x : nullptr;
   Path p;
   p.slot = -1;
   p.has_ray = false;
   p.finished = 0;
-  bool done = false;
+  bool done = lane >= P.lanes;
   long long steps = 0, max_steps = 0;  // vertex bound of the current pixel
-  float2 nu[kMegaLights];              // light-sample draws of the current vertex
   int oc[kMegaLights];                 // the slot that last blocked each light's shadow ray (-1: none)
-  DMat tmat;                           // the Phong set-up at a hit with image maps
   unsigned long long n_ext = 0, n_sh = 0, n_vert = 0, n_hits = 0;
+  // the vertex whose light is being gathered: what its light samples need,
+  // its MIS ray, and the sample that ends with it (its film update is due
+  // once its direct lighting is known)
+  Isect is;
+  Bsdf bsdf;
+  int kind = 0, mcode = 0, scene = 0, light_base = 0, env = -1;
+  unsigned int nee_mask = 0;
+  unsigned long long st_lights = 0;  // the stream before the light samples' draws
+  f3 coef_prev = mk3(0.0f, 0.0f, 0.0f), mo = coef_prev, md = coef_prev, mf = coef_prev;
+  float mpdf = 0.0f, mcos = 0.0f;
+  bool vertex = false, mis = false, mis_trace = false;
+  bool due = false, restart = false;  // a film update is due; the next sample starts after it
+  f3 due_L = coef_prev;
+  float due_x = 0.0f, due_y = 0.0f;
+  int due_slot = 0;
+  const JobDev* due_J = nullptr;
   for (;;) {
-    // lanes without a ray claim pixels until they have one or none are left
+    // owners without a ray claim pixels until they have one or none are left
     for (;;) {
-      const bool want = !done && !p.has_ray;
+      const bool want = !done && !p.has_ray && !restart;
       const unsigned need = __ballot_sync(kFull, want);
       if (!need) break;
       const int leader = __ffs(need) - 1;
@@ -183,7 +299,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_mega(MegaLaunch P) {
       if (lane == leader) base = atomicAdd(P.fetch, (unsigned int)__popc(need));
       base = __shfl_sync(kFull, base, leader);
       if (want) {
-        const unsigned int s = base + (unsigned int)__popc(need & ((1u << lane) - 1u));
+        const unsigned int s = base + (unsigned int)__popc(need & below);
         if (s < (unsigned int)P.nslots) {
           p.slot = (int)s;
           p.J = &job_of(P.jobs, P.njobs, p.slot);
@@ -200,34 +316,177 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_mega(MegaLaunch P) {
         }
       }
     }
-    // the block goes through the phases together (one phase's code in the
-    // instruction cache at a time); it ends when all its lanes are done
-    if (!__syncthreads_or(!done)) break;
-
-    // ---- extend: closest hit of the continuation or camera ray (k_extend)
-    const int scene = p.has_ray ? p.J->scene : 0;
-    const Traced ext = warp_trace<false>(sc, p.has_ray, scene, p.o, p.d, 0.0f, kRealMax, P.err);
-    n_ext += p.has_ray;
-
-    __syncthreads();
-    // ---- vertex (k_logic, then k_material / k_glass)
-    bool vertex = false, term = false, mis = false, mis_trace = false;
-    bool ended = false;  // the sample ended at this hit without direct lighting
-    int kind = 0, mcode = 0;
-    Isect is;
-    f3 coef_prev = mk3(0.0f, 0.0f, 0.0f);
-    f3 mo = coef_prev, md = coef_prev, mf = coef_prev;
-    float mpdf = 0.0f, mcos = 0.0f;
-    unsigned int nee_mask = 0;
+    // the pool's front: the owners' next rays, then their MIS rays
+    const unsigned int m_next = __ballot_sync(kFull, p.has_ray), m_mis = __ballot_sync(kFull, mis_trace);
+    const int i_next = __popc(m_next & below), i_mis = __popc(m_next) + __popc(m_mis & below);
+    const int front = __popc(m_next) + __popc(m_mis);
     if (p.has_ray) {
+      pa[i_next] = make_float4(p.o.x, p.o.y, p.o.z, kRealMax);
+      pb[i_next] = make_float4(p.d.x, p.d.y, p.d.z, __int_as_float(who_of(lane, RAY_NEXT, 0, p.J->scene)));
+    }
+    if (mis_trace) {
+      pa[i_mis] = make_float4(mo.x, mo.y, mo.z, kRealMax);
+      pb[i_mis] = make_float4(md.x, md.y, md.z, __int_as_float(who_of(lane, RAY_MIS, 0, scene)));
+    }
+    n_ext += (p.has_ray ? 1 : 0) + (mis_trace ? 1 : 0);
+    // the block goes through the phases together: one phase's code in the
+    // instruction cache at a time (free-running warps took 2.8 times as long
+    // on a 256x256x16 Cornell box)
+    __syncthreads();
+
+    // ---- lights: the (vertex, light) pairs of the warp, 32 at a time
+    f3 direct = mk3(0.0f, 0.0f, 0.0f);
+    int n_items = __popc(nee_mask), first_item = n_items;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int y = __shfl_up_sync(kFull, first_item, off);
+      if (lane >= off) first_item += y;
+    }
+    const int items = __shfl_sync(kFull, first_item, 31);
+    first_item -= n_items;
+    int n = front, traced = 0, mine = 0, n_mine = 0;  // mine, n_mine: this owner's shadow rays in the pool
+    for (int c0 = 0;; c0 += 32) {
+      bool ray = false;
+      f3 cc, sd, pos;
+      float dist = 0.0f;
+      int owner = 0, l = 0, osc = 0;
+      if (c0 < items) {
+        // lane k takes pair c0 + k; its owner is the last lane whose pairs
+        // start at or before it (a lane without pairs starts where the next does)
+        const int it = c0 + lane;
+        for (int step = 16; step > 0; step >>= 1)
+          if (__shfl_sync(kFull, first_item, owner + step) <= it) owner += step;
+        const int start = __shfl_sync(kFull, first_item, owner);
+        unsigned int mask = __shfl_sync(kFull, nee_mask, owner);
+        const bool on = it < items;
+        for (int k = it - start; on && k > 0; --k) mask &= mask - 1u;
+        l = on ? __ffs((int)mask) - 1 : 0;
+        unsigned long long st = shfl64(st_lights, owner);
+        pos = shfl3(is.pos, owner);
+        Bsdf b;
+        b.g.x = shfl3(bsdf.g.x, owner);
+        b.g.y = shfl3(bsdf.g.y, owner);
+        b.g.z = shfl3(bsdf.g.z, owner);
+        b.s.x = shfl3(bsdf.s.x, owner);
+        b.s.y = shfl3(bsdf.s.y, owner);
+        b.s.z = shfl3(bsdf.s.z, owner);
+        b.lwo = shfl3(bsdf.lwo, owner);
+        const int bits = __shfl_sync(kFull, (bsdf.wo_g ? 1 : 0) | (bsdf.wo_fr ? 2 : 0) | (bsdf.same_n ? 4 : 0) | kind << 3, owner);
+        b.wo_g = bits & 1;
+        b.wo_fr = bits & 2;
+        b.same_n = bits & 4;
+        const int mc = __shfl_sync(kFull, mcode, owner);
+        const f3 coef = shfl3(coef_prev, owner);
+        const int lb = __shfl_sync(kFull, light_base, owner);
+        osc = __shfl_sync(kFull, scene, owner);
+        if (on) {
+          b.m = (MASK & MK_MAPS) && mc < 0 ? tmat + (owner - lane) : sc.mats + mc;
+          for (int k = 0; k < l; ++k) Pcg::skip<5>(st);  // five draws a light, the first two place the sample
+          const float u = Pcg::next(st), v = Pcg::next(st);
+          ray = light_item<MASK>(sc, sc.lights[lb + l], b, bits >> 3, pos, coef, make_float2(u, v), cc, sd, dist);
+        }
+      }
+      const unsigned int m_ray = __ballot_sync(kFull, ray);
+      n_sh += ray;
+      if (ray) {
+        const int e = n + __popc(m_ray & below);
+        pa[e] = make_float4(pos.x, pos.y, pos.z, dist);
+        pb[e] = make_float4(sd.x, sd.y, sd.z, __int_as_float(who_of(owner, RAY_SHADOW, l, osc)));
+        pc[e] = make_float4(cc.x, cc.y, cc.z, __int_as_float(-1));
+      }
+      __syncwarp();
+      {
+        // the owner's share of this round: pairs [lo, hi) of the chunk
+        const int lo = min(max(first_item - c0, 0), 32), hi = min(max(first_item + n_items - c0, 0), 32);
+        const unsigned int below_lo = lo >= 32 ? kFull : (1u << lo) - 1u, below_hi = hi >= 32 ? kFull : (1u << hi) - 1u;
+        if (n_mine == 0) mine = n + __popc(m_ray & below_lo);
+        const int k0 = n + __popc(m_ray & below_lo), k1 = n + __popc(m_ray & below_hi);
+        for (int e = k0; e < k1; ++e)  // the light's last occluder is the owner's to know
+          pc[e].w = __int_as_float(oc[(__float_as_int(pb[e].w) >> 7) & 31]);
+        n_mine += k1 - k0;
+      }
+      n += __popc(m_ray);
+      // the last round, or a full pool: walk it and add the shadow rays' answers
+      const bool more = c0 + 32 < items;
+      if (!more || n + 32 > kPool) {
+        if (!more) __syncthreads();
+        // ---- trace (k_extend, k_shadow)
+        n_hits += pool_trace(sc, pool, traced, n, P.occluder_cache && sc.slot_leaf, P.err);
+        for (int e = mine; e < mine + n_mine; ++e) {
+          const float4 c = pc[e];
+          const int w = __float_as_int(c.w);
+          if (w >= 0 && (w & kBlocked)) oc[(__float_as_int(pb[e].w) >> 7) & 31] = w & ~kBlocked;
+          else direct = direct + mk3(c.x, c.y, c.z);
+        }
+        __syncwarp();
+        n = traced = front;
+        n_mine = 0;
+      }
+      if (!more) break;
+    }
+
+    // ---- finish: the MIS ray's emission, weighted against the light
+    //      (mis_contribution of render.cu, direct_illumination.cpp:144-198), the
+    //      vertex's direct lighting, the film update of a sample that ended
+    if (mis) {
+      float4 mh = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(-1));
+      if (mis_trace) mh = pc[i_mis];  // a ray that can reach no light is not traced: its closest hit would give zero
+      const int pid = __float_as_int(mh.w);
+      f3 c = mk3(0.0f, 0.0f, 0.0f);
+      if (pid < 0) {
+        if ((MASK & MK_ENV) && env >= 0) {
+          const DEnv& e = sc.envs[env];
+          const f3 Le = env_emit(e, md);
+          if (!black(Le)) {
+            const f3 f = muls(mulc(Le, mf), mcos);
+            const float w = power_heuristic(mpdf, env_pdf(e, md));
+            c = divs(muls(f, w), mpdf);
+          }
+        }
+      } else {
+        const DPrim& pr = sc.prims[pid];
+        if (pr.emissive) {
+          const f3 gz = sc.tshade[pr.shape].gz;
+          if (dot(gz, -md) > 0.0f) {
+            const f3 f = muls(mulc(pr.emission, mf), mcos);
+            const f3 pos = mo + scale(md, mh.x);
+            const float lpdf = light_pdf_at(pr.area, mo, pos, gz);
+            const float w = power_heuristic(mpdf, lpdf);
+            c = divs(muls(f, w), mpdf);
+          }
+        }
+      }
+      direct = direct + mulc(coef_prev, c);
+    }
+    if (vertex) {
+      if (due) film_add(*due_J, due_slot, due_x, due_y, film_value(due_L + direct));
+      else p.L = p.L + direct;
+    }
+    vertex = mis = mis_trace = due = false;
+    nee_mask = 0;
+    float4 hit = make_float4(__int_as_float(-1), 0.0f, 0.0f, 0.0f);
+    const bool arrived = p.has_ray;  // the next ray's hit is known
+    if (arrived) {
+      const float4 c = pc[i_next];
+      hit = make_float4(c.w, c.x, c.y, c.z);
+    }
+    if (restart) {
+      restart = false;
+      p.has_ray = start_sample(p);
+    }
+    if (!__syncthreads_or(arrived || p.has_ray || !done)) break;
+
+    // ---- vertex (k_logic, then k_material / k_glass)
+    if (arrived) {
+      bool ended = false;  // the sample ended at this hit without direct lighting
+      bool term = false;
       ++n_vert;
+      p.has_ray = false;
       if (++steps > max_steps) {
         atomicOr(P.err, 2);
-        p.has_ray = false;
         p.slot = -1;
       } else {
-        const int pid = ext.h.prim;
-        const float4 hit = make_float4(__int_as_float(pid), ext.h.t_attr, ext.h.alpha, ext.h.beta);
+        const int pid = __float_as_int(hit.x);
         if (pid < 0) {
           // a camera ray or one after a delta sample left the scene: the
           // environment light's radiance along it (path_trace_renderer.cpp:66-81)
@@ -243,14 +502,13 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_mega(MegaLaunch P) {
           }
           kind = sc.mats[pr.material].kind;
           make_isect(sc, hit, p.o, p.d, is);
-          Bsdf bsdf;
           mcode = pr.material;
           bsdf.m = sc.mats + mcode;
           if ((MASK & MK_MAPS) && bsdf.m->tex_any) {  // image maps: the material at this hit's uv
             float u, v;
             hit_uv(sc, hit, p.o, p.d, u, v);
-            material_at(sc, pr.material, u, v, &tmat);
-            bsdf.m = &tmat;
+            material_at(sc, pr.material, u, v, tmat);
+            bsdf.m = tmat;
             mcode = -1;
           }
           bsdf.g = is.g;
@@ -286,6 +544,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_mega(MegaLaunch P) {
               p.o = is.eps_offset(bs.wi);
               p.d = normalize(normalize(bs.wi));
               p.spec = true;
+              p.has_ray = true;
             }
           } else {
             const float u0 = Pcg::next(p.st), u1 = Pcg::next(p.st), u2 = Pcg::next(p.st);
@@ -294,23 +553,22 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_mega(MegaLaunch P) {
               ended = true;
             } else {
               vertex = true;
-              // next-event estimation draws on every light (sample_area_light)
+              // next-event estimation draws on every light (sample_area_light):
+              // five each, taken in the lights phase from here on
               const JobDev& J = *p.J;
+              st_lights = p.st;
+              scene = J.scene;
+              light_base = J.light_base;
+              env = J.env;
               const float pos_mag = fabsf(is.pos.x) + fabsf(is.pos.y) + fabsf(is.pos.z);
               for (int l = 0; l < J.nl; ++l) {
                 // a vertex well behind a light's plane gets nothing from it
-                // (k_material's skip: its five draws only advance the stream)
+                // (k_material's skip)
                 const DLight& lt = sc.lights[J.light_base + l];
                 const float side = dot(lt.gz, is.pos - lt.A);
                 const float tol = 1e-4f * (pos_mag + lt.extent);
-                if (side < -tol) {
-                  Pcg::skip<5>(p.st);
-                  continue;
-                }
-                const float lu = Pcg::next(p.st), lv = Pcg::next(p.st);
-                Pcg::skip<3>(p.st);
-                nu[l] = make_float2(lu, lv);
-                nee_mask |= 1u << l;
+                Pcg::skip<5>(p.st);
+                if (!(side < -tol)) nee_mask |= 1u << l;
               }
               // the MIS BSDF ray (sample_bsdf, src/renderer/direct_illumination.cpp:144-155)
               const float v0 = Pcg::next(p.st), v1 = Pcg::next(p.st), v2 = Pcg::next(p.st);
@@ -344,156 +602,30 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_mega(MegaLaunch P) {
                 p.o = is.eps_offset(bs.wi);
                 p.d = normalize(normalize(bs.wi));
                 p.spec = false;
+                p.has_ray = true;
               }
             }
           }
         }
-      }
-    }
-
-    __syncthreads();
-    // ---- lights: the light sample and its shadow ray per light (k_nee, k_shadow)
-    f3 direct = mk3(0.0f, 0.0f, 0.0f);
-    Bsdf bsdf;
-    bsdf.m = mcode >= 0 ? sc.mats + mcode : &tmat;
-    bsdf.g = is.g;
-    bsdf.s = is.s;
-    if (vertex) bsdf.look_from(is.wo);
-    for (int l = 0; l < P.nl_max; ++l) {
-      bool trace = false;
-      f3 cc = mk3(0.0f, 0.0f, 0.0f), so = cc, sd = cc;
-      float dist = 0.0f;
-      if (vertex && ((nee_mask >> l) & 1u)) {
-        const float2 uv = nu[l];
-        const DLight& lt = sc.lights[p.J->light_base + l];
-        if ((MASK & MK_ENV) && lt.env >= 0) {
-          // sample_environment_light (src/renderer/direct_illumination.cpp:73-106)
-          f3 Le, lpos;
-          float lpdf;
-          if (env_sample(sc.envs[lt.env], is.pos, uv.x, uv.y, Le, lpdf, lpos) && !black(Le)) {
-            f3 to_light = lpos - is.pos;
-            bool too_close;
-            dist = dist_minus_eps(len2f(to_light), too_close);
-            if (!too_close) {
-              to_light = normalize(to_light);
-              f3 bf;
-              float bpdf;
-              m_value<MASK>(bsdf, kind, to_light, bf, bpdf);
-              trace = !black(bf);
-              if (trace) {
-                const f3 fl = muls(mulc(Le, bf), abs_cos(to_light, bsdf.g.z));
-                const float w = power_heuristic(lpdf, bpdf);
-                cc = mulc(coef_prev, divs(muls(fl, w), lpdf));
-                so = is.pos;
-                sd = normalize(to_light);
-              }
-            }
-          }
-        } else {
-          // sample_area_light (src/renderer/direct_illumination.cpp:35-71) via
-          // UniformSampleTriangle (src/shape/triangle.cpp:61-97)
-          const float su0 = sqrtf(uv.x);
-          const float bx = 1.0f - su0, by = uv.y * su0;
-          const f3 lpos = scale(lt.A, bx) + scale(lt.B, by) + scale(lt.C, 1.0f - bx - by);
-          const f3 sp2ref = is.pos - lpos;
-          if (dot(lt.gz, sp2ref) > 0.0f) {
-            const float dist2 = len2f(sp2ref);
-            const float lpdf = area_to_solid_pdf(lt.area_pdf * dist2, dot(lt.gz, sp2ref), dist2);
-            if (lpdf) {
-              f3 to_light = lpos - is.pos;
-              bool too_close;
-              dist = dist_minus_eps(len2f(to_light), too_close);
-              if (!too_close) {
-                to_light = normalize(to_light);
-                f3 bf;
-                float bpdf;
-                m_value<MASK>(bsdf, kind, to_light, bf, bpdf);
-                trace = !black(bf);
-                if (trace) {
-                  const f3 fl = muls(mulc(lt.emission, bf), abs_cos(to_light, bsdf.g.z));
-                  const float w = power_heuristic(lpdf, bpdf);
-                  cc = mulc(coef_prev, divs(muls(fl, w), lpdf));
-                  so = is.pos;
-                  sd = normalize(to_light);
-                }
-              }
-            }
-          }
+        if (ended || term) {
+          // the sample is over: its film update, now or once its direct
+          // lighting is known, and the pixel's next sample (samples that end
+          // before their first vertex, min_depth below 0, update the film as
+          // they start: they wait for the update that is due)
+          if (ended) film_add(*p.J, p.slot, p.px, p.py, film_value(p.L));
+          due = term;
+          due_L = p.L;
+          due_x = p.px;
+          due_y = p.py;
+          due_slot = p.slot;
+          due_J = p.J;
+          ++p.finished;
+          ++p.sample;
+          restart = due && p.J->min_depth < 0;
+          if (!restart) p.has_ray = start_sample(p);
         }
       }
-      // the shadow ray: the remembered occluder first, then the walk
-      bool blocked = false;
-      bool walk = trace;
-      if (trace && P.occluder_cache && sc.slot_leaf && oc[l] >= 0 &&
-          occluded_by_slot(sc, p.J->scene, oc[l], so, sd, kEps, dist)) {
-        blocked = true;
-        walk = false;
-        ++n_hits;
-      }
-      n_sh += trace;
-      if (__any_sync(kFull, walk)) {
-        const Traced sh = warp_trace<true>(sc, walk, walk ? p.J->scene : 0, so, sd, kEps, dist, P.err);
-        if (walk && sh.occluded) {
-          blocked = true;
-          oc[l] = sh.h.prim;
-        }
-      }
-      if (trace && !blocked) direct = direct + cc;
-      // the block walks each light's shadow rays together: without this
-      // barrier the warps interleave one light's walk with the next light's
-      // sampling (86 against 101 Msamples/s on the Cornell box)
-      __syncthreads();
     }
-
-    __syncthreads();
-    // ---- mis: the BSDF-sampled ray's emission, weighted against the light
-    //      (mis_contribution of render.cu, direct_illumination.cpp:144-198)
-    {
-      // a ray that can reach no light is not traced: its closest hit would give zero
-      Traced mh;
-      mh.h.prim = -1;
-      if (__any_sync(kFull, mis_trace))
-        mh = warp_trace<false>(sc, mis_trace, mis_trace ? p.J->scene : 0, mo, md, 0.0f, kRealMax, P.err);
-      n_ext += mis_trace;
-      if (mis) {
-        const int pid = mis_trace ? mh.h.prim : -1;
-        f3 c = mk3(0.0f, 0.0f, 0.0f);
-        if (pid < 0) {
-          const int ei = p.J->env;
-          if ((MASK & MK_ENV) && ei >= 0) {
-            const DEnv& e = sc.envs[ei];
-            const f3 Le = env_emit(e, md);
-            if (!black(Le)) {
-              const f3 f = muls(mulc(Le, mf), mcos);
-              const float w = power_heuristic(mpdf, env_pdf(e, md));
-              c = divs(muls(f, w), mpdf);
-            }
-          }
-        } else {
-          const DPrim& pr = sc.prims[pid];
-          if (pr.emissive) {
-            const f3 gz = sc.tshade[pr.shape].gz;
-            if (dot(gz, -md) > 0.0f) {
-              const f3 f = muls(mulc(pr.emission, mf), mcos);
-              const f3 pos = mo + scale(md, mh.h.t_attr);
-              const float lpdf = light_pdf_at(pr.area, mo, pos, gz);
-              const float w = power_heuristic(mpdf, lpdf);
-              c = divs(muls(f, w), mpdf);
-            }
-          }
-        }
-        direct = direct + mulc(coef_prev, c);
-      }
-    }
-
-    // ---- finish: the vertex's direct lighting, then the path goes on or ends.
-    // Samples that ended in the vertex phase finish here too (they draw no
-    // more random numbers this iteration). With one inlined copy of the film
-    // update and the camera-ray code instead of four, the kernel spills less
-    // and ran 2.5% faster on the Cornell box.
-    if (vertex) p.L = p.L + direct;
-    if (ended || (vertex && term)) finish_sample(p);
-    if (!done && !p.has_ray) p.slot = -1;  // the pixel's samples are done: claim another
   }
   // statistics (warp sums, one atomic per warp)
   const unsigned long long sums[5] = {p.finished, n_ext, n_sh, n_vert, n_hits};
@@ -524,20 +656,15 @@ unsigned mega_kernel_mask(const DScene& sc, bool has_disney12) {
   return has_disney12 ? kMaskPD : kMaskPhong;
 }
 
-cudaError_t launch_mega(const MegaLaunch& P, unsigned mask, int grid, int threads, cudaStream_t st) {
-  if (mask == kMaskPhong) k_mega<kMaskPhong><<<grid, threads, 0, st>>>(P);
-  else if (mask == kMaskPD) k_mega<kMaskPD><<<grid, threads, 0, st>>>(P);
-  else k_mega<kMaskAll><<<grid, threads, 0, st>>>(P);
+cudaError_t launch_mega(const MegaLaunch& P, unsigned mask, int grid, cudaStream_t st) {
+  const int threads = kMegaThreads;
+  const size_t smem = (size_t)(threads / 32) * kPoolBytes;
+  const cudaError_t e = cudaFuncSetAttribute(kernel_of(mask), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  if (mask == kMaskPhong) k_mega<kMaskPhong><<<grid, threads, smem, st>>>(P);
+  else if (mask == kMaskPD) k_mega<kMaskPD><<<grid, threads, smem, st>>>(P);
+  else k_mega<kMaskAll><<<grid, threads, smem, st>>>(P);
   return cudaGetLastError();
-}
-
-int mega_blocks_per_sm(unsigned mask) {
-  int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel_of(mask), kMegaThreads, 0) != cudaSuccess || n <= 0) {
-    cudaGetLastError();
-    n = 1;
-  }
-  return n;
 }
 
 }  // namespace trg

@@ -18,9 +18,8 @@ enum : unsigned {
   MK_ENV = 1u << 8,   // an environment light
   MK_MAPS = 1u << 9,  // Phong image maps
 };
-// Lights of one scene the persistent kernel keeps per-thread state for
-// (light-sample draws and remembered occluders); sets with more render with
-// the wavefront.
+// Lights of one scene the persistent kernel keeps per-thread state for (the
+// remembered occluders); sets with more render with the wavefront.
 constexpr int kMegaLights = 16;
 
 struct MegaLaunch {
@@ -28,6 +27,8 @@ struct MegaLaunch {
   const JobDev* jobs;
   int njobs, nslots;
   int nl_max;            // most lights of one job's scene (<= kMegaLights)
+  int lanes;             // lanes of a warp that own pixels (1 .. 32)
+  DMat* mt;              // sets with image maps: one material set-up per thread of the launch
   int occluder_cache;    // remember each (slot, light)'s last occluder (tr_tuning.occluder_cache)
   unsigned int* fetch;   // next unclaimed path slot (zeroed by the host)
   int* err;              // bit 0: traversal stack overflow; bit 1: a slot ran past its vertex bound
@@ -37,10 +38,8 @@ struct MegaLaunch {
 // The smallest instantiation covering a scene set (MK_* bits).
 unsigned mega_kernel_mask(const DScene& sc, bool has_disney12);
 // Launches the persistent kernel of instantiation `mask` (grid blocks of
-// `threads` threads, at most kMegaThreads, a multiple of 32) on `st`.
-cudaError_t launch_mega(const MegaLaunch& P, unsigned mask, int grid, int threads, cudaStream_t st);
-// Resident blocks per SM of that instantiation.
-int mega_blocks_per_sm(unsigned mask);
+// kMegaThreads threads, at most one per SM resident) on `st`.
+cudaError_t launch_mega(const MegaLaunch& P, unsigned mask, int grid, cudaStream_t st);
 constexpr int kMegaThreads = 512;
 
 }  // namespace trg

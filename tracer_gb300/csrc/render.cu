@@ -1531,6 +1531,26 @@ static JobDev make_job_dev(tr_ctx* ctx, const JobSpec& j, int slot_base, void* f
   return J;
 }
 
+// Launch shape of the persistent kernel for n pixels: blocks of 512 threads
+// (one per SM), and no more pixel-owning lanes per warp than it takes to have
+// every pixel resident at once: a warp's other lanes walk rays and evaluate
+// light samples all the same, and fewer paths per warp diverge less. Measured
+// (us, lanes 32 / by this rule): all material kinds at 61x47x1 1423 / 782 (2),
+// Cornell 125x93x2 796 / 540 (5), Disney grid 200x150x4 3295 / 2300 (13), all
+// kinds under an environment light 320x180x8 5245 / 4917 (24), Cornell
+// 256x256x16 6503 / 6109 (27). Blocks of 256 and 128 threads at their best
+// lane counts were 0-15% slower.
+struct MegaShape {
+  int lanes, grid;
+};
+static MegaShape mega_shape(int n, int sms) {
+  constexpr int warps = kMegaThreads / 32;
+  MegaShape s;
+  s.lanes = std::min(32, (n + sms * warps - 1) / (sms * warps));
+  s.grid = std::min(sms, (n + warps * s.lanes - 1) / (warps * s.lanes));
+  return s;
+}
+
 tr_status render_jobs(tr_ctx* ctx, const JobSpec* jobs, int njobs, uint32_t flags, tr_stats* stats,
                       const tr_guide_params* gp = nullptr) {
   if (!ctx->has_scene) return set_err(ctx, TR_ERR_STATE, "no scene uploaded");
@@ -1719,18 +1739,16 @@ tr_status render_jobs(tr_ctx* ctx, const JobSpec* jobs, int njobs, uint32_t flag
   // kMegaAutoSlots pixels, which the wavefront's launches cannot fill the GPU with
   bool mega = false;
   unsigned mmask = 0;
-  int mgrid = 0, mthreads = kMegaThreads;
+  int mgrid = 0, mlanes = 0;
   if (!gp && !timed && !count && nl <= kMegaLights && ctx->tune.render_mode != TR_RENDER_MODE_WAVEFRONT) {
     mega = ctx->tune.render_mode == TR_RENDER_MODE_PERSISTENT || (long long)n <= kMegaAutoSlots;
     if (mega) {
       bool d12 = false;
       for (const DMat& m : ctx->hs.mats) d12 |= m.kind == MAT_DISNEY12;
       mmask = mega_kernel_mask(ctx->dsc, d12);
-      // full 512-thread blocks even when fewer than the SMs: spreading a
-      // 65k-pixel render over all 152 SMs in 448-thread blocks was slower
-      // (70.7 against 75.7 Msamples/s on the Cornell box)
-      const long long want = ((long long)n + kMegaThreads - 1) / kMegaThreads;
-      mgrid = (int)std::min<long long>(want, (long long)sms * mega_blocks_per_sm(mmask));
+      const MegaShape sh = mega_shape(n, sms);
+      mlanes = sh.lanes;
+      mgrid = sh.grid;
     }
   }
   std::vector<cudaEvent_t>& ev = rb->ev_pool;
@@ -1760,6 +1778,12 @@ tr_status render_jobs(tr_ctx* ctx, const JobSpec* jobs, int njobs, uint32_t flag
     M.njobs = njobs;
     M.nslots = n;
     M.nl_max = nl;
+    M.lanes = mlanes;
+    M.mt = nullptr;
+    if (ctx->dsc.has_textures) {
+      RCHK(rb->MT.reserve((size_t)mgrid * kMegaThreads * sizeof(DMat)));
+      M.mt = rb->MT.as<DMat>();
+    }
     M.occluder_cache = ctx->tune.occluder_cache;
     M.fetch = P.ctr + C_FEXT;
     M.err = (int*)(P.ctr + C_ERR);
@@ -1772,7 +1796,7 @@ tr_status render_jobs(tr_ctx* ctx, const JobSpec* jobs, int njobs, uint32_t flag
       le = cudaMemsetAsync(jd[k].film, 0, (size_t)jd[k].W * jd[k].H * (jd[k].fp64 ? 32 : 16), st);
     if (le == cudaSuccess) le = cudaMemsetAsync(P.ctr, 0, kCtrWords * 4, st);
     if (le == cudaSuccess) le = cudaMemsetAsync(P.stats, 0, kStatWords * 8, st);
-    if (le == cudaSuccess) le = launch_mega(M, mmask, mgrid, mthreads, st);
+    if (le == cudaSuccess) le = launch_mega(M, mmask, mgrid, st);
     if (use_graph) {
       const cudaError_t ce = cudaStreamEndCapture(st, &graph);
       if (le == cudaSuccess) le = ce;

@@ -236,52 +236,48 @@ struct VisitCount {
   unsigned int cache_hits = 0;  // any-hit rays answered by a remembered occluder
 };
 
-template <bool ANY, bool COUNT = false>
-struct Traversal {
-  // Tests one leaf slot. Returns true when ANY and the ray is occluded.
-  // quick: the ray meets tri_surely_missed's conditions.
-  static __device__ __forceinline__ bool test_slot(const DScene& sc, int slot, f3 o, f3 d, float t_min,
-                                                   float& t_max, Hit& h, bool quick) {
-    const float4 s0 = ldg4(sc.slots + 3 * slot);
-    const float4 s1 = ldg4(sc.slots + 3 * slot + 1);
-    const int kind = __float_as_int(s1.w);
-    if (kind < 0) {
-      const float4 s2 = ldg4(sc.slots + 3 * slot + 2);
-      if (quick && tri_surely_missed(mk3(s1.x, s1.y, s1.z), mk3(s2.x, s2.y, s2.z), s2.w,
-                                     o - mk3(s0.x, s0.y, s0.z), d, t_max))
-        return false;
-      float t, a, b;
-      if (tri_test(s0, s1, s2, o, d, t_min, t_max, t, a, b)) {
-        if (ANY) return true;
-        t_max = t;
-        h.prim = __float_as_int(s0.w);
-        h.t_attr = t;
-        h.alpha = a;
-        h.beta = b;
-      }
-    } else {
-      const DSphere& s = sc.spheres[kind];
-      f3 lo, ld;
-      sphere_local(s, o, d, lo, ld);
-      float t0, t1;
-      if (!sphere_roots(lo, ld, s.radius, t0, t1)) return false;
-      if (ANY) return (t_min <= t0 && t0 <= t_max) || (t_min <= t1 && t1 <= t_max);
-      if (t_max < t0 || t1 < t_min) return false;
-      const bool not_t0 = t0 < t_min;
-      if (not_t0 && t1 > t_max) return false;
-      // Sphere::intersect_p never writes its hit_t argument, so
-      // GeometricPrimitive stores 0 into ray.t_max (src/shape/sphere.cpp:98-119,
-      // src/shape/geometry.cpp:49-57).
-      t_max = 0.0f;
+// Tests one leaf slot. Returns true when `any` and the ray is occluded.
+// quick: the ray meets tri_surely_missed's conditions.
+__device__ __forceinline__ bool test_slot(const DScene& sc, int slot, f3 o, f3 d, float t_min, float& t_max, Hit& h,
+                                          bool any, bool quick) {
+  const float4 s0 = ldg4(sc.slots + 3 * slot);
+  const float4 s1 = ldg4(sc.slots + 3 * slot + 1);
+  const int kind = __float_as_int(s1.w);
+  if (kind < 0) {
+    const float4 s2 = ldg4(sc.slots + 3 * slot + 2);
+    if (quick && tri_surely_missed(mk3(s1.x, s1.y, s1.z), mk3(s2.x, s2.y, s2.z), s2.w,
+                                   o - mk3(s0.x, s0.y, s0.z), d, t_max))
+      return false;
+    float t, a, b;
+    if (tri_test(s0, s1, s2, o, d, t_min, t_max, t, a, b)) {
+      if (any) return true;
+      t_max = t;
       h.prim = __float_as_int(s0.w);
-      h.t_attr = not_t0 ? t1 : t0;
-      h.alpha = 0.0f;
-      h.beta = 0.0f;
+      h.t_attr = t;
+      h.alpha = a;
+      h.beta = b;
     }
-    return false;
+  } else {
+    const DSphere& s = sc.spheres[kind];
+    f3 lo, ld;
+    sphere_local(s, o, d, lo, ld);
+    float t0, t1;
+    if (!sphere_roots(lo, ld, s.radius, t0, t1)) return false;
+    if (any) return (t_min <= t0 && t0 <= t_max) || (t_min <= t1 && t1 <= t_max);
+    if (t_max < t0 || t1 < t_min) return false;
+    const bool not_t0 = t0 < t_min;
+    if (not_t0 && t1 > t_max) return false;
+    // Sphere::intersect_p never writes its hit_t argument, so
+    // GeometricPrimitive stores 0 into ray.t_max (src/shape/sphere.cpp:98-119,
+    // src/shape/geometry.cpp:49-57).
+    t_max = 0.0f;
+    h.prim = __float_as_int(s0.w);
+    h.t_attr = not_t0 ? t1 : t0;
+    h.alpha = 0.0f;
+    h.beta = 0.0f;
   }
-
-};
+  return false;
+}
 
 // Any hit through a remembered occluder: slot s, tested after the box of its
 // BVH leaf (stored in the leaf's parent node). The slab test passes a box
@@ -312,7 +308,7 @@ __device__ __forceinline__ bool occluded_by_slot(const DScene& sc, int scene, in
     return false;
   Hit h;
   float tm = t_max;
-  return Traversal<true>::test_slot(sc, s, o, d, t_min, tm, h, false);
+  return test_slot(sc, s, o, d, t_min, tm, h, true, false);
 }
 
 // ---------------------------------------------------------------------------
@@ -337,9 +333,12 @@ constexpr int kStackBinary = 96;               // entries (a binary walk pushes 
 constexpr int kMaxDepth = kStackBinary - 4;      // the host rejects binary trees this many levels deep
 constexpr int kStackWide = 96;                   // entries; the host keeps four-wide trees whose stack bound fits
 
-template <bool ANY, bool COUNT, bool WIDE = false>
+// MIXED: each ray is a closest-hit or an any-hit ray by the member `any`
+// (ANY is ignored).
+template <bool ANY, bool COUNT, bool WIDE = false, bool MIXED = false>
 struct TravLane {
   static_assert(ANY || !WIDE, "closest-hit traversal keeps the binary order");
+  static_assert(!(MIXED && (COUNT || WIDE)), "mixed rays walk the binary tree, uncounted");
   static constexpr int kStack = WIDE ? kStackWide : kStackBinary;
   static constexpr unsigned kGeneral = 8u, kExactTri = 16u;
   f3 o, d, inv;
@@ -350,6 +349,8 @@ struct TravLane {
   float path_t;      // largest box entry t on the path taken since the last pop
   Hit h;
   bool occluded, failed;
+  bool any;  // MIXED: this ray wants any hit
+  __device__ __forceinline__ bool is_any() const { return MIXED ? any : ANY; }
   int2 st[kStack];      // (ref << 5 | min(count, 31), t bits)
   int big_cnt[kStack];  // counts of 31 or more, by stack index
 
@@ -440,7 +441,7 @@ struct TravLane {
     hl = hl && tl < t_max;
     hr = hr && tr < t_max;
     bool second_near = (neg >> __float_as_int(dd.w)) & 1u;
-    if (ANY && !COUNT && sc.any_order != 0) {
+    if (is_any() && !COUNT && sc.any_order != 0) {
       // any hit: the answer does not depend on the order, only the visits do
       // (the counting walk keeps the reference's visits)
       if (sc.any_order == 1) {
@@ -509,14 +510,14 @@ struct TravLane {
   __device__ __forceinline__ bool postponed_leaf(const DScene& sc, VisitCount& vc) {
     for (int i = 0; i < pc; ++i) {
       if (COUNT) ++vc.prims;
-      if (Traversal<ANY, COUNT>::test_slot(sc, pl + i, o, d, t_min, t_max, h, !(neg & kExactTri))) {
+      if (test_slot(sc, pl + i, o, d, t_min, t_max, h, is_any(), !(neg & kExactTri))) {
         occluded = true;
         h.prim = pl + i;  // any hit: the occluding slot
         return false;
       }
     }
     pc = 0;
-    if (!ANY && cnt >= 0 && !(path_t < t_max)) cnt = -1;
+    if (!is_any() && cnt >= 0 && !(path_t < t_max)) cnt = -1;
     if (cnt < 0) return pop();
     return true;
   }
@@ -568,7 +569,7 @@ struct TravLane {
   __device__ __forceinline__ bool leaf(const DScene& sc, VisitCount& vc) {
     for (int i = 0; i < cnt; ++i) {
       if (COUNT) ++vc.prims;
-      if (Traversal<ANY, COUNT>::test_slot(sc, cur + i, o, d, t_min, t_max, h, !(neg & kExactTri))) {
+      if (test_slot(sc, cur + i, o, d, t_min, t_max, h, is_any(), !(neg & kExactTri))) {
         occluded = true;
         h.prim = cur + i;  // any hit: the occluding slot
         return false;
