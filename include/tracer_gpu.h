@@ -293,8 +293,8 @@ tr_status tr_synchronize(tr_ctx* ctx);
  *  - render_mode: TR_RENDER_MODE_WAVEFRONT runs a render (or a batch) as
  *    the wavefront, about ten launches per path vertex over compacted queues;
  *    TR_RENDER_MODE_PERSISTENT as one launch of the persistent kernel, each
- *    thread running a pixel's samples with the path state in registers (the
- *    launch and the film zeroing captured into a CUDA graph when
+ *    owning lane running a pixel's samples with the path state in registers
+ *    (a batch's launch and film zeroing captured into a CUDA graph when
  *    graph_iterations > 0); TR_RENDER_MODE_AUTO picks the persistent kernel
  *    for renders of at most 2^17 pixels. Guided and instrumented renders
  *    (TR_RENDER_TIME_STAGES, TR_RENDER_COUNT_VISITS) and scenes with more
@@ -422,10 +422,14 @@ tr_status tr_render_dev(tr_ctx* ctx, const tr_camera* cam, const tr_filter* filt
  *  - The array is shared by every context on a device: calls that overlap
  *    in time on one device (two contexts, two threads) race and corrupt
  *    each other's results. Calls on one context run in order.
- *  - Blocks until done. Every 16 wavefront iterations it copies the
- *    live-path count into a host stack variable (a synchronous pageable
- *    copy) and stops once every path has ended, or with TR_ERR_CANCELLED
- *    after tr_cancel; stats->device_ms and stage_ms stay 0.
+ *  - Blocks until done. Renders whose samples' paths are at most 256
+ *    vertices in a row (spp * (max_depth + 2), + 20 with glass) are one launch
+ *    of the persistent kernel (unless tr_tuning.render_mode says wavefront);
+ *    for others it copies, every 16 wavefront iterations, the live-path
+ *    count into a host stack variable (a synchronous pageable copy) and
+ *    stops once every path has ended. TR_ERR_CANCELLED after tr_cancel, when
+ *    the launch or those iterations are over; stats->device_ms and stage_ms
+ *    stay 0.
  *  - Restores the caller's current device before returning. */
 tr_status tr_render_dev_noalloc(tr_ctx* ctx, const tr_camera* cam, const tr_filter* filter,
                                 const tr_render_params* params, float* d_rgbw, tr_stats* stats);

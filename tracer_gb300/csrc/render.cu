@@ -99,6 +99,9 @@ struct RenderBuffers {
   DevBuf q_ord, act_flag;           // the live-slot list in slot order, per-slot marks
   unsigned int tb_count = 0, tb_cap = 0;  // training records of the last guided render
   unsigned int* h_active = nullptr;  // pinned: live-slot count per check
+  DevBuf mega_state;                 // persistent kernel: counters, then statistics
+  char* h_mega = nullptr;            // pinned: their copy
+  cudaEvent_t mega_e0 = nullptr, mega_e1 = nullptr;
   std::vector<cudaEvent_t> ev_pool;  // reused by stage timing
 };
 
@@ -1391,9 +1394,12 @@ void release_render(tr_ctx* ctx) {
                     &rb->HM, &rb->SC, &rb->NU, &rb->SH, &rb->SHC, &rb->acc, &rb->q_ext, &rb->q_act, &rb->q_mat, &rb->q_nee,
                     &rb->q_sh, &rb->ctr, &rb->stats, &rb->VR, &rb->NV, &rb->gfeat, &rb->gout, &rb->tb, &rb->jobs,
                     &rb->GX, &rb->grow, &rb->MT, &rb->q_srt, &rb->bin_key, &rb->bin_cnt, &rb->OC, &rb->q_ord,
-                    &rb->act_flag})
+                    &rb->act_flag, &rb->mega_state})
     b->release();
   if (rb->h_active) cudaFreeHost(rb->h_active);
+  if (rb->h_mega) cudaFreeHost(rb->h_mega);
+  if (rb->mega_e0) cudaEventDestroy(rb->mega_e0);
+  if (rb->mega_e1) cudaEventDestroy(rb->mega_e1);
   for (cudaEvent_t e : rb->ev_pool) cudaEventDestroy(e);
   delete rb;
   ctx->rb = nullptr;
@@ -1551,6 +1557,109 @@ static MegaShape mega_shape(int n, int sms) {
   return s;
 }
 
+static MegaLaunch mega_launch(tr_ctx* ctx, const JobDev* jobs, int njobs, int n, int nl, const MegaShape& shape,
+                              unsigned int* ctr, unsigned long long* st) {
+  MegaLaunch M;
+  M.sc = ctx->dsc;
+  M.jobs = jobs;
+  M.njobs = njobs;
+  M.nslots = n;
+  M.nl_max = nl;
+  M.lanes = shape.lanes;
+  M.mt = nullptr;
+  M.occluder_cache = ctx->tune.occluder_cache;
+  M.fetch = ctr + C_FEXT;
+  M.err = (int*)(ctr + C_ERR);
+  M.stats = st;
+  return M;
+}
+
+static unsigned mega_mask(tr_ctx* ctx) {
+  bool d12 = false;
+  for (const DMat& m : ctx->hs.mats) d12 |= m.kind == MAT_DISNEY12;
+  return mega_kernel_mask(ctx->dsc, d12);
+}
+
+static tr_status mega_result(tr_ctx* ctx, unsigned int err, const unsigned long long* hs, float ms, tr_stats* stats) {
+  if (stats) {
+    std::memset(stats, 0, sizeof(*stats));
+    stats->samples = hs[0];
+    stats->extend_rays = hs[1];
+    stats->shadow_rays = hs[2];
+    stats->shade_items = hs[3];
+    stats->iterations = 1;
+    stats->device_ms = ms;
+    stats->occluder_hits = hs[8];
+  }
+  if (err & 1u) return set_err(ctx, TR_ERR_QUEUE_OVERFLOW, "traversal stack overflow");
+  if (err & 2u) return set_err(ctx, TR_ERR_TIMEOUT, "a path slot ran past its vertex bound");
+  return TR_OK;
+}
+
+// A render (or a batch) by the persistent kernel: every sample of every job
+// in one launch. It needs no path state in memory, so none of the wavefront's
+// buffers are reserved, and the counters and statistics come back in one
+// asynchronous copy. A batch's film zeroing and launch are captured into one
+// CUDA graph (with graphs enabled); one job's three operations are issued
+// directly. Capturing and instantiating those, creating events and two
+// blocking copies took 65 of a 61x47x1 frame's 796 us.
+static tr_status render_persistent(tr_ctx* ctx, const JobSpec* jobs, int njobs, int n, int nl, int sms,
+                                   tr_stats* stats) {
+  if (!ctx->rb) ctx->rb = new RenderBuffers();
+  RenderBuffers* rb = ctx->rb;
+  cudaStream_t st = ctx->stream;
+  const MegaShape shape = mega_shape(n, sms);
+  constexpr size_t kCtrBytes = kCtrWords * 4, kStatBytes = kStatWords * 8;
+  TR_CUDA(ctx, rb->mega_state.reserve(kCtrBytes + kStatBytes));
+  TR_CUDA(ctx, rb->jobs.reserve((size_t)njobs * sizeof(JobDev)));
+  if (!jobs[0].film) TR_CUDA(ctx, rb->acc.reserve((size_t)n * 32));
+  if (ctx->dsc.has_textures) TR_CUDA(ctx, rb->MT.reserve((size_t)shape.grid * kMegaThreads * sizeof(DMat)));
+  if (!rb->h_mega) TR_CUDA(ctx, cudaHostAlloc((void**)&rb->h_mega, kCtrBytes + kStatBytes, cudaHostAllocDefault));
+  for (cudaEvent_t* e : {&rb->mega_e0, &rb->mega_e1})
+    if (!*e) TR_CUDA(ctx, cudaEventCreate(e));
+  std::vector<JobDev> jd(njobs);
+  int base = 0;
+  for (int k = 0; k < njobs; ++k) {
+    jd[k] = make_job_dev(ctx, jobs[k], base, jobs[k].film ? jobs[k].film : rb->acc.p);
+    base += jobs[k].prm.width * jobs[k].prm.height;
+  }
+  TR_CUDA(ctx, cudaMemcpyAsync(rb->jobs.p, jd.data(), jd.size() * sizeof(JobDev), cudaMemcpyHostToDevice, st));
+  unsigned int* ctr = rb->mega_state.as<unsigned int>();
+  MegaLaunch M = mega_launch(ctx, rb->jobs.as<JobDev>(), njobs, n, nl, shape, ctr,
+                             reinterpret_cast<unsigned long long*>(rb->mega_state.as<char>() + kCtrBytes));
+  if (ctx->dsc.has_textures) M.mt = rb->MT.as<DMat>();
+  ctx->cancel.store(0);
+  const unsigned mask = mega_mask(ctx);
+  TR_CUDA(ctx, cudaEventRecord(rb->mega_e0, st));
+  const bool use_graph = njobs > 1 && ctx->tune.graph_iterations > 0;
+  if (use_graph) TR_CUDA(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+  cudaError_t le = cudaSuccess;
+  for (int k = 0; k < njobs && le == cudaSuccess; ++k)
+    le = cudaMemsetAsync(jd[k].film, 0, (size_t)jd[k].W * jd[k].H * (jd[k].fp64 ? 32 : 16), st);
+  if (le == cudaSuccess) le = cudaMemsetAsync(ctr, 0, kCtrBytes + kStatBytes, st);
+  if (le == cudaSuccess) le = launch_mega(M, mask, shape.grid, st);
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t gexec = nullptr;
+  if (use_graph) {
+    const cudaError_t ce = cudaStreamEndCapture(st, &graph);
+    if (le == cudaSuccess) le = ce;
+    if (le == cudaSuccess) le = cudaGraphInstantiate(&gexec, graph, 0);
+    if (le == cudaSuccess) le = cudaGraphLaunch(gexec, st);
+  }
+  if (le == cudaSuccess) le = cudaEventRecord(rb->mega_e1, st);
+  if (le == cudaSuccess)
+    le = cudaMemcpyAsync(rb->h_mega, ctr, kCtrBytes + kStatBytes, cudaMemcpyDeviceToHost, st);
+  const cudaError_t se = cudaStreamSynchronize(st);
+  if (gexec) cudaGraphExecDestroy(gexec);
+  if (graph) cudaGraphDestroy(graph);
+  TR_CUDA(ctx, le == cudaSuccess ? se : le);
+  float ms = 0.0f;
+  cudaEventElapsedTime(&ms, rb->mega_e0, rb->mega_e1);
+  rb->tb_count = 0;
+  return mega_result(ctx, reinterpret_cast<unsigned int*>(rb->h_mega)[C_ERR],
+                     reinterpret_cast<unsigned long long*>(rb->h_mega + kCtrBytes), ms, stats);
+}
+
 tr_status render_jobs(tr_ctx* ctx, const JobSpec* jobs, int njobs, uint32_t flags, tr_stats* stats,
                       const tr_guide_params* gp = nullptr) {
   if (!ctx->has_scene) return set_err(ctx, TR_ERR_STATE, "no scene uploaded");
@@ -1571,6 +1680,19 @@ tr_status render_jobs(tr_ctx* ctx, const JobSpec* jobs, int njobs, uint32_t flag
   const int n = (int)total;
   const int nl = ctx->dsc.max_lights;
   if ((long long)n * std::max(nl, 1) > (1ll << 30)) return set_err(ctx, TR_ERR_ARG, "too many shadow records");
+  int sms = 0;
+  {
+    const cudaError_t ae = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    if (ae != cudaSuccess) return cuda_fail(ctx, ae, "cudaDeviceGetAttribute(multiprocessor count)");
+  }
+  if (sms <= 0) sms = 1;
+  // the persistent kernel (tr_tuning.render_mode) for plain renders whose
+  // scenes have at most kMegaLights lights; by default for renders of at most
+  // kMegaAutoSlots pixels, which the wavefront's launches cannot fill the GPU with
+  if (!gp && !(flags & (TR_RENDER_TIME_STAGES | TR_RENDER_COUNT_VISITS)) && nl <= kMegaLights &&
+      (ctx->tune.render_mode == TR_RENDER_MODE_PERSISTENT ||
+       (ctx->tune.render_mode == TR_RENDER_MODE_AUTO && (long long)n <= kMegaAutoSlots)))
+    return render_persistent(ctx, jobs, njobs, n, nl, sms, stats);
   tr_status s = reserve_render(ctx, n, nl);
   if (s != TR_OK) return s;
   RenderBuffers* rb = ctx->rb;
@@ -1703,12 +1825,6 @@ tr_status render_jobs(tr_ctx* ctx, const JobSpec* jobs, int njobs, uint32_t flag
     }
   }
 
-  int sms = 0;
-  {
-    const cudaError_t ae = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-    if (ae != cudaSuccess) return cuda_fail(ctx, ae, "cudaDeviceGetAttribute(multiprocessor count)");
-  }
-  if (sms <= 0) sms = 1;
   const int grid = sms * ctx->tune.shade_blocks_per_sm, grid_init = sms * 8;
   // the treelet staged by the binary traversal kernels
   P.tl_n = treelet_nodes(ctx);
@@ -1734,23 +1850,6 @@ tr_status render_jobs(tr_ctx* ctx, const JobSpec* jobs, int njobs, uint32_t flag
   cudaGraphExec_t gexec = nullptr;
   const bool timed = (flags & TR_RENDER_TIME_STAGES) != 0;
   const bool count = (flags & TR_RENDER_COUNT_VISITS) != 0;
-  // the persistent kernel (tr_tuning.render_mode) for plain renders whose
-  // scenes have at most kMegaLights lights; by default for renders of at most
-  // kMegaAutoSlots pixels, which the wavefront's launches cannot fill the GPU with
-  bool mega = false;
-  unsigned mmask = 0;
-  int mgrid = 0, mlanes = 0;
-  if (!gp && !timed && !count && nl <= kMegaLights && ctx->tune.render_mode != TR_RENDER_MODE_WAVEFRONT) {
-    mega = ctx->tune.render_mode == TR_RENDER_MODE_PERSISTENT || (long long)n <= kMegaAutoSlots;
-    if (mega) {
-      bool d12 = false;
-      for (const DMat& m : ctx->hs.mats) d12 |= m.kind == MAT_DISNEY12;
-      mmask = mega_kernel_mask(ctx->dsc, d12);
-      const MegaShape sh = mega_shape(n, sms);
-      mlanes = sh.lanes;
-      mgrid = sh.grid;
-    }
-  }
   std::vector<cudaEvent_t>& ev = rb->ev_pool;
   size_t nev = 0;
   auto cleanup = [&]() {
@@ -1768,67 +1867,6 @@ tr_status render_jobs(tr_ctx* ctx, const JobSpec* jobs, int njobs, uint32_t flag
       return cuda_fail(ctx, e_, #call); \
     }                                   \
   } while (0)
-  if (mega) {
-    // The persistent kernel: every sample of every job in one launch. With
-    // graphs enabled, the zeroing of the films and counters and the launch
-    // are captured into one CUDA graph and replayed as one launch.
-    MegaLaunch M;
-    M.sc = P.sc;
-    M.jobs = P.jobs;
-    M.njobs = njobs;
-    M.nslots = n;
-    M.nl_max = nl;
-    M.lanes = mlanes;
-    M.mt = nullptr;
-    if (ctx->dsc.has_textures) {
-      RCHK(rb->MT.reserve((size_t)mgrid * kMegaThreads * sizeof(DMat)));
-      M.mt = rb->MT.as<DMat>();
-    }
-    M.occluder_cache = ctx->tune.occluder_cache;
-    M.fetch = P.ctr + C_FEXT;
-    M.err = (int*)(P.ctr + C_ERR);
-    M.stats = P.stats;
-    const bool use_graph = ctx->tune.graph_iterations > 0;
-    RCHK(cudaEventRecord(e0, st));
-    if (use_graph) RCHK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    cudaError_t le = cudaSuccess;
-    for (int k = 0; k < njobs && le == cudaSuccess; ++k)
-      le = cudaMemsetAsync(jd[k].film, 0, (size_t)jd[k].W * jd[k].H * (jd[k].fp64 ? 32 : 16), st);
-    if (le == cudaSuccess) le = cudaMemsetAsync(P.ctr, 0, kCtrWords * 4, st);
-    if (le == cudaSuccess) le = cudaMemsetAsync(P.stats, 0, kStatWords * 8, st);
-    if (le == cudaSuccess) le = launch_mega(M, mmask, mgrid, st);
-    if (use_graph) {
-      const cudaError_t ce = cudaStreamEndCapture(st, &graph);
-      if (le == cudaSuccess) le = ce;
-      if (le == cudaSuccess) le = cudaGraphInstantiate(&gexec, graph, 0);
-      if (le == cudaSuccess) le = cudaGraphLaunch(gexec, st);
-    }
-    RCHK(le);
-    RCHK(cudaEventRecord(e1, st));
-    RCHK(cudaEventSynchronize(e1));
-    unsigned long long hs[kStatWords] = {};
-    RCHK(cudaMemcpy(hs, P.stats, sizeof(hs), cudaMemcpyDeviceToHost));
-    unsigned int ctrs[kCtrWords];
-    RCHK(cudaMemcpy(ctrs, P.ctr, sizeof(ctrs), cudaMemcpyDeviceToHost));
-    float ms = 0.0f;
-    cudaEventElapsedTime(&ms, e0, e1);
-    cleanup();
-    tr_status result = TR_OK;
-    if (ctrs[C_ERR] & 1u) result = set_err(ctx, TR_ERR_QUEUE_OVERFLOW, "traversal stack overflow");
-    else if (ctrs[C_ERR] & 2u) result = set_err(ctx, TR_ERR_TIMEOUT, "a path slot ran past its vertex bound");
-    rb->tb_count = 0;
-    if (stats) {
-      std::memset(stats, 0, sizeof(*stats));
-      stats->samples = hs[0];
-      stats->extend_rays = hs[1];
-      stats->shadow_rays = hs[2];
-      stats->shade_items = hs[3];
-      stats->iterations = 1;
-      stats->device_ms = ms;
-      stats->occluder_hits = hs[8];
-    }
-    return result;
-  }
   for (int k = 0; k < njobs; ++k)
     RCHK(cudaMemsetAsync(jd[k].film, 0, (size_t)jd[k].W * jd[k].H * (jd[k].fp64 ? 32 : 16), st));
   RCHK(cudaMemsetAsync(P.ctr, 0, kCtrWords * 4, st));
@@ -2202,6 +2240,37 @@ tr_status render_noalloc_impl(tr_ctx* ctx, const tr_camera* cam, const tr_filter
     if (ae != cudaSuccess) return cuda_fail(ctx, ae, "cudaDeviceGetAttribute(multiprocessor count)");
   }
   if (sms <= 0) sms = 1;
+  // Every slot finishes within spp * (max_depth + 2) iterations (plus the
+  // delta samples that do not count toward the depth).
+  const long long iters =
+      (long long)prm->spp * ((long long)prm->max_depth + 2 + (ctx->dsc.has_glass ? kMaxSpecularDepth : 0)) + 4;
+  // Short renders by the persistent kernel, whose state is in registers (two
+  // counters and a job record of the array are all it needs): Cornell 125x93x2
+  // 1550 -> 458 us. It cannot stop early, so renders whose longest path chain
+  // is more than kNoAllocOneLaunch vertices (tens of milliseconds) keep the
+  // wavefront, which looks for tr_cancel between its iterations; so do devices
+  // without the memory to launch it (its local memory per thread is larger).
+  constexpr long long kNoAllocOneLaunch = 256;
+  if (iters <= kNoAllocOneLaunch && nl <= kMegaLights && ctx->tune.render_mode != TR_RENDER_MODE_WAVEFRONT) {
+    const MegaShape shape = mega_shape(n, sms);
+    const MegaLaunch M = mega_launch(ctx, P.jobs, 1, n, nl, shape, P.ctr, P.stats);
+    NCHK(cudaMemsetAsync(d_rgbw, 0, (size_t)n * 16, st));
+    NCHK(cudaMemsetAsync(P.ctr, 0, kCtrWords * 4, st));
+    NCHK(cudaMemsetAsync(P.stats, 0, kStatWords * 8, st));
+    ctx->cancel.store(0);
+    const cudaError_t le = launch_mega(M, mega_mask(ctx), shape.grid, st);
+    if (le == cudaSuccess) {
+      unsigned long long hs[kStatWords];
+      unsigned int ctrs[kCtrWords];
+      NCHK(cudaMemcpyAsync(hs, P.stats, sizeof(hs), cudaMemcpyDeviceToHost, st));
+      NCHK(cudaMemcpyAsync(ctrs, P.ctr, sizeof(ctrs), cudaMemcpyDeviceToHost, st));
+      NCHK(cudaStreamSynchronize(st));
+      const tr_status r = mega_result(ctx, ctrs[C_ERR], hs, 0.0f, stats);
+      return r == TR_OK && ctx->cancel.load() ? set_err(ctx, TR_ERR_CANCELLED, "render cancelled") : r;
+    }
+    if (le != cudaErrorMemoryAllocation && le != cudaErrorLaunchOutOfResources) NCHK(le);
+    cudaGetLastError();
+  }
   const int grid = sms * ctx->tune.shade_blocks_per_sm, grid_init = sms * 8;
   const int grid_ext = traversal_grid(ctx, (const void*)k_extend<false>);
   const bool wide = any_wide(ctx);
@@ -2213,13 +2282,10 @@ tr_status render_noalloc_impl(tr_ctx* ctx, const tr_camera* cam, const tr_filter
   NCHK(cudaMemsetAsync(P.stats, 0, kStatWords * 8, st));
   k_init<<<grid_init, 256, 0, st>>>(P);
   NCHK(cudaGetLastError());
-  // Every slot finishes within spp * (max_depth + 2) iterations (plus the
-  // delta samples that do not count toward the depth): that bound is the
-  // ceiling. Every kDrainCheck iterations the live-slot count is copied into
-  // a host stack variable (a pageable copy: nothing is allocated), and the
-  // loop stops once the wavefront has drained or tr_cancel was called.
-  const long long iters =
-      (long long)prm->spp * ((long long)prm->max_depth + 2 + (ctx->dsc.has_glass ? kMaxSpecularDepth : 0)) + 4;
+  // The vertex bound is the ceiling. Every kDrainCheck iterations the
+  // live-slot count is copied into a host stack variable (a pageable copy:
+  // nothing is allocated), and the loop stops once the wavefront has drained
+  // or tr_cancel was called.
   constexpr int kDrainCheck = 16;  // even: the count read is the list the next iteration starts from
   ctx->cancel.store(0);
   long long it = 0;
