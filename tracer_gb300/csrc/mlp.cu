@@ -79,11 +79,36 @@ __global__ void k_pack(const float* __restrict__ p, uint8_t* __restrict__ img) {
 }
 constexpr int kPackThreads = 64 * 16 + 3 * 64 * 64 + 48 * 64 + 304;  // W0, W1..W3, W4, biases
 
-// x: n x 7 fp32; out: n x 40 fp32. With acts != null, the fp16 outputs of
-// the four hidden layers are stored too (acts[l][row][64]) for training.
+__device__ __forceinline__ uint32_t h2_bits(__half2 h) {
+  uint32_t u;
+  memcpy(&u, &h, 4);
+  return u;
+}
+// max(x, 0) of two values as fp16; NaN gives 0 (as fmaxf does)
+__device__ __forceinline__ uint32_t h2_relu(float a, float b) {
+  return h2_bits(__hmax2(__floats2half2_rn(a, b), __float2half2_rn(0.0f)));
+}
+
+// A hidden layer's epilogue for 32 of a row's columns: c = fp32 sums, plus
+// the bias, ReLU, fp16, into columns c0 .. c0 + 31 of the 64-column operand tile.
+__device__ __forceinline__ void hidden_epilogue(const uint32_t (&c)[32], const float* bias, uint8_t* tile, int row, int c0) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float4 b0 = reinterpret_cast<const float4*>(bias + c0)[2 * q], b1 = reinterpret_cast<const float4*>(bias + c0)[2 * q + 1];
+    const int k = 8 * q;
+    int4 h;
+    h.x = (int)h2_relu(__uint_as_float(c[k]) + b0.x, __uint_as_float(c[k + 1]) + b0.y);
+    h.y = (int)h2_relu(__uint_as_float(c[k + 2]) + b0.z, __uint_as_float(c[k + 3]) + b0.w);
+    h.z = (int)h2_relu(__uint_as_float(c[k + 4]) + b1.x, __uint_as_float(c[k + 5]) + b1.y);
+    h.w = (int)h2_relu(__uint_as_float(c[k + 6]) + b1.z, __uint_as_float(c[k + 7]) + b1.w);
+    *reinterpret_cast<int4*>(tile + tc05::core_off(row, c0 + k, kHid)) = h;
+  }
+}
+
+// x: n x 7 fp32; out: n x 40 fp32 (decode: the 48 mixture floats per row).
 __global__ void __launch_bounds__(128, 1)
-    k_forward(const uint8_t* __restrict__ img, const float* __restrict__ x, int n, float* __restrict__ out,
-              __half* __restrict__ acts, int* err, const unsigned int* __restrict__ n_dev, int decode) {
+    k_forward(const uint8_t* __restrict__ img, const float* __restrict__ x, int n, float* __restrict__ out, int* err,
+              const unsigned int* __restrict__ n_dev, int decode) {
   extern __shared__ __align__(1024) uint8_t sm[];
   if (n_dev) n = (int)*n_dev;  // row count produced on the device (guided rendering)
   const int tid = threadIdx.x, warp = tid >> 5;
@@ -119,15 +144,16 @@ __global__ void __launch_bounds__(128, 1)
     }
     tc05::fence_proxy_async();
     __syncthreads();
-    for (int l = 0; l < kLayers && ok; ++l) {
-      const int K = layer_k(l), N = layer_n(l);
+#pragma unroll
+    for (int l = 0; l < kLayers; ++l) {
       if (tid == 0) {
         tc05::fence_after();
-        const uint32_t sbo = (uint32_t)(K / 8) * 128u;
-        for (int kk = 0; kk < K / 16; ++kk)
-          tc05::mma_f16(tmem, tc05::smem_desc(a_addr + kk * 256u, 128u, sbo),
-                        tc05::smem_desc(w_addr + w_off(l) + kk * 256u, 128u, sbo),
-                        tc05::idesc_f16_f32(128, (uint32_t)N), kk > 0 ? 1u : 0u);
+        const uint32_t sbo = (uint32_t)(layer_k(l) / 8) * 128u;
+        const tc05::Desc a = tc05::desc_of(a_addr, 128u, sbo), w = tc05::desc_of(w_addr + w_off(l), 128u, sbo);
+#pragma unroll
+        for (int kk = 0; kk < layer_k(l) / 16; ++kk)
+          tc05::mma_f16(tmem, tc05::step(a, kk * 256u), tc05::step(w, kk * 256u),
+                        tc05::idesc_f16_f32(128, (uint32_t)layer_n(l)), kk > 0 ? 1u : 0u);
         tc05::commit(mbar);
       }
       const bool got = tc05::mbar_wait(mbar, phase);
@@ -136,20 +162,13 @@ __global__ void __launch_bounds__(128, 1)
       phase ^= 1u;
       tc05::fence_after();
       if (l < kLayers - 1) {
-        for (int c0 = 0; c0 < N; c0 += 16) {
-          float v[16];
-          tc05::tmem_ld16(tmem + lane_base + (uint32_t)c0, v);
-          __align__(16) __half h[16];
-#pragma unroll
-          for (int j = 0; j < 16; ++j) h[j] = __float2half_rn(fmaxf(v[j] + bias[l * 64 + c0 + j], 0.0f));
-          *reinterpret_cast<int4*>(A + tc05::core_off(tid, c0, kHid)) = *reinterpret_cast<const int4*>(h);
-          *reinterpret_cast<int4*>(A + tc05::core_off(tid, c0 + 8, kHid)) = *reinterpret_cast<const int4*>(h + 8);
-          if (acts && row < n) {
-            __half* dst = acts + ((size_t)l * n + row) * kHid + c0;
-            *reinterpret_cast<int4*>(dst) = *reinterpret_cast<const int4*>(h);
-            *reinterpret_cast<int4*>(dst + 8) = *reinterpret_cast<const int4*>(h + 8);
-          }
-        }
+        uint32_t c[32], d[32];
+        tc05::tmem_ld32(tmem + lane_base, c);
+        tc05::tmem_ld32(tmem + lane_base + 32u, d);
+        tc05::tmem_wait(c);
+        tc05::tmem_wait(d);
+        hidden_epilogue(c, bias + 64 * l, A, tid, 0);
+        hidden_epilogue(d, bias + 64 * l, A, tid, 32);
       } else {
         // the output row, whole in this thread: raw, or decoded into the
         // mixture's lobe parameters (guided rendering)
@@ -169,6 +188,10 @@ __global__ void __launch_bounds__(128, 1)
 #pragma unroll
             for (int q = 0; q < kMixFloats / 4; ++q)
               dst[q] = make_float4(dd[4 * q], dd[4 * q + 1], dd[4 * q + 2], dd[4 * q + 3]);
+          } else if (((uintptr_t)out & 15u) == 0) {
+            float4* dst = reinterpret_cast<float4*>(out + (size_t)row * kOut);
+#pragma unroll
+            for (int q = 0; q < kOut / 4; ++q) dst[q] = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
           } else {
 #pragma unroll
             for (int j = 0; j < kOut; ++j) out[(size_t)row * kOut + j] = o[j];
@@ -187,192 +210,6 @@ __global__ void __launch_bounds__(128, 1)
   __syncthreads();
   if (warp == 0) {
     tc05::tmem_dealloc(tmem, 64);
-  }
-}
-
-// ------------------------------------------------------------ backward
-//
-// For a 128-row tile and layer l = 4 .. 0, with in_l the layer's input
-// (x for l = 0, h_{l-1} otherwise):
-//   dW_l (+)= dZ_l^T in_l       M = 128 (rows of dZ^T: the layer's outputs,
-//                                zero-padded), N = 16 or 80, K = 128 rows;
-//                                in_l^T carries a row of ones after its
-//                                inputs, so the same MMA yields db_l
-//   dH     = dZ_l W_l           M = 128 rows, N = 64, K = 48 or 64
-//   dZ_{l-1} = dH * (h_{l-1} > 0)
-// dW accumulates in tensor memory over all tiles of the CTA and is added to
-// the global gradient once at the end.
-
-// transposed weights W_l^T (k_in x n_out, core layout, K = n_out padded) for l = 1..4
-__host__ __device__ constexpr uint32_t wt_off(int l) { return (uint32_t)(l - 1) * 8192u; }
-constexpr uint32_t kWtBytes = 3 * 8192 + 64 * 48 * 2;  // 30720
-__host__ __device__ constexpr int bk_n(int l) { return l == 0 ? 16 : 80; }                 // dW MMA N
-__host__ __device__ constexpr uint32_t bk_col(int l) { return l == 0 ? 64u : 80u + 80u * (uint32_t)(l - 1); }
-constexpr uint32_t kBDz = kWtBytes;                   // dZ tile, 128 x 64 (K = 48 or 64)
-constexpr uint32_t kBDzT = kBDz + 16384;              // dZ^T tile, 128 (outputs) x 128 (rows)
-constexpr uint32_t kBInT = kBDzT + 32768;             // in^T tile, 80 x 128
-constexpr uint32_t kBMbar = kBInT + 80 * 128 * 2;
-constexpr uint32_t kBSlot = kBMbar + 8;
-constexpr uint32_t kBSmemBytes = kBSlot + 8;
-
-__global__ void k_pack_t(const float* __restrict__ p, uint8_t* __restrict__ img) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;  // element (k, n) of W_l^T, l = 1..4
-  int base = 0;
-  for (int l = 1; l < kLayers; ++l) {
-    const int KK = layer_n(l);  // MMA K of dH: the layer's outputs (48 or 64)
-    if (i < base + 64 * KK) {
-      const int e = i - base, k = e / KK, n = e % KK;
-      const float v = n < layer_nout(l) ? p[param_w(l) + n * kHid + k] : 0.0f;
-      *reinterpret_cast<__half*>(img + wt_off(l) + tc05::core_off(k, n, KK)) = __float2half_rn(v);
-      return;
-    }
-    base += 64 * KK;
-  }
-}
-constexpr int kPackTThreads = 3 * 64 * 64 + 64 * 48;
-
-__device__ __forceinline__ void st_half(uint8_t* base, uint32_t off, float v) {
-  *reinterpret_cast<__half*>(base + off) = __float2half_rn(v);
-}
-
-// x: n x 7, acts: 4 x n x 64 (fp16, forward outputs of the hidden layers),
-// dout: n x 40 (gradient of the loss w.r.t. the network outputs).
-// grads (fp32, parameter layout) += this CTA's share.
-__global__ void __launch_bounds__(128, 1)
-    k_backward(const uint8_t* __restrict__ wt_img, const float* __restrict__ x, const __half* __restrict__ acts,
-               const float* __restrict__ dout, int n, float* __restrict__ grads, int* err) {
-  extern __shared__ __align__(1024) uint8_t sm[];
-  const int tid = threadIdx.x, warp = tid >> 5;
-  for (int i = tid; i < (int)(kWtBytes / 16); i += blockDim.x)
-    reinterpret_cast<int4*>(sm)[i] = reinterpret_cast<const int4*>(wt_img)[i];
-  for (int i = tid; i < (int)((kBMbar - kBDz) / 16); i += blockDim.x)
-    reinterpret_cast<int4*>(sm + kBDz)[i] = make_int4(0, 0, 0, 0);
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + kBMbar);
-  uint32_t* slot = reinterpret_cast<uint32_t*>(sm + kBSlot);
-  if (tid == 0) tc05::mbar_init(mbar, 1);
-  if (warp == 0) {
-    tc05::tmem_alloc(slot, 512);
-    tc05::tmem_relinquish();
-  }
-  tc05::fence_before();
-  __syncthreads();
-  tc05::fence_after();
-  const uint32_t tmem = *slot;
-  const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
-  uint8_t* Dz = sm + kBDz;
-  uint8_t* DzT = sm + kBDzT;
-  uint8_t* InT = sm + kBInT;
-  const uint32_t a_dz = tc05::smem_u32(Dz), a_dzt = tc05::smem_u32(DzT), a_int = tc05::smem_u32(InT),
-                 a_wt = tc05::smem_u32(sm);
-  uint32_t phase = 0;
-  bool ok = true;
-  int tiles_done = 0;
-  const int ntiles = (n + kTile - 1) / kTile;
-  for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-    const int r = tid, g = t * kTile + tid;
-    const bool live = g < n;
-    // layer 4: dZ4 = dout, in_4 = h3
-    float hin[64];  // in_l of the current layer (the ReLU mask of the next dZ)
-    {
-      float dz[48];
-#pragma unroll
-      for (int c = 0; c < 48; ++c) dz[c] = (live && c < kOut) ? dout[(size_t)g * kOut + c] : 0.0f;
-#pragma unroll
-      for (int c = 0; c < 48; ++c) st_half(Dz, tc05::core_off(r, c, 48), dz[c]);
-#pragma unroll
-      for (int c = 0; c < 64; ++c) st_half(DzT, tc05::core_off(c, r, 128), c < 48 ? dz[c] : 0.0f);
-    }
-#pragma unroll
-    for (int k = 0; k < 64; ++k) hin[k] = live ? __half2float(acts[((size_t)3 * n + g) * kHid + k]) : 0.0f;
-#pragma unroll
-    for (int k = 0; k < 80; ++k)
-      st_half(InT, tc05::core_off(k, r, 128), k < 64 ? hin[k] : (k == 64 && live ? 1.0f : 0.0f));
-    for (int l = kLayers - 1; l >= 0 && ok; --l) {
-      tc05::fence_proxy_async();
-      __syncthreads();
-      if (tid == 0) {
-        tc05::fence_after();
-        const uint32_t acc0 = tiles_done > 0 ? 1u : 0u;
-        for (int kk = 0; kk < 8; ++kk)
-          tc05::mma_f16(tmem + bk_col(l), tc05::smem_desc(a_dzt + kk * 256u, 128u, 2048u),
-                        tc05::smem_desc(a_int + kk * 256u, 128u, 2048u), tc05::idesc_f16_f32(128, bk_n(l)),
-                        (acc0 || kk > 0) ? 1u : 0u);
-        if (l > 0) {
-          const int KK = layer_n(l);
-          const uint32_t sbo = (uint32_t)(KK / 8) * 128u;
-          for (int kk = 0; kk < KK / 16; ++kk)
-            tc05::mma_f16(tmem, tc05::smem_desc(a_dz + kk * 256u, 128u, sbo),
-                          tc05::smem_desc(a_wt + wt_off(l) + kk * 256u, 128u, sbo), tc05::idesc_f16_f32(128, 64),
-                          kk > 0 ? 1u : 0u);
-        }
-        tc05::commit(mbar);
-      }
-      const bool got = tc05::mbar_wait(mbar, phase);
-      ok = __syncthreads_and(got) != 0;
-      if (!ok) break;
-      phase ^= 1u;
-      if (l == 0) break;
-      tc05::fence_after();
-      // dZ_{l-1} = dH * (h_{l-1} > 0); h_{l-1} is this layer's input (hin)
-      float dz[64];
-#pragma unroll
-      for (int c0 = 0; c0 < 64; c0 += 16) {
-        float v[16];
-        tc05::tmem_ld16(tmem + lane_base + (uint32_t)c0, v);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) dz[c0 + j] = hin[c0 + j] > 0.0f ? v[j] : 0.0f;
-      }
-      tc05::fence_before();
-#pragma unroll
-      for (int c = 0; c < 64; ++c) st_half(Dz, tc05::core_off(r, c, 64), dz[c]);
-#pragma unroll
-      for (int c = 0; c < 64; ++c) st_half(DzT, tc05::core_off(c, r, 128), dz[c]);
-      // the input of layer l-1
-      if (l - 1 > 0) {
-#pragma unroll
-        for (int k = 0; k < 64; ++k)
-          hin[k] = live ? __half2float(acts[((size_t)(l - 2) * n + g) * kHid + k]) : 0.0f;
-#pragma unroll
-        for (int k = 0; k < 80; ++k)
-          st_half(InT, tc05::core_off(k, r, 128), k < 64 ? hin[k] : (k == 64 && live ? 1.0f : 0.0f));
-      } else {
-#pragma unroll
-        for (int k = 0; k < 16; ++k)
-          st_half(InT, tc05::core_off(k, r, 128),
-                  k < kIn ? (live ? x[(size_t)g * kIn + k] : 0.0f) : (k == kIn && live ? 1.0f : 0.0f));
-      }
-    }
-    ++tiles_done;
-  }
-  if (!ok) {
-    if (tid == 0) atomicOr(err, 1);
-    tc05::mbar_wait(mbar, phase);
-  }
-  __syncthreads();
-  tc05::fence_after();
-  if (ok && tiles_done > 0 && warp < 2) {
-    // rows (lanes) 0..63 of the dW accumulators: output unit `o` of each layer
-    const int o = tid;
-    for (int l = 0; l < kLayers; ++l) {
-      const int N = bk_n(l), kin = layer_kin(l);
-      for (int c0 = 0; c0 < N; c0 += 16) {
-        float v[16];
-        tc05::tmem_ld16(tmem + lane_base + bk_col(l) + (uint32_t)c0, v);
-        if (o < layer_nout(l)) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int k = c0 + j;
-            if (k < kin) atomicAdd(grads + param_w(l) + o * kin + k, v[j]);
-            else if (k == kin) atomicAdd(grads + param_b(l) + o, v[j]);
-          }
-        }
-      }
-    }
-  }
-  tc05::fence_before();
-  __syncthreads();
-  if (warp == 0) {
-    tc05::tmem_dealloc(tmem, 512);
   }
 }
 
@@ -395,19 +232,27 @@ __device__ __forceinline__ float vmf_log_norm(float kappa) {
   return logf(kappa) - 1.8378770664093453f - log1pf(-expf(-2.0f * kappa));
 }
 
-// log p(omega | z) of one row, and d[0..39] = the gradient of -wi log p
-// w.r.t. the row's 40 network outputs z.
-__device__ __forceinline__ float row_nll_grad(const float* z, float3 om, float wi, float* d) {
+// log p(omega | z) of one row, and the gradient of -wi log p w.r.t. the row's
+// network outputs z. The lobes may be split over several threads: this thread
+// has LOBES of them (z, d: their 5 * LOBES outputs), and `all` combines a
+// partial maximum (max) or sum over the row's threads.
+template <int LOBES, class All>
+__device__ __forceinline__ float row_nll_grad(const float* z, float3 om, float wi, float* d, All all) {
   float a_max = -INFINITY;
-  for (int j = 0; j < kLobes; ++j) a_max = fmaxf(a_max, z[5 * j]);
-  float esum = 0.0f, lq[kLobes], pi[kLobes];
-  for (int j = 0; j < kLobes; ++j) {
+#pragma unroll
+  for (int j = 0; j < LOBES; ++j) a_max = fmaxf(a_max, z[5 * j]);
+  a_max = all(a_max, true);
+  float esum = 0.0f, lq[LOBES], pi[LOBES];
+#pragma unroll
+  for (int j = 0; j < LOBES; ++j) {
     pi[j] = expf(z[5 * j] - a_max);
     esum += pi[j];
   }
+  esum = all(esum, false);
   float lmax = -INFINITY;
-  Lobe L[kLobes];
-  for (int j = 0; j < kLobes; ++j) {
+  Lobe L[LOBES];
+#pragma unroll
+  for (int j = 0; j < LOBES; ++j) {
     pi[j] /= esum;
     const float s = fminf(fmaxf(z[5 * j + 1], TR_GUIDE_LOG_KAPPA_MIN), TR_GUIDE_LOG_KAPPA_MAX);
     const float kappa = expf(s);
@@ -419,10 +264,13 @@ __device__ __forceinline__ float row_nll_grad(const float* z, float3 om, float w
     lq[j] = logf(fmaxf(pi[j], 1e-30f)) + vmf_log_norm(kappa) + kappa * (c - 1.0f);
     lmax = fmaxf(lmax, lq[j]);
   }
+  lmax = all(lmax, true);
   float qs = 0.0f;
-  for (int j = 0; j < kLobes; ++j) qs += expf(lq[j] - lmax);
-  const float logp = lmax + logf(qs);
-  for (int j = 0; j < kLobes; ++j) {
+#pragma unroll
+  for (int j = 0; j < LOBES; ++j) qs += expf(lq[j] - lmax);
+  const float logp = lmax + logf(all(qs, false));
+#pragma unroll
+  for (int j = 0; j < LOBES; ++j) {
     const float q = expf(lq[j] - logp);  // responsibility
     const Lobe& b = L[j];
     d[5 * j] = -wi * (q - b.pi);
@@ -445,7 +293,8 @@ __global__ void k_loss(const float* __restrict__ out, const float* __restrict__ 
   if (i < n) {
     const float3 om = make_float3(dir[3 * i], dir[3 * i + 1], dir[3 * i + 2]);
     const float wi = w[i] / fmaxf(*wsum, 1e-30f);
-    li = -wi * row_nll_grad(out + (size_t)i * kOut, om, wi, dout + (size_t)i * kOut);
+    li = -wi * row_nll_grad<kLobes>(out + (size_t)i * kOut, om, wi, dout + (size_t)i * kOut,
+                                    [](float v, bool) { return v; });
   }
   // block sum of the loss
   for (int o = 16; o > 0; o >>= 1) li += __shfl_xor_sync(0xffffffffu, li, o);
@@ -459,59 +308,69 @@ __global__ void k_sum(const float* __restrict__ w, int n, float* __restrict__ ou
   if ((threadIdx.x & 31) == 0) atomicAdd(out, s);
 }
 
-__global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, float lr, float c1, float c2) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kParams) return;
-  const float gi = g[i];
-  const float mi = 0.9f * m[i] + 0.1f * gi;
-  const float vi = 0.999f * v[i] + 0.001f * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + 1e-8f);
-}
-
 // ------------------------------------------------------------ fused training step
 //
-// One Adam step on a batch is two launches: k_train and k_update.
+// One Adam step on a batch is two launches: k_train and k_update; a gradient
+// for given output gradients is k_train<false> and k_grad_sum.
 //
-// k_train does the batch's forward pass, loss and backward pass on the
-// tensor cores. CTAs (one per SM, 256 threads, all 512 TMEM columns) walk
-// 128-row tiles. A tile's rows are gathered from the record arrays; each
-// layer's input is kept in shared memory twice, as the forward MMA's A
-// operand and transposed (in_l^T) as the B operand of the weight-gradient
-// MMA; the last layer's epilogue evaluates the loss and its gradient; the
-// backward chain is the one of k_backward, with the ReLU masks held in
-// registers. Weight gradients accumulate in TMEM over the CTA's tiles and are
-// written once per CTA as a partial sum (no atomics).
+// k_train does a batch's forward pass, loss (or takes the outputs' gradient)
+// and backward pass on the tensor cores. For a 128-row tile and layer l, with
+// in_l the layer's input (x for l = 0, h_{l-1} otherwise):
+//   Z_l    = in_l W_l^T          M = 128 rows, N = 64 or 48, K = 16 or 64
+//   dW_l (+)= dZ_l^T in_l        M = 128 (64 outputs used), N = 16 or 64, K = 128 rows
+//   db_l (+)= dZ_l^T 1           N = 16, a constant tile of ones (layer 0: a column of in_0)
+//   dH     = dZ_l W_l            M = 128 rows, N = 64, K = 48 or 64
+//   dZ_{l-1} = dH * (h_{l-1} > 0)
+// A tile's in_l, its dZ and the weights lie in shared memory once, in the
+// core-matrix layout; the products that need them transposed read the same
+// bytes as MN-major operands (tc05.cuh). dW accumulates in tensor memory over
+// the CTA's tiles and is written once per CTA as a partial sum (no atomics);
+// k_update or k_grad_sum add the partials in a fixed order, so a step is
+// deterministic.
 //
-// k_update sums the partials in a fixed order (the step is deterministic),
-// takes the Adam step and writes the updated fp16 weights and fp32 biases
-// into both packed images in place.
+// A tile is a chain of ten dependent MMAs and epilogues of a microsecond or
+// two each, so a CTA (one per SM: the accumulators take 464 of the 512 TMEM
+// columns) works on two tiles at once: two groups of four warps (a row per
+// thread) run the epilogues and one thread of a ninth warp issues both
+// groups' MMAs, each group's while the other's epilogue runs. The first
+// version kept one tile per CTA with a __syncthreads per step and stored
+// every activation and gradient a second time transposed (80 two-byte stores
+// per row and layer): 93 us for 65,536 rows, 45 now; the gradient of 100,003
+// rows 51 us instead of about 250 with stored activations. The MMA thread is
+// busy 60% of that time: a product of 64 or 16 columns reads its 4 KB of A per
+// 16 rows at shared-memory speed.
 //
 // Loss weighting: loss = sum_i -w_i log p_i / sum_i w_i. The rows carry
 // s * w_i into the fp16 gradient chain, s = N / (64 W) for the weight sum W
 // of N rows (the whole record set, or the batch), so the per-row values sit
 // in fp16's normal range; k_update divides by s * sum_i w_i.
 
-constexpr uint32_t kTWt = 34048;                           // transposed weights, kWtBytes
-constexpr uint32_t kTA = kTWt + kWtBytes;                  // forward A operand / backward dZ (128 x 64)
-constexpr uint32_t kTDzT = kTA + kTile * kHid * 2;         // dZ^T (128 x 128)
-constexpr uint32_t kTIn = kTDzT + 128 * kTile * 2;         // in_l^T, l = 0..4
-__host__ __device__ constexpr uint32_t tin_off(int l) {
-  return l == 0 ? kTIn : kTIn + (uint32_t)kInPad * kTile * 2 + (uint32_t)(l - 1) * 80u * kTile * 2;
+constexpr uint32_t kTOnes = 34048;                          // 128 x 16, column 0 one
+constexpr uint32_t kTGroup = kTOnes + kTile * 16 * 2;       // per group: in_0, in_1..in_4, dZ
+constexpr uint32_t kTileBytes = kTile * kHid * 2;           // 128 x 64 fp16
+constexpr uint32_t kIn0Bytes = kTile * kInPad * 2;
+constexpr uint32_t kGroupBytes = kIn0Bytes + 5 * kTileBytes;
+__host__ __device__ constexpr uint32_t tin_off(int g, int l) {
+  return kTGroup + (uint32_t)g * kGroupBytes + (l == 0 ? 0u : kIn0Bytes + (uint32_t)(l - 1) * kTileBytes);
 }
-constexpr uint32_t kTRed = tin_off(4) + 80u * kTile * 2;   // block-reduction scratch
-constexpr uint32_t kTMbar = kTRed + 64;
-constexpr uint32_t kTSlot = kTMbar + 8;
-constexpr uint32_t kTSmemBytes = kTSlot + 8;
-static_assert(kPackedBytes <= kTWt && kTWt % 128 == 0 && kTA % 128 == 0 && kTIn % 128 == 0, "k_train layout");
+__host__ __device__ constexpr uint32_t tdz_off(int g) { return tin_off(g, 5); }
+// M = 128 reads 64 outputs beyond dZ's columns: the next row group, at the
+// tile's end 1 KB past it (their products land in unused TMEM lanes)
+constexpr uint32_t kTRed = kTGroup + 2 * kGroupBytes + 1024;  // per-warp sums
+constexpr uint32_t kTXch = kTRed + 128;                     // per group: the two halves' partial values of a row
+constexpr uint32_t kTMbar = kTXch + 2 * 2 * kTile * 4;      // ready[2], done[2], drain
+constexpr uint32_t kTSlot = kTMbar + 5 * 8;
+constexpr uint32_t kTSmemBytes = kTSlot + 16;
+static_assert(kPackedBytes <= kTOnes && kTOnes % 128 == 0 && kTGroup % 128 == 0 && kTRed % 128 == 0, "k_train layout");
 static_assert(kTSmemBytes <= 227 * 1024, "k_train shared memory");
+// TMEM columns: a 64-column accumulator per group, then the weight gradients
+__host__ __device__ constexpr uint32_t dw_col(int l) { return l == 0 ? 128u : 144u + 80u * (uint32_t)(l - 1); }
+static_assert(dw_col(4) + 80 <= 512, "k_train tensor memory");
 constexpr int kPartStride = kParams + 16;  // per-CTA partial: gradients, then weight sum and loss sum
 constexpr int kWsumParts = 128;            // blocks of k_wsum
 constexpr float kRowScale = 1.0f / 64.0f;
-constexpr int kTrainThreads = 256;         // k_train: two warps per TMEM lane quarter
-static_assert(kTRed + 8 * kTrainThreads / 32 <= kTMbar, "k_train reduction scratch");
+constexpr int kGroupThreads = 256;
+constexpr int kTrainThreads = 2 * kGroupThreads + 32;  // two groups and the MMA warp
 
 // The batch's row i: a record index drawn by a hash of (seed, i).
 __device__ __forceinline__ unsigned int batch_record(unsigned long long seed, unsigned int i, unsigned int count) {
@@ -536,236 +395,308 @@ __global__ void k_wsum(const float* __restrict__ w, unsigned int n, float* __res
   if (threadIdx.x == 0) parts[blockIdx.x] = red[0];
 }
 
-// The row scale s = nrows / (64 W) from k_wsum's partial sums, in a fixed order.
-__global__ void k_scale(const float* __restrict__ parts, float nrows, float* __restrict__ scale) {
+// The row scale s = nrows / (64 W) from k_wsum's partial sums, in a fixed
+// order (every thread of a block of at least kWsumParts calls it).
+__device__ __forceinline__ float row_scale(const float* __restrict__ parts, float nrows, int tid) {
   __shared__ float red[kWsumParts];
-  red[threadIdx.x] = parts[threadIdx.x];
+  if (tid < kWsumParts) red[tid] = parts[tid];
   __syncthreads();
   for (int o = kWsumParts / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+    if (tid < o) red[tid] += red[tid + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) *scale = nrows * kRowScale / fmaxf(red[0], 1e-30f);
+  return nrows * kRowScale / fmaxf(red[0], 1e-30f);
 }
 
-__device__ __forceinline__ __half sat_half(float v) {
-  return __float2half_rn(fminf(fmaxf(v, -65504.0f), 65504.0f));
+// Two gradient values as fp16, clamped to the finite range with SAT (NaN to
+// its lower end, as fminf(fmaxf()) does).
+template <bool SAT>
+__device__ __forceinline__ uint32_t h2_grad(float a, float b) {
+  __half2 h = __floats2half2_rn(a, b);
+  if (SAT) h = __hmin2(__hmax2(h, __float2half2_rn(-65504.0f)), __float2half2_rn(65504.0f));
+  return h2_bits(h);
+}
+// The halves of u where those of h are not zero (h: ReLU outputs).
+__device__ __forceinline__ uint32_t h2_where(uint32_t u, uint32_t h) {
+  return u & ((h & 0x7fffu ? 0xffffu : 0u) | (h & 0x7fff0000u ? 0xffff0000u : 0u));
+}
+// Meets the other threads of one group of k_train.
+__device__ __forceinline__ void group_sync(int g) {
+  asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(256) : "memory");
 }
 
-// rec_in: count x 7, rec_dir: count x 3, rec_w: count. gather != 0: row i of
-// the batch is record batch_record(seed, i, count); else record i.
-// part: gridDim.x x kPartStride floats.
-//
-// Eight warps: warp w reads TMEM lanes 32 (w % 4) .. + 31, so threads t and
-// t + 128 own the same tile row; in the epilogues of the hidden layers and of
-// the backward chain each of the two takes half of the row's 64 columns
-// (grp = w / 4). The loss epilogue, which needs a whole output row, runs on
-// the first four warps.
+// The MMAs of one step of a tile: forward layer L, and backward layer L.
+template <int L>
+__device__ __forceinline__ void train_forward_mma(uint32_t sm, uint32_t tmem, int g) {
+  constexpr uint32_t sbo = (uint32_t)(layer_k(L) / 8) * 128u;
+  const tc05::Desc in = tc05::desc_of(sm + tin_off(g, L), 128u, sbo), w = tc05::desc_of(sm + w_off(L), 128u, sbo);
+#pragma unroll
+  for (uint32_t kk = 0; kk < layer_k(L) / 16; ++kk)
+    tc05::mma_f16(tmem + 64u * (uint32_t)g, tc05::step(in, kk * 256u), tc05::step(w, kk * 256u),
+                  tc05::idesc_f16_f32(128, (uint32_t)layer_n(L)), kk > 0 ? 1u : 0u);
+}
+template <int L>
+__device__ __forceinline__ void train_backward_mma(uint32_t sm, uint32_t tmem, int g, bool first) {
+  constexpr uint32_t cols = L == 0 ? kInPad : kHid;
+  const uint32_t dz = sm + tdz_off(g);
+  const tc05::Desc a = tc05::desc_of(dz, 1024u, 128u), in = tc05::desc_of(sm + tin_off(g, L), cols * 16u, 128u),
+                   one = tc05::desc_of(sm + kTOnes, 256u, 128u);
+  if (L > 0) {  // first: the group's next epilogue waits for it
+    const tc05::Desc ak = tc05::desc_of(dz, 128u, 1024u), w = tc05::desc_of(sm + w_off(L), 1024u, 128u);
+#pragma unroll
+    for (uint32_t kk = 0; kk < layer_n(L) / 16; ++kk)
+      tc05::mma_f16(tmem + 64u * (uint32_t)g, tc05::step(ak, kk * 256u), tc05::step(w, kk * 2048u),
+                    tc05::idesc_f16_f32(128, 64) | tc05::kTransB, kk > 0 ? 1u : 0u);
+  }
+#pragma unroll
+  for (uint32_t kk = 0; kk < kTile / 16; ++kk) {
+    const uint32_t acc = (!first || kk > 0) ? 1u : 0u;
+    tc05::mma_f16(tmem + dw_col(L), tc05::step(a, kk * 2048u), tc05::step(in, kk * cols * 32u),
+                  tc05::idesc_f16_f32(128, cols) | tc05::kTransA | tc05::kTransB, acc);
+    if (L > 0)
+      tc05::mma_f16(tmem + dw_col(L) + 64u, tc05::step(a, kk * 2048u), tc05::step(one, kk * 512u),
+                    tc05::idesc_f16_f32(128, 16) | tc05::kTransA | tc05::kTransB, acc);
+  }
+}
+// Step `step` of a tile: the forward layers 0 .. FWD - 1, then the backward
+// layers 4 .. 0.
+template <int FWD>
+__device__ __forceinline__ void train_mma(int step, uint32_t sm, uint32_t tmem, int g, bool first) {
+  switch (step) {
+    case 0: train_forward_mma<0>(sm, tmem, g); return;
+    case 1: train_forward_mma<1>(sm, tmem, g); return;
+    case 2: train_forward_mma<2>(sm, tmem, g); return;
+    case 3: train_forward_mma<3>(sm, tmem, g); return;
+    case 4: if (FWD == 5) { train_forward_mma<4>(sm, tmem, g); return; }
+  }
+  switch (step - FWD) {
+    case 0: train_backward_mma<4>(sm, tmem, g, first); return;
+    case 1: train_backward_mma<3>(sm, tmem, g, first); return;
+    case 2: train_backward_mma<2>(sm, tmem, g, first); return;
+    case 3: train_backward_mma<1>(sm, tmem, g, first); return;
+    default: train_backward_mma<0>(sm, tmem, g, first);
+  }
+}
+
+// LOSS: rin: count x 7, rdir: count x 3, rw: count; gather != 0: row i of the
+// batch is record batch_record(seed, i, count), else record i. Otherwise rin
+// and rdir are the n inputs and the n x 40 gradients of the outputs.
+// wparts: k_wsum's sums over the wrows weights. part: gridDim.x x kPartStride floats.
+template <bool LOSS>
 __global__ void __launch_bounds__(kTrainThreads, 1)
-    k_train(const uint8_t* __restrict__ img, const uint8_t* __restrict__ img_t, const float* __restrict__ rin,
-            const float* __restrict__ rdir, const float* __restrict__ rw, unsigned int count, int n,
-            unsigned long long seed, int gather, const float* __restrict__ scale, float* __restrict__ part,
-            int* err) {
+    k_train(const uint8_t* __restrict__ img, const float* __restrict__ rin, const float* __restrict__ rdir,
+            const float* __restrict__ rw, unsigned int count, int n, unsigned long long seed, int gather,
+            const float* __restrict__ wparts, float wrows, float* __restrict__ part, int* err) {
   extern __shared__ __align__(1024) uint8_t sm[];
   const int tid = threadIdx.x, warp = tid >> 5;
-  const int grp = warp >> 2;                         // column half of the epilogues
-  const int r = ((warp & 3) << 5) | (tid & 31);      // this thread's tile row (TMEM lane)
-  for (int i = tid; i < (int)(kPackedBytes / 16); i += blockDim.x)
+  const int grp = warp >> 3;        // 0, 1: epilogue groups; 2: the MMA warp
+  const int half = (warp >> 2) & 1;  // which half of the row's columns is this thread's
+  const int r = tid & (kTile - 1);   // this thread's tile row (TMEM lane)
+  for (int i = tid; i < (int)(kPackedBytes / 16); i += kTrainThreads)
     reinterpret_cast<int4*>(sm)[i] = reinterpret_cast<const int4*>(img)[i];
-  for (int i = tid; i < (int)(kWtBytes / 16); i += blockDim.x)
-    reinterpret_cast<int4*>(sm + kTWt)[i] = reinterpret_cast<const int4*>(img_t)[i];
-  // operands start zero: padding rows and columns are never written again
-  for (int i = tid; i < (int)((kTRed - kTA) / 16); i += blockDim.x)
-    reinterpret_cast<int4*>(sm + kTA)[i] = make_int4(0, 0, 0, 0);
+  // the ones tile: column 0 (the other operands are written whole for every tile)
+  if (tid < kTile) {
+    uint8_t* one = sm + kTOnes;
+    *reinterpret_cast<int4*>(one + tc05::core_off(tid, 0, 16)) = make_int4(0x3c00, 0, 0, 0);  // 1.0 in fp16
+    *reinterpret_cast<int4*>(one + tc05::core_off(tid, 8, 16)) = make_int4(0, 0, 0, 0);
+  }
   uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + kTMbar);
+  uint64_t *ready = mbar, *done = mbar + 2, *drain = mbar + 4;
   uint32_t* slot = reinterpret_cast<uint32_t*>(sm + kTSlot);
-  if (tid == 0) tc05::mbar_init(mbar, 1);
-  if (warp == 0) {
+  int* failed = reinterpret_cast<int*>(sm + kTSlot + 4);
+  if (tid == 0) {
+    for (int g = 0; g < 2; ++g) {
+      tc05::mbar_init(ready + g, kGroupThreads);
+      tc05::mbar_init(done + g, 1);
+    }
+    tc05::mbar_init(drain, 1);
+    *failed = 0;
+  }
+  if (warp == 16) {
     tc05::tmem_alloc(slot, 512);
     tc05::tmem_relinquish();
   }
   tc05::fence_before();
+  tc05::fence_proxy_async();
   __syncthreads();
   tc05::fence_after();
   const uint32_t tmem = *slot;
-  const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-  const float* bias = reinterpret_cast<const float*>(sm + kBiasOff);
-  uint8_t* A = sm + kTA;
-  uint8_t* DzT = sm + kTDzT;
-  const uint32_t w_addr = tc05::smem_u32(sm), wt_addr = tc05::smem_u32(sm + kTWt), a_addr = tc05::smem_u32(A),
-                 dzt_addr = tc05::smem_u32(DzT);
-  const float s = *scale;
+  const uint32_t smem = tc05::smem_u32(sm);
+  const int ntiles = (n + kTile - 1) / kTile, stride = 2 * (int)gridDim.x;
+  constexpr int kFwd = LOSS ? 5 : 4;  // without a loss the outputs are not needed
+  const float s = LOSS ? row_scale(wparts, wrows, tid) : 1.0f;
   float w_acc = 0.0f, l_acc = 0.0f;
-  uint32_t phase = 0;
-  bool ok = true;
-  int tiles_done = 0;
-  const int ntiles = (n + kTile - 1) / kTile;
-  for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-    const int i = t * kTile + r;
-    const bool live = i < n;
-    float x[kIn], om[3], w = 0.0f;
-    {
-      const unsigned int j = live ? (gather ? batch_record(seed, (unsigned int)i, count) : (unsigned int)i) : 0u;
+  if (grp == 2) {
+    if (tid == 2 * kGroupThreads) {
+      uint32_t phase[2] = {0u, 0u};
+      bool ok = true, first = true;
+      for (int t = blockIdx.x; t < ntiles && ok; t += stride) {
+        const int groups = t + (int)gridDim.x < ntiles ? 2 : 1;
+        for (int step = 0; step < kFwd + 5 && ok; ++step)
+          for (int g = 0; g < groups && ok; ++g) {
+            ok = tc05::mbar_wait(ready + g, phase[g]);
+            if (!ok) break;
+            phase[g] ^= 1u;
+            tc05::fence_after();
+            train_mma<kFwd>(step, smem, tmem, g, first && g == 0);
+            tc05::commit(done + g);
+          }
+        first = false;
+      }
+      if (!ok) {
+        *failed = 1;
+        tc05::commit(drain);
+        tc05::mbar_wait(drain, 0u);  // bounded: let the MMAs in flight finish
+      }
+    }
+    __syncwarp();
+  } else {
+    const uint32_t acc = tmem + 64u * (uint32_t)grp + ((uint32_t)((warp & 3) * 32) << 16);
+    const float* bias = reinterpret_cast<const float*>(sm + kBiasOff);
+    uint8_t* dZ = sm + tdz_off(grp);
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int t = blockIdx.x + grp * (int)gridDim.x; t < ntiles && ok; t += stride) {
+      const int i = t * kTile + r;
+      const bool live = i < n;
+      float x[kIn], om[3] = {0.0f, 0.0f, 0.0f}, w = 0.0f;
+      const unsigned int j =
+          live ? (LOSS && gather ? batch_record(seed, (unsigned int)i, count) : (unsigned int)i) : 0u;
 #pragma unroll
       for (int k = 0; k < kIn; ++k) x[k] = live ? rin[(size_t)j * kIn + k] : 0.0f;
+      if (LOSS && live) {
 #pragma unroll
-      for (int k = 0; k < 3; ++k) om[k] = live ? rdir[(size_t)j * 3 + k] : 0.0f;
-      if (live) w = rw[j];
-    }
-    // layer 0's input: the A operand (zero-padded to 16; first four warps) and
-    // in_0^T (ones row at 7 for the bias; last four)
-    if (grp == 0) {
-      __align__(16) __half h[16];
-#pragma unroll
-      for (int k = 0; k < 16; ++k) h[k] = __float2half_rn(k < kIn ? x[k] : 0.0f);
-      *reinterpret_cast<int4*>(A + tc05::core_off(r, 0, kInPad)) = *reinterpret_cast<const int4*>(h);
-      *reinterpret_cast<int4*>(A + tc05::core_off(r, 8, kInPad)) = *reinterpret_cast<const int4*>(h + 8);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 16; ++k)
-        st_half(sm + tin_off(0), tc05::core_off(k, r, kTile), k < kIn ? x[k] : (k == kIn && live ? 1.0f : 0.0f));
-    }
-    uint32_t mask[4];  // ReLU masks (h > 0 in fp16) of this thread's 32 hidden units per layer
-    tc05::fence_proxy_async();
-    __syncthreads();
-    // ---- forward
-    for (int l = 0; l < kLayers && ok; ++l) {
-      const int K = layer_k(l), N = layer_n(l);
-      if (tid == 0) {
-        tc05::fence_after();
-        const uint32_t sbo = (uint32_t)(K / 8) * 128u;
-        for (int kk = 0; kk < K / 16; ++kk)
-          tc05::mma_f16(tmem, tc05::smem_desc(a_addr + kk * 256u, 128u, sbo),
-                        tc05::smem_desc(w_addr + w_off(l) + kk * 256u, 128u, sbo),
-                        tc05::idesc_f16_f32(128, (uint32_t)N), kk > 0 ? 1u : 0u);
-        tc05::commit(mbar);
+        for (int k = 0; k < 3; ++k) om[k] = rdir[(size_t)j * 3 + k];
+        w = rw[j];
       }
-      const bool got = tc05::mbar_wait(mbar, phase);
-      ok = __syncthreads_and(got) != 0;
-      if (!ok) break;
-      phase ^= 1u;
-      tc05::fence_after();
-      if (l < kLayers - 1) {
-        uint8_t* inT = sm + tin_off(l + 1);
-        uint32_t mk = 0u;
+      {  // in_0: the inputs, a one for the bias gradient (its weights are zero), zeros; eight columns a thread
+        __align__(16) __half h[8];
 #pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          const int c0 = 32 * grp + 16 * hf;
-          float v[16];
-          tc05::tmem_ld16(tmem + lane_base + (uint32_t)c0, v);
-          __align__(16) __half h[16];
+        for (int k = 0; k < 8; ++k) h[k] = __float2half_rn(half ? 0.0f : (k < kIn ? x[k < kIn ? k : 0] : 1.0f));
+        *reinterpret_cast<int4*>(sm + tin_off(grp, 0) + tc05::core_off(r, 8 * half, kInPad)) =
+            *reinterpret_cast<const int4*>(h);
+      }
+      tc05::fence_proxy_async();
+      tc05::mbar_arrive(ready + grp);
+      const int c0 = 32 * half;
+      // ---- forward
+      for (int l = 0; l < 4; ++l) {
+        ok = ok && tc05::mbar_wait(done + grp, phase);
+        phase ^= 1u;
+        tc05::fence_after();
+        uint32_t c[32];
+        tc05::tmem_ld32(acc + (uint32_t)c0, c);
+        tc05::tmem_wait(c);
+        hidden_epilogue(c, bias + 64 * l, sm + tin_off(grp, l + 1), r, c0);
+        if (LOSS || l < 3) {
+          tc05::fence_before();
+          tc05::fence_proxy_async();
+          tc05::mbar_arrive(ready + grp);
+        }
+      }
+      {  // dZ_4: the loss and its gradient w.r.t. the outputs, or the given gradient (20 outputs a thread)
+        constexpr int kMine = kOut / 2;
+        float d[kMine];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            h[j] = __float2half_rn(fmaxf(v[j] + bias[l * 64 + c0 + j], 0.0f));
-            if (__half2float(h[j]) > 0.0f) mk |= 1u << (16 * hf + j);
-            *reinterpret_cast<__half*>(inT + tc05::core_off(c0 + j, r, kTile)) = h[j];
+        for (int k = 0; k < kMine; ++k) d[k] = 0.0f;
+        if (LOSS) {
+          ok = ok && tc05::mbar_wait(done + grp, phase);
+          phase ^= 1u;
+          tc05::fence_after();
+          uint32_t c[32];
+          tc05::tmem_ld32(acc + (uint32_t)(kMine * half), c);
+          tc05::tmem_wait(c);
+          float z[kMine];
+#pragma unroll
+          for (int k = 0; k < kMine; ++k) z[k] = __uint_as_float(c[k]) + bias[256 + kMine * half + k];
+          float* xch = reinterpret_cast<float*>(sm + kTXch) + 2 * kTile * grp;
+          const float logp = row_nll_grad<kLobes / 2>(
+              z, make_float3(om[0], om[1], om[2]), w * s, d, [&](float v, bool max) {
+                group_sync(grp);
+                xch[kTile * half + r] = v;
+                group_sync(grp);
+                const float a = xch[r], b = xch[kTile + r];
+                return max ? fmaxf(a, b) : a + b;
+              });
+          if (live && half == 0) {
+            w_acc += w;
+            l_acc -= w * logp;
           }
-          *reinterpret_cast<int4*>(A + tc05::core_off(r, c0, kHid)) = *reinterpret_cast<const int4*>(h);
-          *reinterpret_cast<int4*>(A + tc05::core_off(r, c0 + 8, kHid)) = *reinterpret_cast<const int4*>(h + 8);
+        } else if (live) {
+#pragma unroll
+          for (int k = 0; k < kMine; ++k) d[k] = rdir[(size_t)i * kOut + kMine * half + k];
         }
-        mask[l] = mk;
-        if (grp == 1) st_half(inT, tc05::core_off(kHid, r, kTile), live ? 1.0f : 0.0f);
-      } else if (grp == 0) {
-        // loss and its gradient w.r.t. the outputs: dZ_4 into dZ (K = 48) and dZ^T
-        float z[kOutPad];
+        // columns 20 half .. + 19, in pairs (zeros from column 40 on stay)
 #pragma unroll
-        for (int c = 0; c < kOutPad / 16; ++c) {
-          float v[16];
-          tc05::tmem_ld16(tmem + lane_base + (uint32_t)(16 * c), v);
+        for (int k = 0; k < kMine; k += 2)
+          *reinterpret_cast<uint32_t*>(dZ + tc05::core_off(r, kMine * half + k, kHid)) =
+              live ? h2_grad<LOSS>(d[k], d[k + 1]) : 0u;
+        if (half == 1) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) z[16 * c + j] = 16 * c + j < kOut ? v[j] + bias[256 + 16 * c + j] : 0.0f;
+          for (int k = kOut; k < kHid; k += 8)
+            *reinterpret_cast<int4*>(dZ + tc05::core_off(r, k, kHid)) = make_int4(0, 0, 0, 0);
         }
-        float d[kOut];
-        if (live) {
-          const float logp = row_nll_grad(z, make_float3(om[0], om[1], om[2]), w * s, d);
-          w_acc += w;
-          l_acc -= w * logp;
-        } else {
-#pragma unroll
-          for (int c = 0; c < kOut; ++c) d[c] = 0.0f;
-        }
-#pragma unroll
-        for (int c = 0; c < kOutPad; ++c)
-          *reinterpret_cast<__half*>(A + tc05::core_off(r, c, kOutPad)) = sat_half(c < kOut ? d[c] : 0.0f);
-#pragma unroll
-        for (int c = 0; c < kHid; ++c)
-          *reinterpret_cast<__half*>(DzT + tc05::core_off(c, r, kTile)) = sat_half(c < kOut ? d[c] : 0.0f);
+        tc05::fence_before();
+        tc05::fence_proxy_async();
+        tc05::mbar_arrive(ready + grp);
       }
-      tc05::fence_before();
-      tc05::fence_proxy_async();
-      __syncthreads();
-    }
-    // ---- backward: dW_l (+)= dZ_l^T in_l, dH = dZ_l W_l, dZ_{l-1} = dH * mask
-    for (int l = kLayers - 1; l >= 0 && ok; --l) {
-      if (tid == 0) {
+      // ---- backward: dZ_{l-1} = dH * (h_{l-1} > 0); the step's MMAs have read dZ_l by now
+      for (int l = kLayers - 1; l >= 0; --l) {
+        ok = ok && tc05::mbar_wait(done + grp, phase);
+        phase ^= 1u;
+        if (l == 0) break;
         tc05::fence_after();
-        const uint32_t acc0 = tiles_done > 0 ? 1u : 0u;
-        for (int kk = 0; kk < kTile / 16; ++kk)
-          tc05::mma_f16(tmem + bk_col(l), tc05::smem_desc(dzt_addr + kk * 256u, 128u, 2048u),
-                        tc05::smem_desc(tc05::smem_u32(sm + tin_off(l)) + kk * 256u, 128u, 2048u),
-                        tc05::idesc_f16_f32(128, bk_n(l)), (acc0 || kk > 0) ? 1u : 0u);
-        if (l > 0) {
-          const int KK = layer_n(l);
-          const uint32_t sbo = (uint32_t)(KK / 8) * 128u;
-          for (int kk = 0; kk < KK / 16; ++kk)
-            tc05::mma_f16(tmem, tc05::smem_desc(a_addr + kk * 256u, 128u, sbo),
-                          tc05::smem_desc(wt_addr + wt_off(l) + kk * 256u, 128u, sbo), tc05::idesc_f16_f32(128, 64),
-                          kk > 0 ? 1u : 0u);
-        }
-        tc05::commit(mbar);
-      }
-      const bool got = tc05::mbar_wait(mbar, phase);
-      ok = __syncthreads_and(got) != 0;
-      if (!ok) break;
-      phase ^= 1u;
-      if (l == 0) break;
-      tc05::fence_after();
-      const uint32_t mk = mask[l - 1];
+        uint32_t c[32];
+        tc05::tmem_ld32(acc + (uint32_t)c0, c);
+        tc05::tmem_wait(c);
+        const uint8_t* in = sm + tin_off(grp, l);
 #pragma unroll
-      for (int hf = 0; hf < 2; ++hf) {
-        const int c0 = 32 * grp + 16 * hf;
-        float v[16];
-        tc05::tmem_ld16(tmem + lane_base + (uint32_t)c0, v);
-        __align__(16) __half h[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          h[j] = sat_half((mk >> (16 * hf + j)) & 1u ? v[j] : 0.0f);
-          *reinterpret_cast<__half*>(DzT + tc05::core_off(c0 + j, r, kTile)) = h[j];
+        for (int q = 0; q < 4; ++q) {
+          const uint32_t off = tc05::core_off(r, c0 + 8 * q, kHid);
+          const int4 h = *reinterpret_cast<const int4*>(in + off);
+          const int k = 8 * q;
+          int4 u;
+          u.x = (int)h2_where(h2_grad<LOSS>(__uint_as_float(c[k]), __uint_as_float(c[k + 1])), (uint32_t)h.x);
+          u.y = (int)h2_where(h2_grad<LOSS>(__uint_as_float(c[k + 2]), __uint_as_float(c[k + 3])), (uint32_t)h.y);
+          u.z = (int)h2_where(h2_grad<LOSS>(__uint_as_float(c[k + 4]), __uint_as_float(c[k + 5])), (uint32_t)h.z);
+          u.w = (int)h2_where(h2_grad<LOSS>(__uint_as_float(c[k + 6]), __uint_as_float(c[k + 7])), (uint32_t)h.w);
+          *reinterpret_cast<int4*>(dZ + off) = u;
         }
-        *reinterpret_cast<int4*>(A + tc05::core_off(r, c0, kHid)) = *reinterpret_cast<const int4*>(h);
-        *reinterpret_cast<int4*>(A + tc05::core_off(r, c0 + 8, kHid)) = *reinterpret_cast<const int4*>(h + 8);
+        tc05::fence_before();
+        tc05::fence_proxy_async();
+        tc05::mbar_arrive(ready + grp);
       }
-      tc05::fence_before();
-      tc05::fence_proxy_async();
-      __syncthreads();
     }
-    ++tiles_done;
+    if (!ok) *failed = 1;
   }
-  if (!ok) {
-    if (tid == 0) atomicOr(err, 1);
-    tc05::mbar_wait(mbar, phase);  // the same phase, bounded: let an MMA still in flight finish
-  }
+  tc05::fence_before();
   __syncthreads();
   tc05::fence_after();
+  const bool ok = *failed == 0;
+  if (!ok && tid == 0) atomicOr(err, 1);
   // this CTA's partial: weight gradients from TMEM lanes 0..63 (one output
-  // unit per lane; warps 0, 1, 4, 5), the two column halves' 16-column
-  // chunks alternating
+  // unit per lane), the layers split between the warps that read those lanes
   float* mine = part + (size_t)blockIdx.x * kPartStride;
-  if ((warp & 3) < 2) {
-    const int o = r;
-    for (int l = 0; l < kLayers; ++l) {
-      const int N = bk_n(l), kin = layer_kin(l);
-      for (int c0 = 16 * grp; c0 < N; c0 += 32) {
+  if (grp < 2 && (warp & 3) < 2) {
+    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+    for (int l = 2 * grp + half; l < kLayers; l += 4) {
+      const int kin = layer_kin(l), nout = layer_nout(l);
+      for (int c0 = 0; c0 < (l == 0 ? kInPad : kHid + 16); c0 += 16) {
         float v[16];
-        tc05::tmem_ld16(tmem + lane_base + bk_col(l) + (uint32_t)c0, v);
-        if (o < layer_nout(l)) {
+        tc05::tmem_ld16(tmem + lanes + dw_col(l) + (uint32_t)c0, v);
+        if (r >= nout) continue;
+        if (l > 0 && c0 < kHid) {
+          float4* dst = reinterpret_cast<float4*>(mine + param_w(l) + r * kHid + c0);
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int k = c0 + j;
-            const float g = (ok && tiles_done > 0) ? v[j] : 0.0f;
-            if (k < kin) mine[param_w(l) + o * kin + k] = g;
-            else if (k == kin) mine[param_b(l) + o] = g;
-          }
+          for (int q = 0; q < 4; ++q)
+            dst[q] = ok ? make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3])
+                        : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        } else if (l > 0) {
+          mine[param_b(l) + r] = ok ? v[0] : 0.0f;
+        } else {
+#pragma unroll
+          for (int k = 0; k < kIn; ++k) mine[r * kin + k] = ok ? v[k] : 0.0f;
+          mine[param_b(0) + r] = ok ? v[kIn] : 0.0f;
         }
       }
     }
@@ -775,7 +706,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     l_acc += __shfl_xor_sync(0xffffffffu, l_acc, off);
   }
   float* red = reinterpret_cast<float*>(sm + kTRed);
-  if ((tid & 31) == 0) {
+  if ((tid & 31) == 0 && warp < 16) {
     red[2 * warp] = w_acc;
     red[2 * warp + 1] = l_acc;
   }
@@ -783,57 +714,74 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
   __syncthreads();
   if (tid == 0) {
     float ws = 0.0f, ls = 0.0f;
-    for (int k = 0; k < kTrainThreads / 32; ++k) {
+    for (int k = 0; k < 16; ++k) {
       ws += red[2 * k];
       ls += red[2 * k + 1];
     }
     mine[kParams] = ws;
     mine[kParams + 1] = ls;
   }
-  if (warp == 0) {
-    tc05::tmem_dealloc(tmem, 512);
-  }
+  if (warp == 16) tc05::tmem_dealloc(tmem, 512);
 }
 
-// Sums the nparts partials (32 parameters x 8 partial slices per block),
-// takes the Adam step, and writes the new weight (or bias) into the forward
-// image and, for layers 1..4, the transposed image. loss_out (optional)
-// receives the batch loss.
-__global__ void __launch_bounds__(256)
-    k_update(const float* __restrict__ part, int nparts, const float* __restrict__ scale,
-             float* __restrict__ p, float* __restrict__ m, float* __restrict__ v, float lr, float c1, float c2,
-             uint8_t* __restrict__ img, uint8_t* __restrict__ img_t, float* __restrict__ loss_out) {
-  __shared__ float red[8][33];
-  __shared__ float tot[8][2];
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int i = blockIdx.x * 32 + tx;
-  float g = 0.0f, ws = 0.0f, ls = 0.0f;
-  for (int c = ty; c < nparts; c += 8) {
-    const float* pc = part + (size_t)c * kPartStride;
-    if (i < kParams) g += pc[i];
-    if (tx == 0) {
-      ws += pc[kParams];
-      ls += pc[kParams + 1];
-    }
+// Column i of the partials, summed over this thread's share of them (blocks of
+// 32 columns x kSlices slices, ten loads in flight); the order is fixed.
+constexpr int kSlices = 16;
+__device__ __forceinline__ float part_slice(const float* __restrict__ part, int nparts, int i) {
+  float g = 0.0f;
+  for (int c0 = threadIdx.y; c0 < nparts; c0 += 10 * kSlices) {
+    float v[10];
+#pragma unroll
+    for (int k = 0; k < 10; ++k)
+      v[k] = c0 + k * kSlices < nparts ? part[(size_t)(c0 + k * kSlices) * kPartStride + i] : 0.0f;
+#pragma unroll
+    for (int k = 0; k < 10; ++k) g += v[k];
   }
-  red[ty][tx] = g;
-  if (tx == 0) {
-    tot[ty][0] = ws;
-    tot[ty][1] = ls;
-  }
+  return g;
+}
+
+// The gradient itself: the sum of the partials.
+__global__ void __launch_bounds__(32 * kSlices)
+    k_grad_sum(const float* __restrict__ part, int nparts, float* __restrict__ grads) {
+  __shared__ float red[kSlices][33];
+  const int tx = threadIdx.x, ty = threadIdx.y, i = blockIdx.x * 32 + tx;
+  red[ty][tx] = i < kParams ? part_slice(part, nparts, i) : 0.0f;
   __syncthreads();
   if (ty != 0 || i >= kParams) return;
-  g = 0.0f;
-  ws = 0.0f;
-  ls = 0.0f;
+  float g = 0.0f;
 #pragma unroll
-  for (int y = 0; y < 8; ++y) {
+  for (int y = 0; y < kSlices; ++y) g += red[y][tx];
+  grads[i] = g;
+}
+
+// Sums the nparts partials (32 parameters x kSlices partial slices per block),
+// takes the Adam step, and writes the new weight (or bias) into the packed
+// image. loss_out (optional) receives the batch loss.
+__global__ void __launch_bounds__(32 * kSlices)
+    k_update(const float* __restrict__ part, int nparts, const float* __restrict__ wparts, float wrows,
+             float* __restrict__ p, float* __restrict__ m, float* __restrict__ v, float lr, float c1, float c2,
+             uint8_t* __restrict__ img, float* __restrict__ loss_out) {
+  __shared__ float red[kSlices][33];
+  __shared__ float tot[kSlices][2];
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int i = blockIdx.x * 32 + tx;
+  float g = i < kParams ? part_slice(part, nparts, i) : 0.0f, ws = 0.0f, ls = 0.0f;
+  if (tx < 2) {
+    const float t = part_slice(part, nparts, kParams + tx);
+    tot[ty][tx] = t;
+  }
+  red[ty][tx] = g;
+  const float scale = row_scale(wparts, wrows, 32 * ty + tx);  // (its barriers publish red and tot)
+  if (ty != 0 || i >= kParams) return;
+  g = 0.0f;
+#pragma unroll
+  for (int y = 0; y < kSlices; ++y) {
     g += red[y][tx];
     ws += tot[y][0];
     ls += tot[y][1];
   }
   if (loss_out && i == 0) *loss_out = ls / fmaxf(ws, 1e-30f);
-  const float denom = *scale * ws;
+  const float denom = scale * ws;
   g = denom > 1e-30f ? g / denom : 0.0f;
   const float mi = 0.9f * m[i] + 0.1f * g;
   const float vi = 0.999f * v[i] + 0.001f * g * g;
@@ -847,7 +795,6 @@ __global__ void __launch_bounds__(256)
   if (e < layer_nout(l) * kin) {
     const int o = e / kin, k = e % kin;
     *reinterpret_cast<__half*>(img + w_off(l) + tc05::core_off(o, k, layer_k(l))) = __float2half_rn(pi);
-    if (l > 0) *reinterpret_cast<__half*>(img_t + wt_off(l) + tc05::core_off(k, o, layer_n(l))) = __float2half_rn(pi);
   } else {
     const int o = e - layer_nout(l) * kin;
     reinterpret_cast<float*>(img + kBiasOff)[l < kLayers - 1 ? l * 64 + o : 256 + o] = pi;
@@ -876,7 +823,7 @@ tr_status guide_reserve(tr_ctx* ctx) {
   if (g->params.p) return TR_OK;
   cudaError_t e = cudaSuccess;
   for (auto pr : {std::make_pair(&g->params, (size_t)mlp::kParams * 4), std::make_pair(&g->img, (size_t)mlp::kPackedBytes),
-                  std::make_pair(&g->img_t, (size_t)mlp::kWtBytes), std::make_pair(&g->grads, (size_t)mlp::kParams * 4),
+                  
                   std::make_pair(&g->adam_m, (size_t)mlp::kParams * 4),
                   std::make_pair(&g->adam_v, (size_t)mlp::kParams * 4),
                   std::make_pair(&g->scal, (size_t)(16 + mlp::kWsumParts) * 4)})
@@ -884,10 +831,10 @@ tr_status guide_reserve(tr_ctx* ctx) {
   if (!g->attr_set) {
     if ((e = cudaFuncSetAttribute(mlp::k_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, mlp::kSmemBytes)) !=
             cudaSuccess ||
-        (e = cudaFuncSetAttribute(mlp::k_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, mlp::kBSmemBytes)) !=
-            cudaSuccess ||
-        (e = cudaFuncSetAttribute(mlp::k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, mlp::kTSmemBytes)) !=
-            cudaSuccess)
+        (e = cudaFuncSetAttribute(mlp::k_train<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  mlp::kTSmemBytes)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(mlp::k_train<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  mlp::kTSmemBytes)) != cudaSuccess)
       return cuda_fail(ctx, e, "guide kernels' shared memory");
     g->attr_set = true;
   }
@@ -906,15 +853,13 @@ static tr_status guide_reset_adam(tr_ctx* ctx) {
 tr_status guide_pack(tr_ctx* ctx) {
   GuideModel* g = ctx->guide;
   mlp::k_pack<<<(mlp::kPackThreads + 255) / 256, 256, 0, ctx->stream>>>(g->params.as<float>(), g->img.as<uint8_t>());
-  mlp::k_pack_t<<<(mlp::kPackTThreads + 255) / 256, 256, 0, ctx->stream>>>(g->params.as<float>(),
-                                                                            g->img_t.as<uint8_t>());
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TR_OK : cuda_fail(ctx, e, "guide weight packing");
 }
 
 // Forward: up to four CTAs per SM (50 KB of shared memory and 64 TMEM
 // columns each), so that one CTA's MMAs overlap another's epilogue.
-// Backward: one per SM (each holds 512 TMEM columns, the whole SM's).
+// Training and backward: one per SM (each holds 512 TMEM columns, the whole SM's).
 static int guide_grid(tr_ctx* ctx, int n, int per_sm) {
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
@@ -922,9 +867,9 @@ static int guide_grid(tr_ctx* ctx, int n, int per_sm) {
   return std::max(1, std::min(tiles, sms * per_sm));
 }
 
-tr_status guide_forward(tr_ctx* ctx, const float* d_in, int n, float* d_out, __half* d_acts) {
+tr_status guide_forward(tr_ctx* ctx, const float* d_in, int n, float* d_out) {
   mlp::k_forward<<<guide_grid(ctx, n, 4), 128, mlp::kSmemBytes, ctx->stream>>>(
-      ctx->guide->img.as<uint8_t>(), d_in, n, d_out, d_acts, ctx->d_err.as<int>() + 2, nullptr, 0);
+      ctx->guide->img.as<uint8_t>(), d_in, n, d_out, ctx->d_err.as<int>() + 2, nullptr, 0);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TR_OK : cuda_fail(ctx, e, "k_forward");
 }
@@ -933,7 +878,7 @@ tr_status guide_forward_rows_on_device(tr_ctx* ctx, const float* d_in, const uns
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   mlp::k_forward<<<std::max(sms, 1) * 4, 128, mlp::kSmemBytes, ctx->stream>>>(
-      ctx->guide->img.as<uint8_t>(), d_in, 0, d_out, nullptr, ctx->d_err.as<int>() + 2, d_n, 1);
+      ctx->guide->img.as<uint8_t>(), d_in, 0, d_out, ctx->d_err.as<int>() + 2, d_n, 1);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TR_OK : cuda_fail(ctx, e, "k_forward");
 }
@@ -942,7 +887,6 @@ tr_status guide_forward_rows_on_device(tr_ctx* ctx, const float* d_in, const uns
 static tr_status guide_scale(tr_ctx* ctx, const float* w, unsigned int n) {
   float* scal = ctx->guide->scal.as<float>();
   mlp::k_wsum<<<mlp::kWsumParts, 256, 0, ctx->stream>>>(w, n, scal + 16);
-  mlp::k_scale<<<1, mlp::kWsumParts, 0, ctx->stream>>>(scal + 16, (float)n, scal + 2);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TR_OK : cuda_fail(ctx, e, "guide weight sum");
 }
@@ -956,15 +900,15 @@ static tr_status guide_fused_step(tr_ctx* ctx, const float* in, const float* dir
   cudaError_t e;
   if ((e = g->part.reserve((size_t)grid * mlp::kPartStride * 4)) != cudaSuccess)
     return cuda_fail(ctx, e, "guide gradient partials");
-  const float* scale = g->scal.as<float>() + 2;
-  mlp::k_train<<<grid, mlp::kTrainThreads, mlp::kTSmemBytes, ctx->stream>>>(g->img.as<uint8_t>(), g->img_t.as<uint8_t>(), in, dir, w,
-                                                              count, n, seed, gather, scale, g->part.as<float>(),
-                                                              ctx->d_err.as<int>() + 2);
+  const float* wparts = g->scal.as<float>() + 16;  // guide_scale's sums over the `count` records
+  mlp::k_train<true><<<grid, mlp::kTrainThreads, mlp::kTSmemBytes, ctx->stream>>>(
+      g->img.as<uint8_t>(), in, dir, w, count, n, seed, gather, wparts, (float)count, g->part.as<float>(),
+      ctx->d_err.as<int>() + 2);
   ++g->step;
   const float c1 = 1.0f - std::pow(0.9f, (float)g->step), c2 = 1.0f - std::pow(0.999f, (float)g->step);
-  mlp::k_update<<<(mlp::kParams + 31) / 32, dim3(32, 8), 0, ctx->stream>>>(
-      g->part.as<float>(), grid, scale, g->params.as<float>(), g->adam_m.as<float>(), g->adam_v.as<float>(), lr, c1,
-      c2, g->img.as<uint8_t>(), g->img_t.as<uint8_t>(), d_loss);
+  mlp::k_update<<<(mlp::kParams + 31) / 32, dim3(32, mlp::kSlices), 0, ctx->stream>>>(
+      g->part.as<float>(), grid, wparts, (float)count, g->params.as<float>(), g->adam_m.as<float>(), g->adam_v.as<float>(), lr, c1,
+      c2, g->img.as<uint8_t>(), d_loss);
   e = cudaGetLastError();
   return e == cudaSuccess ? TR_OK : cuda_fail(ctx, e, "guide training step");
 }
@@ -995,24 +939,23 @@ tr_status guide_train_on(tr_ctx* ctx, const float* rec_in, const float* rec_dir,
 static tr_status guide_workspace(tr_ctx* ctx, int n) {
   GuideModel* g = ctx->guide;
   cudaError_t e;
-  if ((e = g->acts.reserve((size_t)4 * n * mlp::kHid * 2)) != cudaSuccess ||
-      (e = g->out.reserve((size_t)n * mlp::kOut * 4)) != cudaSuccess ||
+  if ((e = g->out.reserve((size_t)n * mlp::kOut * 4)) != cudaSuccess ||
       (e = g->dout.reserve((size_t)n * mlp::kOut * 4)) != cudaSuccess)
     return cuda_fail(ctx, e, "guide training workspace");
   return TR_OK;
 }
 
 tr_status guide_backward(tr_ctx* ctx, const float* d_in, const float* d_dout, int n, float* d_grads) {
-  tr_status s = guide_workspace(ctx, n);
-  if (s != TR_OK) return s;
   GuideModel* g = ctx->guide;
-  s = guide_forward(ctx, d_in, n, g->out.as<float>(), g->acts.as<__half>());
-  if (s != TR_OK) return s;
-  TR_CUDA(ctx, cudaMemsetAsync(d_grads, 0, mlp::kParams * 4, ctx->stream));
-  mlp::k_backward<<<guide_grid(ctx, n, 1), 128, mlp::kBSmemBytes, ctx->stream>>>(
-      g->img_t.as<uint8_t>(), d_in, g->acts.as<__half>(), d_dout, n, d_grads, ctx->d_err.as<int>() + 2);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? TR_OK : cuda_fail(ctx, e, "k_backward");
+  const int grid = guide_grid(ctx, n, 1);
+  cudaError_t e = g->part.reserve((size_t)grid * mlp::kPartStride * 4);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "guide gradient partials");
+  mlp::k_train<false><<<grid, mlp::kTrainThreads, mlp::kTSmemBytes, ctx->stream>>>(
+      g->img.as<uint8_t>(), d_in, d_dout, nullptr, 0u, n, 0ull, 0, nullptr, 0.0f, g->part.as<float>(),
+      ctx->d_err.as<int>() + 2);
+  mlp::k_grad_sum<<<(mlp::kParams + 31) / 32, dim3(32, mlp::kSlices), 0, ctx->stream>>>(g->part.as<float>(), grid, d_grads);
+  e = cudaGetLastError();
+  return e == cudaSuccess ? TR_OK : cuda_fail(ctx, e, "guide backward pass");
 }
 
 // Loss and its gradient w.r.t. the network outputs (g->dout) for a batch;
@@ -1021,7 +964,7 @@ static tr_status guide_loss(tr_ctx* ctx, const float* d_in, const float* d_dir, 
   tr_status s = guide_workspace(ctx, n);
   if (s != TR_OK) return s;
   GuideModel* g = ctx->guide;
-  s = guide_forward(ctx, d_in, n, g->out.as<float>(), g->acts.as<__half>());
+  s = guide_forward(ctx, d_in, n, g->out.as<float>());
   if (s != TR_OK) return s;
   float* scal = g->scal.as<float>();
   TR_CUDA(ctx, cudaMemsetAsync(scal, 0, 8, ctx->stream));
@@ -1053,7 +996,7 @@ static tr_status guide_check(tr_ctx* ctx) {
 void release_guide(tr_ctx* ctx) {
   if (!ctx->guide) return;
   GuideModel* g = ctx->guide;
-  for (DevBuf* b : {&g->params, &g->img, &g->img_t, &g->grads, &g->adam_m, &g->adam_v, &g->acts, &g->out, &g->dout,
+  for (DevBuf* b : {&g->params, &g->img, &g->adam_m, &g->adam_v, &g->out, &g->dout,
                     &g->scal, &g->part, &g->losses})
     b->release();
   delete g;
@@ -1114,7 +1057,7 @@ tr_status tr_guide_forward_dev(tr_ctx* ctx, const float* d_in, size_t n, float* 
   if (n > (1u << 30)) return set_err(ctx, TR_ERR_ARG, "too many rows");
   if (n == 0) return TR_OK;
   TR_DEVICE_SCOPE(ctx);
-  tr_status s = guide_forward(ctx, d_in, (int)n, d_out, nullptr);
+  tr_status s = guide_forward(ctx, d_in, (int)n, d_out);
   return s != TR_OK ? s : guide_check(ctx);
 }
 
