@@ -234,21 +234,18 @@ __device__ __forceinline__ float vmf_log_norm(float kappa) {
 
 // log p(omega | z) of one row, and the gradient of -wi log p w.r.t. the row's
 // network outputs z. The lobes may be split over several threads: this thread
-// has LOBES of them (z, d: their 5 * LOBES outputs), and `all` combines a
-// partial maximum (max) or sum over the row's threads.
-template <int LOBES, class All>
-__device__ __forceinline__ float row_nll_grad(const float* z, float3 om, float wi, float* d, All all) {
+// has LOBES of them (z, d: their 5 * LOBES outputs), and `row` gives a maximum
+// (row.max) or the sum in lobe order (row.sum) over the row's threads.
+template <int LOBES, class Row>
+__device__ __forceinline__ float row_nll_grad(const float* z, float3 om, float wi, float* d, Row row) {
   float a_max = -INFINITY;
 #pragma unroll
   for (int j = 0; j < LOBES; ++j) a_max = fmaxf(a_max, z[5 * j]);
-  a_max = all(a_max, true);
-  float esum = 0.0f, lq[LOBES], pi[LOBES];
+  a_max = row.max(a_max);
+  float lq[LOBES], pi[LOBES];
 #pragma unroll
-  for (int j = 0; j < LOBES; ++j) {
-    pi[j] = expf(z[5 * j] - a_max);
-    esum += pi[j];
-  }
-  esum = all(esum, false);
+  for (int j = 0; j < LOBES; ++j) pi[j] = expf(z[5 * j] - a_max);
+  const float esum = row.sum(pi);
   float lmax = -INFINITY;
   Lobe L[LOBES];
 #pragma unroll
@@ -264,11 +261,11 @@ __device__ __forceinline__ float row_nll_grad(const float* z, float3 om, float w
     lq[j] = logf(fmaxf(pi[j], 1e-30f)) + vmf_log_norm(kappa) + kappa * (c - 1.0f);
     lmax = fmaxf(lmax, lq[j]);
   }
-  lmax = all(lmax, true);
-  float qs = 0.0f;
+  lmax = row.max(lmax);
+  float qe[LOBES];
 #pragma unroll
-  for (int j = 0; j < LOBES; ++j) qs += expf(lq[j] - lmax);
-  const float logp = lmax + logf(all(qs, false));
+  for (int j = 0; j < LOBES; ++j) qe[j] = expf(lq[j] - lmax);
+  const float logp = lmax + logf(row.sum(qe));
 #pragma unroll
   for (int j = 0; j < LOBES; ++j) {
     const float q = expf(lq[j] - logp);  // responsibility
@@ -286,6 +283,17 @@ __device__ __forceinline__ float row_nll_grad(const float* z, float3 om, float w
   return logp;
 }
 
+// A row whose eight lobes are all this thread's.
+struct WholeRow {
+  __device__ __forceinline__ float max(float v) const { return v; }
+  __device__ __forceinline__ float sum(const float (&v)[kLobes]) const {
+    float s = 0.0f;
+#pragma unroll
+    for (int j = 0; j < kLobes; ++j) s += v[j];
+    return s;
+  }
+};
+
 __global__ void k_loss(const float* __restrict__ out, const float* __restrict__ dir, const float* __restrict__ w,
                        int n, const float* __restrict__ wsum, float* __restrict__ dout, float* __restrict__ loss) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -294,7 +302,7 @@ __global__ void k_loss(const float* __restrict__ out, const float* __restrict__ 
     const float3 om = make_float3(dir[3 * i], dir[3 * i + 1], dir[3 * i + 2]);
     const float wi = w[i] / fmaxf(*wsum, 1e-30f);
     li = -wi * row_nll_grad<kLobes>(out + (size_t)i * kOut, om, wi, dout + (size_t)i * kOut,
-                                    [](float v, bool) { return v; });
+                                    WholeRow());
   }
   // block sum of the loss
   for (int o = 16; o > 0; o >>= 1) li += __shfl_xor_sync(0xffffffffu, li, o);
@@ -424,6 +432,37 @@ __device__ __forceinline__ uint32_t h2_where(uint32_t u, uint32_t h) {
 __device__ __forceinline__ void group_sync(int g) {
   asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(256) : "memory");
 }
+
+// A row whose lobes are split between two threads of a k_train group: the
+// second half's sum goes on from the first half's, in lobe order.
+struct HalfRow {
+  float* x;  // two values per row of the group
+  int g, half, r;
+  __device__ __forceinline__ float max(float v) const {
+    group_sync(g);
+    x[kTile * half + r] = v;
+    group_sync(g);
+    return fmaxf(x[r], x[kTile + r]);
+  }
+  __device__ __forceinline__ float sum(const float (&v)[kLobes / 2]) const {
+    float s = 0.0f;
+    if (half == 0) {
+#pragma unroll
+      for (int j = 0; j < kLobes / 2; ++j) s += v[j];
+    }
+    group_sync(g);
+    if (half == 0) x[r] = s;
+    group_sync(g);
+    if (half == 1) {
+      s = x[r];
+#pragma unroll
+      for (int j = 0; j < kLobes / 2; ++j) s += v[j];
+      x[kTile + r] = s;
+    }
+    group_sync(g);
+    return x[kTile + r];
+  }
+};
 
 // The MMAs of one step of a tile: forward layer L, and backward layer L.
 template <int L>
@@ -568,6 +607,12 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
 #pragma unroll
         for (int k = 0; k < 3; ++k) om[k] = rdir[(size_t)j * 3 + k];
         w = rw[j];
+        // the weight sum, tile by tile in order: group 0 adds both groups' rows
+        if (grp == 0 && half == 0) {
+          w_acc += w;
+          const long long i2 = (long long)i + (long long)gridDim.x * kTile;
+          if (i2 < n) w_acc += rw[gather ? batch_record(seed, (unsigned int)i2, count) : (unsigned int)i2];
+        }
       }
       {  // in_0: the inputs, a one for the bias gradient (its weights are zero), zeros; eight columns a thread
         __align__(16) __half h[8];
@@ -610,18 +655,9 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
 #pragma unroll
           for (int k = 0; k < kMine; ++k) z[k] = __uint_as_float(c[k]) + bias[256 + kMine * half + k];
           float* xch = reinterpret_cast<float*>(sm + kTXch) + 2 * kTile * grp;
-          const float logp = row_nll_grad<kLobes / 2>(
-              z, make_float3(om[0], om[1], om[2]), w * s, d, [&](float v, bool max) {
-                group_sync(grp);
-                xch[kTile * half + r] = v;
-                group_sync(grp);
-                const float a = xch[r], b = xch[kTile + r];
-                return max ? fmaxf(a, b) : a + b;
-              });
-          if (live && half == 0) {
-            w_acc += w;
-            l_acc -= w * logp;
-          }
+          const float logp = row_nll_grad<kLobes / 2>(z, make_float3(om[0], om[1], om[2]), w * s, d,
+                                                      HalfRow{xch, grp, half, r});
+          if (live && half == 0) l_acc -= w * logp;
         } else if (live) {
 #pragma unroll
           for (int k = 0; k < kMine; ++k) d[k] = rdir[(size_t)i * kOut + kMine * half + k];
@@ -726,7 +762,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
 
 // Column i of the partials, summed over this thread's share of them (blocks of
 // 32 columns x kSlices slices, ten loads in flight); the order is fixed.
-constexpr int kSlices = 16;
+constexpr int kSlices = 8;
 __device__ __forceinline__ float part_slice(const float* __restrict__ part, int nparts, int i) {
   float g = 0.0f;
   for (int c0 = threadIdx.y; c0 < nparts; c0 += 10 * kSlices) {
