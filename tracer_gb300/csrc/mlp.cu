@@ -910,10 +910,11 @@ tr_status guide_forward(tr_ctx* ctx, const float* d_in, int n, float* d_out) {
   return e == cudaSuccess ? TR_OK : cuda_fail(ctx, e, "k_forward");
 }
 
-tr_status guide_forward_rows_on_device(tr_ctx* ctx, const float* d_in, const unsigned int* d_n, float* d_out) {
+tr_status guide_forward_rows_on_device(tr_ctx* ctx, const float* d_in, const unsigned int* d_n, float* d_out,
+                                       cudaStream_t st) {
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-  mlp::k_forward<<<std::max(sms, 1) * 4, 128, mlp::kSmemBytes, ctx->stream>>>(
+  mlp::k_forward<<<std::max(sms, 1) * 4, 128, mlp::kSmemBytes, st>>>(
       ctx->guide->img.as<uint8_t>(), d_in, 0, d_out, ctx->d_err.as<int>() + 2, d_n, 1);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TR_OK : cuda_fail(ctx, e, "k_forward");

@@ -62,20 +62,30 @@ __host__ __device__ constexpr int nee_index(int kind) {
   return kind == MAT_METAL ? 2 : (kind == MAT_DISNEY15 ? 3 : kind);
 }
 
-enum : int {  // counter slots
-  C_EXT = 0,      // 2: extend queue sizes (double-buffered)
-  C_ACT = 2,      // 2: live-slot list sizes
-  C_SH = 4,       // shadow queue size
-  C_MAT = 5,      // 5: per-material hit queue sizes (Phong, Disney12, glass, metal, Disney15)
-  C_NEE = 10,     // 4: light-sample queue sizes (Phong, Disney12, metal, Disney15; glass has none)
-  C_FEXT = 14,    // extend kernel's work-fetch position
-  C_FSH = 15,     // shadow kernel's work-fetch position
-  C_TB = 16,      // guiding training records written (whole render)
-  C_ERR = 17,     // traversal error word
-  C_ORD = 18,     // live slots written in slot order (this iteration)
-  C_GROW = 19,    // network rows of this iteration's guided vertices
+// Counter words. The queues between iterations are double-buffered (iteration
+// i reads words + (i & 1) and fills the other), and so are the queues inside
+// an iteration (bank(i & 1)), so that each set can be zeroed by a kernel of
+// the iteration before instead of by launches of its own (k_logic,
+// k_act_order), while that iteration's other branches still run.
+enum : int {
+  C_EXT = 0,      // 2: extend queue sizes
+  C_ACT = 2,      // 2: live slots
+  C_FEXT = 4,     // 2: extend kernel's work-fetch position
+  C_ORD = 6,      // live slots written in slot order
+  C_TB = 7,       // guiding training records written (whole render)
+  C_ERR = 8,      // traversal error word
+  C_BANK = 16,    // 2 x kBankWords
 };
-constexpr int kCtrWords = 32;  // the counter array
+enum : int {  // of a bank
+  B_SH = 0,       // shadow queue size
+  B_FSH = 1,      // shadow kernel's work-fetch position
+  B_MAT = 2,      // 5: per-material hit queue sizes (Phong, Disney12, glass, metal, Disney15)
+  B_NEE = 7,      // 4: light-sample queue sizes (Phong, Disney12, metal, Disney15; glass has none)
+  B_GROW = 11,    // network rows of this iteration's guided vertices
+};
+constexpr int kBankWords = 16;
+__host__ __device__ constexpr int bank(int cur) { return C_BANK + kBankWords * cur; }
+constexpr int kCtrWords = C_BANK + 2 * kBankWords;  // the counter array
 // Statistics words: samples, extend rays, shadow rays, shade items, visit
 // counts (4-7), occluder-cache hits (8).
 constexpr int kStatWords = 16;
@@ -87,7 +97,7 @@ constexpr int kMatScratch = 1 << 30;
 
 struct RenderBuffers {
   int n = 0, nl = 0;
-  DevBuf P0, P1, P2, P3, P4, rng, M0, M1, M2, HC, HM, SC, NU, SH, SHC, acc, q_ext, q_act, q_mat, q_nee, q_sh, ctr,
+  DevBuf P0, P1, P2, P3, P4, rng, M0, M1, M2, HC, HM, SC, NU, SH, SHC, acc, q_ext, q_mat, q_nee, q_sh, ctr,
       stats;
   DevBuf VR, NV, gfeat, gout, tb;  // path guiding: vertex records, network rows, training records
   DevBuf GX;                        // path guiding: the continuation's MIS data (4 float4 per slot)
@@ -97,6 +107,8 @@ struct RenderBuffers {
   DevBuf q_srt, bin_key, bin_cnt;   // ray binning: the reordered queue, keys, bin counts
   DevBuf OC;                        // occluder cache, one int per (slot, light)
   DevBuf q_ord, act_flag;           // the live-slot list in slot order, per-slot marks
+  cudaStream_t side[5] = {};        // branches of an iteration's graph
+  cudaEvent_t fork_ev[12] = {};
   unsigned int tb_count = 0, tb_cap = 0;  // training records of the last guided render
   unsigned int* h_active = nullptr;  // pinned: live-slot count per check
   DevBuf mega_state;                 // persistent kernel: counters, then statistics
@@ -123,7 +135,6 @@ struct Launch {
   float4* SHC;           // per (slot, light): the light sample's contribution|valid (0: none or occluded)
   DMat* MT;              // per slot: the Phong set-up at a hit with image maps (null without maps)
   int* q_ext[2];
-  int* q_act[2];
   int* q_mat[kMatKinds];
   int* q_nee[kNeeKinds];
   int* q_sh;
@@ -135,7 +146,7 @@ struct Launch {
   // occluder cache (null: off): per (slot, light) item, the slot that last
   // blocked its shadow ray, or -1
   int* OC;
-  // the live-slot list in slot order (null: k_logic reads the list as appended)
+  // the live-slot list in slot order, made from per-slot marks (k_act_order)
   int* q_ord;
   int mis_all;  // trace every MIS ray (visit-counting renders match the oracle's queries)
   // guided renders: vertices at path depth < guide_depth (0: all) are
@@ -407,8 +418,8 @@ __global__ void __launch_bounds__(256) k_init(Launch P) {
     reserve<2, 8, 0u>(sh, ctr, want, pos);
     if (live) {
       P.q_ext[0][pos[0]] = 2 * s;
-      P.q_act[0][pos[1]] = s;
     }
+    if (s < n) P.act_flag[s] = live ? 1 : 0;
   }
   block_count<8>(P.stats, finished);
 }
@@ -443,9 +454,10 @@ struct ExtendJob {
 // Work items of the shadow kernel: shadow records o|t_max, d, contrib|valid.
 struct ShadowJob {
   const Launch& P;
+  int cur;
   const int* q;  // the queue (shadow rays keep queue order: a vertex's rays to every light are adjacent)
-  __device__ explicit ShadowJob(const Launch& P_) : P(P_), q(P_.q_sh) {}
-  __device__ __forceinline__ unsigned int count() const { return P.ctr[C_SH]; }
+  __device__ ShadowJob(const Launch& P_, int cur_) : P(P_), cur(cur_), q(P_.q_sh) {}
+  __device__ __forceinline__ unsigned int count() const { return P.ctr[bank(cur) + B_SH]; }
   // the slot that last blocked this (pixel slot, light) item's shadow ray
   __device__ __forceinline__ int cached(unsigned int i) const { return P.OC ? P.OC[q[i]] : -1; }
   __device__ __forceinline__ void load(unsigned int i, f3& o, f3& d, float& t_min, float& t_max, int& scene) const {
@@ -490,7 +502,7 @@ __global__ void __launch_bounds__(128) k_extend(Launch P, int cur) {
   ExtendJob job(P, cur);
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(P.stats + 1, (unsigned long long)job.count());
   VisitCount vc;
-  persistent_traverse<false, COUNT>(P.sc, job, P.ctr + C_FEXT, (int*)(P.ctr + C_ERR), vc, P.refill, P.tl_n);
+  persistent_traverse<false, COUNT>(P.sc, job, P.ctr + C_FEXT + cur, (int*)(P.ctr + C_ERR), vc, P.refill, P.tl_n);
   if (COUNT) {
     count_add(P.stats + 4, vc.boxes);
     count_add(P.stats + 5, vc.prims);
@@ -498,11 +510,11 @@ __global__ void __launch_bounds__(128) k_extend(Launch P, int cur) {
 }
 
 template <bool COUNT, bool WIDE = false>
-__global__ void __launch_bounds__(128) k_shadow(Launch P) {
-  ShadowJob job(P);
+__global__ void __launch_bounds__(128) k_shadow(Launch P, int cur) {
+  ShadowJob job(P, cur);
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(P.stats + 2, (unsigned long long)job.count());
   VisitCount vc;
-  persistent_traverse<true, COUNT, WIDE>(P.sc, job, P.ctr + C_FSH, (int*)(P.ctr + C_ERR), vc, P.refill, P.tl_n);
+  persistent_traverse<true, COUNT, WIDE>(P.sc, job, P.ctr + bank(cur) + B_FSH, (int*)(P.ctr + C_ERR), vc, P.refill, P.tl_n);
   if (P.OC) count_add(P.stats + 8, vc.cache_hits);
   if (COUNT) {
     count_add(P.stats + 6, vc.boxes);
@@ -631,19 +643,14 @@ __device__ __forceinline__ f3 continuation_emission(const Launch& P, int slot, f
   return pr.emission;
 }
 
-// Marks the slots of the live-slot list, which is in append order.
-__global__ void __launch_bounds__(256) k_act_mark(Launch P, int cur) {
-  const unsigned int n = P.ctr[C_ACT + cur];
-  for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    P.act_flag[P.q_act[cur][i]] = 1;
-}
-
-// The marked slots in slot order within each 256-slot range (the ranges in
+// The slots marked live for iteration `cur` (k_init and the shading kernels
+// mark act_flag), in slot order within each 256-slot range (the ranges in
 // the order their blocks reach the counter), marks cleared. k_logic then
 // reads the path state of consecutive slots together, and the queues it
 // fills, so the kernels after it, follow slot order too; the order of work
-// changes no result.
-__global__ void __launch_bounds__(256) k_act_order(Launch P) {
+// changes no result. Also zeroes the count that k_logic's iteration fills.
+__global__ void __launch_bounds__(256) k_act_order(Launch P, int cur) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) P.ctr[C_ACT + (cur ^ 1)] = 0;
   __shared__ unsigned int wsum[8];
   __shared__ unsigned int base;
   const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5);
@@ -677,7 +684,19 @@ __global__ void __launch_bounds__(128) k_logic(Launch P, int cur) {
   __shared__ QueueSlots<kMatKinds + 3, 4> sh;
   const int nxt = cur ^ 1;
   const unsigned int n = P.ctr[C_ACT + cur];
-  if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(P.stats + 3, (unsigned long long)n);
+  if (blockIdx.x == 0) {
+    if (threadIdx.x == 0) {
+      atomicAdd(P.stats + 3, (unsigned long long)n);
+      // counters whose last readers ran before this kernel: the next
+      // iteration's bank, the extend queue this iteration has traced
+      P.ctr[C_ORD] = 0;
+      P.ctr[C_EXT + cur] = 0;
+      P.ctr[C_FEXT + cur] = 0;
+    }
+    if (threadIdx.x < kBankWords) P.ctr[bank(nxt) + threadIdx.x] = 0;
+  }
+  if (P.bin_bits)  // and the ray bins
+    for (int i = blockIdx.x * 128 + threadIdx.x; i < 1 << (3 + 3 * P.bin_bits); i += gridDim.x * 128) P.bin_cnt[i] = 0;
   unsigned int finished = 0;
   for (unsigned int b = blockIdx.x * 128u; b < n; b += gridDim.x * 128u) {
     const unsigned int i = b + threadIdx.x;
@@ -685,7 +704,7 @@ __global__ void __launch_bounds__(128) k_logic(Launch P, int cur) {
     bool fresh = false;        // the slot starts another sample
     bool row = false;          // guided: the vertex takes a network row
     if (i < n) {
-      slot = P.q_ord ? P.q_ord[i] : P.q_act[cur][i];
+      slot = P.q_ord[i];
       const float4 p0 = P.P0[slot], p3 = P.P3[slot], hit = P.HC[slot], p1 = P.P1[slot];
       const int flags = __float_as_int(p0.w);
       f3 L = mk3(p3.x, p3.y, p3.z);
@@ -768,13 +787,13 @@ __global__ void __launch_bounds__(128) k_logic(Launch P, int cur) {
     unsigned int want[kMatKinds + 3], pos[kMatKinds + 3];
 #pragma unroll
     for (int k = 0; k < kMatKinds; ++k) {
-      ctr[k] = P.ctr + C_MAT + k;
+      ctr[k] = P.ctr + bank(cur) + B_MAT + k;
       want[k] = kind == k ? 1u : 0u;
     }
     ctr[kMatKinds] = P.ctr + C_EXT + nxt;
     ctr[kMatKinds + 1] = P.ctr + C_ACT + nxt;
     want[kMatKinds] = want[kMatKinds + 1] = fresh ? 1u : 0u;
-    ctr[kMatKinds + 2] = P.ctr + C_GROW;
+    ctr[kMatKinds + 2] = P.ctr + bank(cur) + B_GROW;
     want[kMatKinds + 2] = row ? 1u : 0u;
     reserve<kMatKinds + 3, 4, 0u>(sh, ctr, want, pos);
 #pragma unroll
@@ -782,7 +801,7 @@ __global__ void __launch_bounds__(128) k_logic(Launch P, int cur) {
       if (kind == k) P.q_mat[k][pos[k]] = slot;
     if (fresh) {
       P.q_ext[nxt][pos[kMatKinds]] = 2 * slot;
-      P.q_act[nxt][pos[kMatKinds + 1]] = slot;
+      P.act_flag[slot] = 1;
     }
     if (GUIDED && kind == MAT_PHONG && P.guide_alpha > 0.0f) {
       // network inputs of the vertex, a row of this iteration's forward pass
@@ -918,7 +937,8 @@ struct VertexAdds {
 // from the BSDF sample to the next continuation ray
 // (src/renderer/path_trace_renderer.cpp:125-163).
 template <int KIND, bool GUIDED>
-__device__ __forceinline__ void shade_vertex(const Launch& P, int slot, unsigned int& finished, VertexAdds& add) {
+__device__ __forceinline__ void shade_vertex(const Launch& P, int cur, int slot, unsigned int& finished,
+                                             VertexAdds& add) {
   unsigned long long st = P.rng[slot];
   const float4 p0 = P.P0[slot], p1 = P.P1[slot], p2 = P.P2[slot];
   const f3 ro = mk3(p0.x, p0.y, p0.z), rd = mk3(p1.x, p1.y, p1.z);
@@ -996,7 +1016,7 @@ __device__ __forceinline__ void shade_vertex(const Launch& P, int slot, unsigned
     Pcg::skip<3>(st);
     P.NU[item] = make_float2(lu, lv);
     if (l < 64) add.lights |= 1ull << l;
-    else P.q_nee[nee_index(KIND)][append(P.ctr + C_NEE + nee_index(KIND))] = item;
+    else P.q_nee[nee_index(KIND)][append(P.ctr + bank(cur) + B_NEE + nee_index(KIND))] = item;
   }
   float4* sc = P.SC + 7 * (size_t)slot;
   sc[0] = make_float4(is.pos.x, is.pos.y, is.pos.z, __int_as_float(mat));
@@ -1130,21 +1150,21 @@ template <int KIND, bool GUIDED = false>
 __global__ void __launch_bounds__(128, KIND == MAT_DISNEY12 ? 8 : 5) k_material(Launch P, int cur) {
   __shared__ QueueSlots<3, 4> sh;
   const int nxt = cur ^ 1;
-  const unsigned int n = P.ctr[C_MAT + KIND];
+  const unsigned int n = P.ctr[bank(cur) + B_MAT + KIND];
   unsigned int finished = 0;
   for (unsigned int b = blockIdx.x * 128u; b < n; b += gridDim.x * 128u) {
     const unsigned int i = b + threadIdx.x;
     const int slot = i < n ? P.q_mat[KIND][i] : -1;
     VertexAdds add;
-    if (i < n) shade_vertex<KIND, GUIDED>(P, slot, finished, add);
-    unsigned int* const ctr[3] = {P.ctr + C_EXT + nxt, P.ctr + C_ACT + nxt, P.ctr + C_NEE + nee_index(KIND)};
+    if (i < n) shade_vertex<KIND, GUIDED>(P, cur, slot, finished, add);
+    unsigned int* const ctr[3] = {P.ctr + C_EXT + nxt, P.ctr + C_ACT + nxt, P.ctr + bank(cur) + B_NEE + nee_index(KIND)};
     const unsigned int want[3] = {(add.ext_mis ? 1u : 0u) + (add.ext_cont ? 1u : 0u), add.act ? 1u : 0u,
                                   (unsigned int)__popcll(add.lights)};
     unsigned int pos[3];
     reserve<3, 4, 5u>(sh, ctr, want, pos);
     if (add.ext_mis) P.q_ext[nxt][pos[0]++] = 2 * slot + 1;
     if (add.ext_cont) P.q_ext[nxt][pos[0]] = 2 * slot;
-    if (add.act) P.q_act[nxt][pos[1]] = slot;
+    if (add.act) P.act_flag[slot] = 1;
     // a vertex's lights next to each other: k_nee's neighbouring lanes read
     // one shading context, and k_shadow's walk from one origin
     for (unsigned long long m = add.lights; m; m &= m - 1)
@@ -1218,7 +1238,7 @@ __device__ __forceinline__ bool glass_vertex(const Launch& P, int slot, unsigned
 __global__ void __launch_bounds__(128) k_glass(Launch P, int cur) {
   __shared__ QueueSlots<2, 4> sh;
   const int nxt = cur ^ 1;
-  const unsigned int n = P.ctr[C_MAT + MAT_GLASS];
+  const unsigned int n = P.ctr[bank(cur) + B_MAT + MAT_GLASS];
   unsigned int finished = 0;
   for (unsigned int b = blockIdx.x * 128u; b < n; b += gridDim.x * 128u) {
     const unsigned int i = b + threadIdx.x;
@@ -1230,7 +1250,7 @@ __global__ void __launch_bounds__(128) k_glass(Launch P, int cur) {
     reserve<2, 4, 0u>(sh, ctr, want, pos);
     if (more) {
       P.q_ext[nxt][pos[0]] = 2 * slot;
-      P.q_act[nxt][pos[1]] = slot;
+      P.act_flag[slot] = 1;
     }
   }
   block_count<4>(P.stats, finished);
@@ -1371,15 +1391,15 @@ __device__ __forceinline__ bool nee_item(const Launch& P, int item) {
 // registers, a few bytes of spill) measured faster than the five its free
 // allocation (91 registers) allows.
 template <int KIND, bool MAPS = false>
-__global__ void __launch_bounds__(128, 6) k_nee(Launch P) {
+__global__ void __launch_bounds__(128, 6) k_nee(Launch P, int cur) {
   __shared__ QueueSlots<1, 4> sh;
-  const unsigned int n = P.ctr[C_NEE + nee_index(KIND)];
+  const unsigned int n = P.ctr[bank(cur) + B_NEE + nee_index(KIND)];
   for (unsigned int b = blockIdx.x * 128u; b < n; b += gridDim.x * 128u) {
     const unsigned int i = b + threadIdx.x;
     const int item = i < n ? P.q_nee[nee_index(KIND)][i] : -1;
     const bool ok = i < n && nee_item<KIND, MAPS>(P, item);
     if (i < n && !ok) P.SHC[item] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    unsigned int* const ctr[1] = {P.ctr + C_SH};
+    unsigned int* const ctr[1] = {P.ctr + bank(cur) + B_SH};
     const unsigned int want[1] = {ok ? 1u : 0u};
     unsigned int pos[1];
     reserve<1, 4, 0u>(sh, ctr, want, pos);
@@ -1391,7 +1411,7 @@ void release_render(tr_ctx* ctx) {
   if (!ctx->rb) return;
   RenderBuffers* rb = ctx->rb;
   for (DevBuf* b : {&rb->P0, &rb->P1, &rb->P2, &rb->P3, &rb->P4, &rb->rng, &rb->M0, &rb->M1, &rb->M2, &rb->HC,
-                    &rb->HM, &rb->SC, &rb->NU, &rb->SH, &rb->SHC, &rb->acc, &rb->q_ext, &rb->q_act, &rb->q_mat, &rb->q_nee,
+                    &rb->HM, &rb->SC, &rb->NU, &rb->SH, &rb->SHC, &rb->acc, &rb->q_ext, &rb->q_mat, &rb->q_nee,
                     &rb->q_sh, &rb->ctr, &rb->stats, &rb->VR, &rb->NV, &rb->gfeat, &rb->gout, &rb->tb, &rb->jobs,
                     &rb->GX, &rb->grow, &rb->MT, &rb->q_srt, &rb->bin_key, &rb->bin_cnt, &rb->OC, &rb->q_ord,
                     &rb->act_flag, &rb->mega_state})
@@ -1400,6 +1420,10 @@ void release_render(tr_ctx* ctx) {
   if (rb->h_mega) cudaFreeHost(rb->h_mega);
   if (rb->mega_e0) cudaEventDestroy(rb->mega_e0);
   if (rb->mega_e1) cudaEventDestroy(rb->mega_e1);
+  for (cudaStream_t t : rb->side)
+    if (t) cudaStreamDestroy(t);
+  for (cudaEvent_t e : rb->fork_ev)
+    if (e) cudaEventDestroy(e);
   for (cudaEvent_t e : rb->ev_pool) cudaEventDestroy(e);
   delete rb;
   ctx->rb = nullptr;
@@ -1421,7 +1445,7 @@ tr_status reserve_render(tr_ctx* ctx, int n, int nl) {
                {&rb->M0, N * f4},           {&rb->M1, N * f4},          {&rb->M2, N * f4},
                {&rb->HC, N * f4},           {&rb->HM, N * f4},          {&rb->SC, N * 7 * f4},
                {&rb->NU, N * NL * 8},       {&rb->SH, N * NL * 2 * f4}, {&rb->SHC, N * NL * f4}, {&rb->acc, N * 32},
-               {&rb->q_ext, 2 * 2 * N * 4}, {&rb->q_act, 2 * N * 4},   {&rb->q_mat, kMatKinds * N * 4},
+               {&rb->q_ext, 2 * 2 * N * 4}, {&rb->q_mat, kMatKinds * N * 4},
                {&rb->q_nee, kNeeKinds * N * NL * 4}, {&rb->q_sh, N * NL * 4},  {&rb->ctr, kCtrWords * 4},
                {&rb->stats, kStatWords * 8}};
   for (auto& nd : needs) {
@@ -1741,7 +1765,6 @@ tr_status render_jobs(tr_ctx* ctx, const JobSpec* jobs, int njobs, uint32_t flag
   }
   for (int k = 0; k < 2; ++k) {
     P.q_ext[k] = rb->q_ext.as<int>() + (size_t)k * 2 * n;
-    P.q_act[k] = rb->q_act.as<int>() + (size_t)k * n;
   }
   for (int k = 0; k < kNeeKinds; ++k) P.q_nee[k] = rb->q_nee.as<int>() + (size_t)k * n * std::max(nl, 1);
   for (int k = 0; k < kMatKinds; ++k) P.q_mat[k] = rb->q_mat.as<int>() + (size_t)k * n;
@@ -1872,7 +1895,7 @@ tr_status render_jobs(tr_ctx* ctx, const JobSpec* jobs, int njobs, uint32_t flag
   RCHK(cudaMemsetAsync(P.ctr, 0, kCtrWords * 4, st));
   RCHK(cudaMemsetAsync(P.stats, 0, kStatWords * 8, st));
   if (P.OC) RCHK(cudaMemsetAsync(P.OC, 0xff, (size_t)n * P.nl_max * 4, st));
-  if (P.act_flag) RCHK(cudaMemsetAsync(P.act_flag, 0, (size_t)n, st));
+  if (P.bin_bits) RCHK(cudaMemsetAsync(P.bin_cnt, 0, (size_t)4 << (3 + 3 * P.bin_bits), st));
   RCHK(cudaEventRecord(e0, st));
   k_init<<<grid_init, 256, 0, st>>>(P);
   RCHK(cudaGetLastError());
@@ -1888,82 +1911,173 @@ tr_status render_jobs(tr_ctx* ctx, const JobSpec* jobs, int njobs, uint32_t flag
     }
     cudaEventRecord(ev[nev++], st);
   };
-  // one wavefront iteration; returns the first launch error
+  // The kernels of an iteration (of queue parity cur), by stage.
   const int bin_nb = P.bin_bits ? 1 << (3 + 3 * P.bin_bits) : 0;
-  auto iteration = [&](int cur) -> tr_status {
-    const int nxt = cur ^ 1;
-    mark();
-    if (P.bin_bits) {  // the extend queue in ray-key order
-      cudaMemsetAsync(P.bin_cnt, 0, (size_t)bin_nb * 4, st);
-      k_bin_count<<<grid, 128, 0, st>>>(ExtendSrc{P, cur}, P.sc, P.bin_cnt, P.bin_key, P.bin_bits);
-      k_bin_scan<<<1, kBinScanThreads, 0, st>>>(P.bin_cnt, bin_nb);
-      k_bin_scatter<<<grid, 128, 0, st>>>(ExtendSrc{P, cur}, P.bin_cnt, P.bin_key, P.q_srt);
+  bool kinds[kMatKinds] = {};
+  for (const DMat& m : ctx->hs.mats) kinds[m.kind] = true;
+  auto bin = [&](int cur, cudaStream_t t) {  // the extend queue in ray-key order
+    if (!P.bin_bits) return;
+    k_bin_count<<<grid, 128, 0, t>>>(ExtendSrc{P, cur}, P.sc, P.bin_cnt, P.bin_key, P.bin_bits);
+    k_bin_scan<<<1, kBinScanThreads, 0, t>>>(P.bin_cnt, bin_nb);
+    k_bin_scatter<<<grid, 128, 0, t>>>(ExtendSrc{P, cur}, P.bin_cnt, P.bin_key, P.q_srt);
+  };
+  auto extend = [&](int cur, cudaStream_t t) {
+    if (count) k_extend<true><<<grid_ext, 128, tl_smem, t>>>(P, cur);
+    else k_extend<false><<<grid_ext, 128, tl_smem, t>>>(P, cur);
+  };
+  auto order = [&](int cur, cudaStream_t t) { k_act_order<<<grid_init, 256, 0, t>>>(P, cur); };
+  auto logic = [&](int cur, cudaStream_t t) {
+    if (gp) k_logic<true><<<grid, 128, 0, t>>>(P, cur);
+    else k_logic<false><<<grid, 128, 0, t>>>(P, cur);
+  };
+  // decoded mixtures for this iteration's Phong-material vertices (inputs written by k_logic)
+  auto guide = [&](int cur, cudaStream_t t) -> tr_status {
+    if (!(P.guide_alpha > 0.0f)) return TR_OK;
+    return guide_forward_rows_on_device(ctx, P.gfeat, P.ctr + bank(cur) + B_GROW, P.gout, t);
+  };
+  auto material = [&](int kind, int cur, cudaStream_t t) {
+    if (!kinds[kind]) return;
+    switch (kind) {
+      case MAT_PHONG:
+        // the guided instantiation only when guiding (its code would slow the plain kernel)
+        if (P.guide_alpha > 0.0f) k_material<MAT_PHONG, true><<<grid, 128, 0, t>>>(P, cur);
+        else k_material<MAT_PHONG><<<grid, 128, 0, t>>>(P, cur);
+        break;
+      case MAT_DISNEY12: k_material<MAT_DISNEY12><<<grid, 128, 0, t>>>(P, cur); break;
+      case MAT_GLASS: k_glass<<<grid, 128, 0, t>>>(P, cur); break;
+      case MAT_METAL: k_material<MAT_METAL><<<grid, 128, 0, t>>>(P, cur); break;
+      case MAT_DISNEY15: k_material<MAT_DISNEY15><<<grid, 128, 0, t>>>(P, cur); break;
     }
-    mark();
-    if (count) k_extend<true><<<grid_ext, 128, tl_smem, st>>>(P, cur);
-    else k_extend<false><<<grid_ext, 128, tl_smem, st>>>(P, cur);
-    mark();
-    // next iteration's extend and live counts; this iteration's shadow,
-    // material and light-sample counts and the fetch positions
-    cudaMemsetAsync(P.ctr + C_EXT + nxt, 0, 4, st);
-    cudaMemsetAsync(P.ctr + C_ACT + nxt, 0, 4, st);
-    cudaMemsetAsync(P.ctr + C_SH, 0, 4 * (C_FSH + 1 - C_SH), st);  // C_SH, C_MAT, C_NEE, C_FEXT, C_FSH
-    if (P.guide_alpha > 0.0f) cudaMemsetAsync(P.ctr + C_GROW, 0, 4, st);
-    mark();
-    if (P.q_ord) {  // the live slots in slot order (timed with k_logic)
-      cudaMemsetAsync(P.ctr + C_ORD, 0, 4, st);
-      k_act_mark<<<grid, 256, 0, st>>>(P, cur);
-      k_act_order<<<grid_init, 256, 0, st>>>(P);
-    }
-    if (gp) k_logic<true><<<grid, 128, 0, st>>>(P, cur);
-    else k_logic<false><<<grid, 128, 0, st>>>(P, cur);
-    if (P.guide_alpha > 0.0f) {
-      // decoded mixtures for this iteration's Phong-material vertices (inputs written by k_logic)
-      tr_status gs = guide_forward_rows_on_device(ctx, P.gfeat, P.ctr + C_GROW, P.gout);
-      if (gs != TR_OK) return gs;
-    }
-    mark();
-    // the guided instantiation only when guiding (its code would slow the plain kernel)
-    if (P.guide_alpha > 0.0f) k_material<MAT_PHONG, true><<<grid, 128, 0, st>>>(P, cur);
-    else k_material<MAT_PHONG><<<grid, 128, 0, st>>>(P, cur);
-    mark();
-    k_material<MAT_DISNEY12><<<grid, 128, 0, st>>>(P, cur);
-    if (P.sc.has_glass) k_glass<<<grid, 128, 0, st>>>(P, cur);  // timed with Disney12
-    if (P.sc.has_metal) k_material<MAT_METAL><<<grid, 128, 0, st>>>(P, cur);
-    if (P.sc.has_disney15) k_material<MAT_DISNEY15><<<grid, 128, 0, st>>>(P, cur);
-    mark();
-    if (P.MT) k_nee<MAT_PHONG, true><<<grid, 128, 0, st>>>(P);
-    else k_nee<MAT_PHONG><<<grid, 128, 0, st>>>(P);
-    mark();
+  };
+  auto nee = [&](int kind, int cur, cudaStream_t t) {
     // (MAPS instantiations: hits of materials with image maps read the slot's set-up)
-    if (P.MT) k_nee<MAT_DISNEY12, true><<<grid, 128, 0, st>>>(P);
-    else k_nee<MAT_DISNEY12><<<grid, 128, 0, st>>>(P);
-    if (P.sc.has_metal) {  // timed with Disney12
-      if (P.MT) k_nee<MAT_METAL, true><<<grid, 128, 0, st>>>(P);
-      else k_nee<MAT_METAL><<<grid, 128, 0, st>>>(P);
+    if (!kinds[kind]) return;
+    switch (kind) {
+      case MAT_PHONG:
+        if (P.MT) k_nee<MAT_PHONG, true><<<grid, 128, 0, t>>>(P, cur);
+        else k_nee<MAT_PHONG><<<grid, 128, 0, t>>>(P, cur);
+        break;
+      case MAT_DISNEY12:
+        if (P.MT) k_nee<MAT_DISNEY12, true><<<grid, 128, 0, t>>>(P, cur);
+        else k_nee<MAT_DISNEY12><<<grid, 128, 0, t>>>(P, cur);
+        break;
+      case MAT_METAL:
+        if (P.MT) k_nee<MAT_METAL, true><<<grid, 128, 0, t>>>(P, cur);
+        else k_nee<MAT_METAL><<<grid, 128, 0, t>>>(P, cur);
+        break;
+      case MAT_DISNEY15:
+        if (P.MT) k_nee<MAT_DISNEY15, true><<<grid, 128, 0, t>>>(P, cur);
+        else k_nee<MAT_DISNEY15><<<grid, 128, 0, t>>>(P, cur);
+        break;
     }
-    if (P.sc.has_disney15) {
-      if (P.MT) k_nee<MAT_DISNEY15, true><<<grid, 128, 0, st>>>(P);
-      else k_nee<MAT_DISNEY15><<<grid, 128, 0, st>>>(P);
-    }
-    mark();
-    if (count && wide) k_shadow<true, true><<<grid_sh, 128, 0, st>>>(P);
-    else if (count) k_shadow<true><<<grid_sh, 128, sh_smem, st>>>(P);
-    else if (wide) k_shadow<false, true><<<grid_sh, 128, 0, st>>>(P);
-    else k_shadow<false><<<grid_sh, 128, sh_smem, st>>>(P);
-    mark();
-    cudaError_t e = cudaGetLastError();
+  };
+  auto shadow = [&](int cur, cudaStream_t t) {
+    if (count && wide) k_shadow<true, true><<<grid_sh, 128, 0, t>>>(P, cur);
+    else if (count) k_shadow<true><<<grid_sh, 128, sh_smem, t>>>(P, cur);
+    else if (wide) k_shadow<false, true><<<grid_sh, 128, 0, t>>>(P, cur);
+    else k_shadow<false><<<grid_sh, 128, sh_smem, t>>>(P, cur);
+  };
+  auto launched = [&]() -> tr_status {
+    const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TR_OK : cuda_fail(ctx, e, "wavefront launch");
   };
+  // One iteration, one kernel after another, with the events of stage timing
+  // (the reset stage has no launches of its own any more).
+  auto iteration = [&](int cur) -> tr_status {
+    mark();
+    bin(cur, st);
+    mark();
+    extend(cur, st);
+    mark();
+    mark();
+    order(cur, st);  // timed with k_logic, as is the guiding network
+    logic(cur, st);
+    const tr_status gs = guide(cur, st);
+    if (gs != TR_OK) return gs;
+    mark();
+    material(MAT_PHONG, cur, st);
+    mark();
+    for (int k : {MAT_DISNEY12, MAT_GLASS, MAT_METAL, MAT_DISNEY15}) material(k, cur, st);  // timed with Disney12
+    mark();
+    nee(MAT_PHONG, cur, st);
+    mark();
+    for (int k : {MAT_DISNEY12, MAT_METAL, MAT_DISNEY15}) nee(k, cur, st);
+    mark();
+    shadow(cur, st);
+    mark();
+    return launched();
+  };
+  // The same as a graph whose branches run side by side. It starts with the
+  // extend queue traced and the live slots ordered, and does both for the next
+  // iteration:
+  //
+  //   logic -> material of each kind -> (all) -> bin, extend  -> (join)
+  //                    |                  `----> order       ---'
+  //                    `-> light samples of the kind -> (all) -> shadow
+  //
+  // The next rays do not depend on the shadow rays, nor one material on
+  // another. A tail iteration (a few hundred paths left) is a chain of
+  // kernels that each take one warp's time, and this chain is half as long;
+  // in full iterations the traversal kernels' last rays overlap. Measured (ms,
+  // one kernel after another / this): maps on every material 1001x563x4 14.6 /
+  // 8.7, Disney grid 1024x1024x16 56.9 / 47.5, the 1024x768x16 room 184 / 165,
+  // its guided pass 106 / 98, a batch of 12 scenes 82 / 56.
+  auto branch = [&](cudaStream_t from, cudaStream_t to, int ev_k) {
+    cudaEventRecord(rb->fork_ev[ev_k], from);
+    cudaStreamWaitEvent(to, rb->fork_ev[ev_k], 0);
+  };
+  auto iteration_graph = [&](int cur) -> tr_status {
+    static const int kSide[kMatKinds] = {-1, 0, 1, 2, 3};  // the stream of a kind (Phong: the main one)
+    cudaStream_t sh_st = rb->side[4];
+    logic(cur, st);
+    cudaEventRecord(rb->fork_ev[0], st);
+    for (int k = 1; k < kMatKinds; ++k)
+      if (kinds[k]) {
+        cudaStreamWaitEvent(rb->side[kSide[k]], rb->fork_ev[0], 0);
+        material(k, cur, rb->side[kSide[k]]);
+        cudaEventRecord(rb->fork_ev[k], rb->side[kSide[k]]);
+      }
+    const tr_status gs = guide(cur, st);
+    if (gs != TR_OK) return gs;
+    material(MAT_PHONG, cur, st);
+    branch(st, sh_st, 5);
+    nee(MAT_PHONG, cur, sh_st);
+    for (int k = 1; k < kMatKinds; ++k)
+      if (kinds[k]) {
+        nee(k, cur, rb->side[kSide[k]]);
+        branch(rb->side[kSide[k]], sh_st, 5 + k);
+        cudaStreamWaitEvent(st, rb->fork_ev[k], 0);
+      }
+    shadow(cur, sh_st);
+    // (the glass stream has no light samples to wait for)
+    cudaStream_t or_st = rb->side[1];
+    branch(st, or_st, 10);
+    order(cur ^ 1, or_st);
+    bin(cur ^ 1, st);
+    extend(cur ^ 1, st);
+    branch(or_st, st, 11);
+    branch(sh_st, st, 5);
+    return launched();
+  };
+  const bool graphs = !timed && !count && ctx->tune.graph_iterations > 0;
+  if (graphs) {
+    for (cudaStream_t& t : rb->side)
+      if (!t) RCHK(cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking));
+    for (cudaEvent_t& e : rb->fork_ev)
+      if (!e) RCHK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    bin(0, st);
+    extend(0, st);
+    order(0, st);
+  }
   // Without per-kernel instrumentation, a chunk of iterations (an even
   // number, so each chunk starts on the same queue parity) is captured once
-  // into a CUDA graph and replayed: one launch per chunk instead of ten
-  // per iteration. The host still polls the live count between chunks.
-  const int chunk = (!timed && !count && ctx->tune.graph_iterations > 0) ? (ctx->tune.graph_iterations + 1) & ~1 : 4;
-  if (!timed && !count && ctx->tune.graph_iterations > 0) {
+  // into a CUDA graph and replayed. The host still polls the live count
+  // between chunks.
+  const int chunk = graphs ? (ctx->tune.graph_iterations + 1) & ~1 : 4;
+  if (graphs) {
     RCHK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     tr_status cs = TR_OK;
-    for (int c = 0; c < chunk && cs == TR_OK; ++c) cs = iteration(c & 1);
+    for (int c = 0; c < chunk && cs == TR_OK; ++c) cs = iteration_graph(c & 1);
     cudaError_t ee = cudaStreamEndCapture(st, &graph);
     if (cs != TR_OK) {
       cleanup();
@@ -2153,7 +2267,7 @@ tr_status render_noalloc_impl(tr_ctx* ctx, const tr_camera* cam, const tr_filter
   const size_t oP = L.take(5 * N * f4), oRng = L.take(N * 8), oM = L.take(3 * N * f4), oH = L.take(2 * N * f4),
                oSC = L.take(N * 7 * f4), oNU = L.take(N * NL * 8), oSH = L.take(N * NL * 2 * f4),
                oSHC = L.take(N * NL * f4),
-               oQe = L.take(2 * 2 * N * 4), oQa = L.take(2 * N * 4), oQm = L.take(kMatKinds * N * 4),
+               oQe = L.take(2 * 2 * N * 4), oQa = L.take(N * 4), oAf = L.take(N), oQm = L.take(kMatKinds * N * 4),
                oQn = L.take(kNeeKinds * N * NL * 4), oQs = L.take(N * NL * 4), oCtr = L.take(kCtrWords * 4),
                oSt = L.take(kStatWords * 8),
                oJob = L.take(sizeof(JobDev));
@@ -2221,12 +2335,12 @@ tr_status render_noalloc_impl(tr_ctx* ctx, const tr_camera* cam, const tr_filter
   P.SH = reinterpret_cast<float4*>(base + oSH);
   P.SHC = reinterpret_cast<float4*>(base + oSHC);
   int* qe = reinterpret_cast<int*>(base + oQe);
-  int* qa = reinterpret_cast<int*>(base + oQa);
+  P.q_ord = reinterpret_cast<int*>(base + oQa);
+  P.act_flag = base + oAf;
   int* qm = reinterpret_cast<int*>(base + oQm);
   int* qn = reinterpret_cast<int*>(base + oQn);
   for (int k = 0; k < 2; ++k) {
     P.q_ext[k] = qe + (size_t)k * 2 * N;
-    P.q_act[k] = qa + (size_t)k * N;
   }
   for (int k = 0; k < kNeeKinds; ++k) P.q_nee[k] = qn + (size_t)k * N * NL;
   for (int k = 0; k < kMatKinds; ++k) P.q_mat[k] = qm + (size_t)k * N;
@@ -2292,23 +2406,21 @@ tr_status render_noalloc_impl(tr_ctx* ctx, const tr_camera* cam, const tr_filter
   unsigned int live = 1;
   bool cancelled = false;
   while (it < iters && live != 0 && !cancelled) {
-    const int cur = (int)(it & 1), nxt = cur ^ 1;
+    const int cur = (int)(it & 1);
     k_extend<false><<<grid_ext, 128, 0, st>>>(P, cur);
-    NCHK(cudaMemsetAsync(P.ctr + C_EXT + nxt, 0, 4, st));
-    NCHK(cudaMemsetAsync(P.ctr + C_ACT + nxt, 0, 4, st));
-    NCHK(cudaMemsetAsync(P.ctr + C_SH, 0, 4 * (C_FSH + 1 - C_SH), st));  // C_SH, C_MAT, C_NEE, C_FEXT, C_FSH
+    k_act_order<<<grid_init, 256, 0, st>>>(P, cur);
     k_logic<false><<<grid, 128, 0, st>>>(P, cur);
     k_material<MAT_PHONG><<<grid, 128, 0, st>>>(P, cur);
     k_material<MAT_DISNEY12><<<grid, 128, 0, st>>>(P, cur);
     if (P.sc.has_glass) k_glass<<<grid, 128, 0, st>>>(P, cur);
     if (P.sc.has_metal) k_material<MAT_METAL><<<grid, 128, 0, st>>>(P, cur);
     if (P.sc.has_disney15) k_material<MAT_DISNEY15><<<grid, 128, 0, st>>>(P, cur);
-    k_nee<MAT_PHONG><<<grid, 128, 0, st>>>(P);
-    k_nee<MAT_DISNEY12><<<grid, 128, 0, st>>>(P);
-    if (P.sc.has_metal) k_nee<MAT_METAL><<<grid, 128, 0, st>>>(P);
-    if (P.sc.has_disney15) k_nee<MAT_DISNEY15><<<grid, 128, 0, st>>>(P);
-    if (wide) k_shadow<false, true><<<grid_sh, 128, 0, st>>>(P);
-    else k_shadow<false><<<grid_sh, 128, 0, st>>>(P);
+    k_nee<MAT_PHONG><<<grid, 128, 0, st>>>(P, cur);
+    k_nee<MAT_DISNEY12><<<grid, 128, 0, st>>>(P, cur);
+    if (P.sc.has_metal) k_nee<MAT_METAL><<<grid, 128, 0, st>>>(P, cur);
+    if (P.sc.has_disney15) k_nee<MAT_DISNEY15><<<grid, 128, 0, st>>>(P, cur);
+    if (wide) k_shadow<false, true><<<grid_sh, 128, 0, st>>>(P, cur);
+    else k_shadow<false><<<grid_sh, 128, 0, st>>>(P, cur);
     ++it;
     if (it % kDrainCheck == 0 || it == iters) {
       NCHK(cudaGetLastError());
