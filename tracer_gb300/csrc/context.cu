@@ -483,7 +483,8 @@ struct BatchJob {
   const int* perm;  // ray binning: work item i is ray perm[i] (null: ray i)
   __device__ __forceinline__ unsigned int count() const { return n; }
   __device__ __forceinline__ int cached(unsigned int) const { return -1; }
-  __device__ __forceinline__ void load(unsigned int w, f3& o, f3& d, float& t_min, float& t_max, int& scene) const {
+  __device__ __forceinline__ unsigned int load(unsigned int w, f3& o, f3& d, float& t_min, float& t_max,
+                                               int& scene) const {
     scene = 0;
     const unsigned int i = perm ? (unsigned int)perm[w] : w;
     const float4 r0 = __ldg(rays + 2 * (size_t)i), r1 = __ldg(rays + 2 * (size_t)i + 1);
@@ -491,9 +492,9 @@ struct BatchJob {
     d = mk3(r0.w, r1.x, r1.y);
     t_min = r1.z;
     t_max = r1.w;
+    return i;
   }
-  __device__ __forceinline__ void store(unsigned int w, const Hit& h, float t_max, bool occluded) const {
-    const unsigned int i = perm ? (unsigned int)perm[w] : w;
+  __device__ __forceinline__ void store(unsigned int i, const Hit& h, float t_max, bool occluded) const {
     if (prim) {
       prim[i] = h.prim;
       tout[i] = t_max;

@@ -432,7 +432,8 @@ struct ExtendJob {
   __device__ ExtendJob(const Launch& P_, int cur_) : P(P_), cur(cur_), q(P_.bin_bits ? P_.q_srt : P_.q_ext[cur_]) {}
   __device__ __forceinline__ unsigned int count() const { return P.ctr[C_EXT + cur]; }
   __device__ __forceinline__ int cached(unsigned int) const { return -1; }
-  __device__ __forceinline__ void load(unsigned int i, f3& o, f3& d, float& t_min, float& t_max, int& scene) const {
+  __device__ __forceinline__ unsigned int load(unsigned int i, f3& o, f3& d, float& t_min, float& t_max,
+                                               int& scene) const {
     const int e = q[i];
     const int slot = e >> 1;
     scene = job_of(P, slot).scene;
@@ -442,9 +443,9 @@ struct ExtendJob {
     d = mk3(b.x, b.y, b.z);
     t_min = 0.0f;
     t_max = kRealMax;
+    return (unsigned int)e;
   }
-  __device__ __forceinline__ void store(unsigned int i, const Hit& h, float, bool) const {
-    const int e = q[i];
+  __device__ __forceinline__ void store(unsigned int e, const Hit& h, float, bool) const {
     const float4 rec = make_float4(__int_as_float(h.prim), h.t_attr, h.alpha, h.beta);
     if (e & 1) P.HM[e >> 1] = rec;
     else P.HC[e >> 1] = rec;
@@ -459,8 +460,9 @@ struct ShadowJob {
   __device__ ShadowJob(const Launch& P_, int cur_) : P(P_), cur(cur_), q(P_.q_sh) {}
   __device__ __forceinline__ unsigned int count() const { return P.ctr[bank(cur) + B_SH]; }
   // the slot that last blocked this (pixel slot, light) item's shadow ray
-  __device__ __forceinline__ int cached(unsigned int i) const { return P.OC ? P.OC[q[i]] : -1; }
-  __device__ __forceinline__ void load(unsigned int i, f3& o, f3& d, float& t_min, float& t_max, int& scene) const {
+  __device__ __forceinline__ int cached(unsigned int r) const { return P.OC ? P.OC[r] : -1; }
+  __device__ __forceinline__ unsigned int load(unsigned int i, f3& o, f3& d, float& t_min, float& t_max,
+                                               int& scene) const {
     const int r = q[i];
     scene = job_of(P, r / P.nl_max).scene;
     const float4 a = P.SH[2 * r], b = P.SH[2 * r + 1];
@@ -468,11 +470,12 @@ struct ShadowJob {
     d = mk3(b.x, b.y, b.z);
     t_min = kEps;
     t_max = a.w;
+    return (unsigned int)r;
   }
-  __device__ __forceinline__ void store(unsigned int i, const Hit& h, float, bool occluded) const {
+  __device__ __forceinline__ void store(unsigned int r, const Hit& h, float, bool occluded) const {
     if (occluded) {
-      P.SHC[q[i]].w = 0.0f;
-      if (P.OC) P.OC[q[i]] = h.prim;
+      P.SHC[r].w = 0.0f;
+      if (P.OC) P.OC[r] = h.prim;
     }
   }
 };

@@ -38,6 +38,19 @@ struct Hit {
 
 __device__ __forceinline__ float4 ldg4(const float4* p) { return __ldg(p); }
 
+// Two float4 in one 32-byte load (p 32-byte aligned). Not in the persistent
+// render kernel: ptxas 13.0 does not compile that with it.
+__device__ __forceinline__ void ldg8(const float4* p, float4& a, float4& b) {
+#if defined(TRG_MATH_OUT_OF_LINE)
+  a = ldg4(p);
+  b = ldg4(p + 1);
+#else
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+#endif
+}
+
 // The shared-memory treelet (DScene::treelet, staged by each block of a
 // traversal kernel into its dynamic shared memory). Float4 k of treelet node j
 // sits at 4 * j + (k ^ ((j >> 1) & 3)): eight lanes reading the same field of
@@ -423,10 +436,8 @@ struct TravLane {
       dd = trav_smem[treelet_slot(j, 3)];
     } else {
       const float4* np = reinterpret_cast<const float4*>(sc.nodes + cur);
-      a = ldg4(np);
-      b = ldg4(np + 1);
-      c = ldg4(np + 2);
-      dd = ldg4(np + 3);
+      ldg8(np, a, b);
+      ldg8(np + 2, c, dd);
     }
     if (COUNT) vc.boxes += 2;
     float tl, tr;
@@ -580,13 +591,22 @@ struct TravLane {
 };
 
 // Job: unsigned count() const;
-//      void load(unsigned i, f3& o, f3& d, float& t_min, float& t_max, int& scene);
+//      unsigned load(unsigned i, f3& o, f3& d, float& t_min, float& t_max, int& scene);
+//        ray i of the queue; what it returns names the ray to cached and store
 //      int cached(unsigned i) const;  any hits: a slot to test first (occluded_by_slot), or -1
 //      void store(unsigned i, const Hit& h, float t_max, bool occluded).
 // For an occluded any-hit ray h.prim is the occluding slot.
 // tl_n: treelet nodes to stage in shared memory (the launch gives the block
 // at least tl_n * 64 bytes of dynamic shared memory; 0: none). The four-wide
 // walk does not use the treelet.
+// Lanes still looking for a leaf below which the warp tests the leaves it has:
+// waiting for the last few costs more than coming back for them. 1024x768x16
+// room 165 -> 158 ms (its any hits 37.3 -> 32.9 ms), 2M closest + 2M any hits
+// in 1M triangles 4.94 -> 4.79 ms, the sphere grid 48.9 -> 50.1 ms; with 8:
+// 160, 4.80, 51.0. With the 32-byte node loads and the queue entry kept in the
+// lane: 155, 4.55, 49.4 ms.
+constexpr int kWalkLanes = 4;
+
 template <bool ANY, bool COUNT, bool WIDE = false, class Job>
 __device__ __forceinline__ void persistent_traverse(const DScene& sc, Job& job, unsigned int* fetch, int* err,
                                                     VisitCount& vc, int refill, int tl_n = 0) {
@@ -611,7 +631,7 @@ __device__ __forceinline__ void persistent_traverse(const DScene& sc, Job& job, 
           f3 o, d;
           float tmin, tmax;
           int scene;
-          job.load(item, o, d, tmin, tmax, scene);
+          item = job.load(item, o, d, tmin, tmax, scene);
           const int cs = ANY ? job.cached(item) : -1;
           if (ANY && cs >= 0 && occluded_by_slot(sc, scene, cs, o, d, tmin, tmax)) {
             ++vc.cache_hits;
@@ -647,13 +667,14 @@ __device__ __forceinline__ void persistent_traverse(const DScene& sc, Job& job, 
         if (__popc(__ballot_sync(0xffffffffu, live)) < refill) break;
       }
     } else {
-      // speculative while-while: interior steps go on while some lane has
-      // not found a leaf; a lane holding a postponed leaf keeps walking
+      // speculative while-while: interior steps go on while kWalkLanes lanes
+      // have not found a leaf; a lane holding a postponed leaf keeps walking
       // (and waits at a second leaf); then the postponed leaves are tested
       for (;;) {
         for (;;) {
           if (live && L.cnt > 0 && L.pc == 0) L.postpone();
-          if (!__any_sync(0xffffffffu, live && L.pc == 0)) break;
+          const unsigned int walking = __ballot_sync(0xffffffffu, live && L.pc == 0);
+          if (__popc(walking) < kWalkLanes && (walking == 0 || __any_sync(0xffffffffu, live && L.pc > 0))) break;
           if (live && L.cnt == 0) {
             const bool more = WIDE ? L.interior4(sc, err, vc) : L.interior(sc, err, vc);
             if (!more) {
@@ -666,7 +687,7 @@ __device__ __forceinline__ void persistent_traverse(const DScene& sc, Job& job, 
             }
           }
         }
-        if (live) {
+        if (live && L.pc > 0) {
           live = L.postponed_leaf(sc, vc);
           if (!live) job.store(item, L.h, L.t_max, L.occluded);
         }
