@@ -265,7 +265,8 @@ tr_status tr_synchronize(tr_ctx* ctx);
  *  - shade_blocks_per_sm: 128-thread blocks per SM of the shading kernels
  *    (grid-stride loops);
  *  - graph_iterations: wavefront iterations captured into one CUDA graph
- *    and replayed as one launch (rounded up to even; 0: no graph);
+ *    and replayed as one launch (at most two, one per queue parity; 0: no
+ *    graph, one launch after another);
  *  - any_node_width (2 or 4): BVH node width of any-hit (shadow) traversal.
  *    Width 4 walks a tree collapsed from the reference's binary BVH: its
  *    boxes are a subset of the binary tree's, and the slab test passes a box
