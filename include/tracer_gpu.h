@@ -297,7 +297,7 @@ tr_status tr_synchronize(tr_ctx* ctx);
  *    owning lane running a pixel's samples with the path state in registers
  *    (a batch's launch and film zeroing captured into a CUDA graph when
  *    graph_iterations > 0); TR_RENDER_MODE_AUTO picks the persistent kernel
- *    for renders of at most 2^17 pixels. Guided and instrumented renders
+ *    for renders of at most 2^16 pixels (2^15 with image maps). Guided and instrumented renders
  *    (TR_RENDER_TIME_STAGES, TR_RENDER_COUNT_VISITS) and scenes with more
  *    than 16 lights always use the wavefront. Films are identical.
  *  - any_hit_order: the child a binary any-hit walk enters first when both

@@ -90,8 +90,15 @@ constexpr int kCtrWords = C_BANK + 2 * kBankWords;  // the counter array
 // Statistics words: samples, extend rays, shadow rays, shade items, visit
 // counts (4-7), occluder-cache hits (8).
 constexpr int kStatWords = 16;
-// render_mode auto: renders of at most this many pixels use the persistent kernel
-constexpr long long kMegaAutoSlots = 1 << 17;
+// render_mode auto: renders of at most this many pixels use the persistent
+// kernel, of scenes with image maps half as many (their set-ups at a hit
+// diverge most). Wavefront / persistent us, 16 samples, at 30,000, 66,000 and
+// 128,000 pixels: Cornell box 6640/4010, 7370/5930, 10130/10020; outdoor
+// 9280/7680, 10660/11310, 12170/16430; sphere grid 10250/7470, 12140/11400,
+// 14250/18630; occluded room 30490/20930, 37220/39900, 47870/67860; maps on
+// every material 11580/14500, 12960/21440, 15610/31680 (2 samples 2370/1990,
+// 2510/2780, 3560/4060).
+constexpr long long kMegaAutoSlots = 1 << 16;
 // Material code in the shading context: the material index, or with this bit
 // set the slot's own set-up in Launch::MT (a Phong material with maps).
 constexpr int kMatScratch = 1 << 30;
@@ -1767,7 +1774,7 @@ tr_status render_jobs(tr_ctx* ctx, const JobSpec* jobs, int njobs, uint32_t flag
   // kMegaAutoSlots pixels, which the wavefront's launches cannot fill the GPU with
   if (!gp && !(flags & (TR_RENDER_TIME_STAGES | TR_RENDER_COUNT_VISITS)) && nl <= kMegaLights &&
       (ctx->tune.render_mode == TR_RENDER_MODE_PERSISTENT ||
-       (ctx->tune.render_mode == TR_RENDER_MODE_AUTO && (long long)n <= kMegaAutoSlots)))
+       (ctx->tune.render_mode == TR_RENDER_MODE_AUTO && (long long)n <= kMegaAutoSlots >> (ctx->dsc.has_textures ? 1 : 0))))
     return render_persistent(ctx, jobs, njobs, n, nl, sms, stats);
   tr_status s = reserve_render(ctx, n, nl);
   if (s != TR_OK) return s;
