@@ -519,7 +519,7 @@ struct BatchSrc {
 };
 
 template <bool ANY, bool WIDE = false>
-__global__ void __launch_bounds__(128) k_trace_batch(DScene sc, BatchJob job, unsigned int* fetch, int* err,
+__global__ void __launch_bounds__(128, ANY ? 8 : 9) k_trace_batch(DScene sc, BatchJob job, unsigned int* fetch, int* err,
                                                     int refill, int tl_n) {
   VisitCount vc;
   persistent_traverse<ANY, false, WIDE>(sc, job, fetch, err, vc, refill, tl_n);
