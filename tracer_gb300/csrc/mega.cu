@@ -255,8 +255,8 @@ __device__ __forceinline__ bool light_item(const DScene& sc, const DLight& lt, c
   return true;
 }
 
-template <unsigned MASK>
-__global__ void __launch_bounds__(kMegaThreads, 1) k_mega(MegaLaunch P) {
+template <unsigned MASK, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) k_mega(MegaLaunch P) {
   extern __shared__ float4 pools[];
   const DScene& sc = P.sc;
   const int lane = (int)(threadIdx.x & 31u);
@@ -643,10 +643,21 @@ constexpr unsigned kMaskPhong = MK_PHONG;
 constexpr unsigned kMaskPD = MK_PHONG | MK_DISNEY12;
 constexpr unsigned kMaskAll = MK_PHONG | MK_DISNEY12 | MK_GLASS | MK_METAL | MK_DISNEY15 | MK_ENV | MK_MAPS;
 
-const void* kernel_of(unsigned mask) {
-  if (mask == kMaskPhong) return (const void*)k_mega<kMaskPhong>;
-  if (mask == kMaskPD) return (const void*)k_mega<kMaskPD>;
-  return (const void*)k_mega<kMaskAll>;
+template <unsigned MASK, int THREADS>
+cudaError_t launch(const MegaLaunch& P, int grid, cudaStream_t st) {
+  constexpr size_t smem = (size_t)(THREADS / 32) * kPoolBytes;
+  const cudaError_t e = cudaFuncSetAttribute((const void*)k_mega<MASK, THREADS>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k_mega<MASK, THREADS><<<grid, THREADS, smem, st>>>(P);
+  return cudaGetLastError();
+}
+
+template <int THREADS>
+cudaError_t launch(const MegaLaunch& P, unsigned mask, int grid, cudaStream_t st) {
+  if (mask == kMaskPhong) return launch<kMaskPhong, THREADS>(P, grid, st);
+  if (mask == kMaskPD) return launch<kMaskPD, THREADS>(P, grid, st);
+  return launch<kMaskAll, THREADS>(P, grid, st);
 }
 
 }  // namespace
@@ -656,15 +667,9 @@ unsigned mega_kernel_mask(const DScene& sc, bool has_disney12) {
   return has_disney12 ? kMaskPD : kMaskPhong;
 }
 
-cudaError_t launch_mega(const MegaLaunch& P, unsigned mask, int grid, cudaStream_t st) {
-  const int threads = kMegaThreads;
-  const size_t smem = (size_t)(threads / 32) * kPoolBytes;
-  const cudaError_t e = cudaFuncSetAttribute(kernel_of(mask), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  if (mask == kMaskPhong) k_mega<kMaskPhong><<<grid, threads, smem, st>>>(P);
-  else if (mask == kMaskPD) k_mega<kMaskPD><<<grid, threads, smem, st>>>(P);
-  else k_mega<kMaskAll><<<grid, threads, smem, st>>>(P);
-  return cudaGetLastError();
+cudaError_t launch_mega(const MegaLaunch& P, unsigned mask, const MegaShape& shape, cudaStream_t st) {
+  return shape.threads == kMegaFewThreads ? launch<kMegaFewThreads>(P, mask, shape.grid, st)
+                                          : launch<kMegaThreads>(P, mask, shape.grid, st);
 }
 
 }  // namespace trg

@@ -37,9 +37,14 @@ struct MegaLaunch {
 
 // The smallest instantiation covering a scene set (MK_* bits).
 unsigned mega_kernel_mask(const DScene& sc, bool has_disney12);
-// Launches the persistent kernel of instantiation `mask` (grid blocks of
-// kMegaThreads threads, at most one per SM resident) on `st`.
-cudaError_t launch_mega(const MegaLaunch& P, unsigned mask, int grid, cudaStream_t st);
-constexpr int kMegaThreads = 512;
+// Threads of a block, of which one is resident per SM: of the usual
+// instantiations (128 registers a thread) and of those for few pixels (255).
+constexpr int kMegaThreads = 512, kMegaFewThreads = 256;
+struct MegaShape {
+  int threads, lanes, grid;
+};
+// Launches the persistent kernel of instantiation `mask` and of the shape's
+// block size on `st`.
+cudaError_t launch_mega(const MegaLaunch& P, unsigned mask, const MegaShape& shape, cudaStream_t st);
 
 }  // namespace trg

@@ -1628,21 +1628,27 @@ static JobDev make_job_dev(tr_ctx* ctx, const JobSpec& j, int slot_base, void* f
   return J;
 }
 
-// Launch shape of the persistent kernel for n pixels: blocks of 512 threads
-// (one per SM), and no more pixel-owning lanes per warp than it takes to have
-// every pixel resident at once: a warp's other lanes walk rays and evaluate
-// light samples all the same, and fewer paths per warp diverge less. Measured
-// (us, lanes 32 / by this rule): all material kinds at 61x47x1 1423 / 782 (2),
-// Cornell 125x93x2 796 / 540 (5), Disney grid 200x150x4 3295 / 2300 (13), all
-// kinds under an environment light 320x180x8 5245 / 4917 (24), Cornell
-// 256x256x16 6503 / 6109 (27). Blocks of 256 and 128 threads at their best
-// lane counts were 0-15% slower.
-struct MegaShape {
-  int lanes, grid;
-};
+// Launch shape of the persistent kernel for n pixels: one block per SM, and no
+// more pixel-owning lanes per warp than it takes to have every pixel resident
+// at once: a warp's other lanes walk rays and evaluate light samples all the
+// same, and fewer paths per warp diverge less. Measured (us, lanes 32 / by
+// this rule): all material kinds at 61x47x1 1423 / 782 (2), Cornell 125x93x2
+// 796 / 540 (5), Disney grid 200x150x4 3295 / 2300 (13), all kinds under an
+// environment light 320x180x8 5245 / 4917 (24), Cornell 256x256x16 6503 /
+// 6109 (27).
+// Half the warps with twice the registers (255, which end the spills) where
+// they need at most kFewLanes lanes each: with few paths per warp a vertex's
+// latency counts, with many the warps to hide it. 512 / 256 threads, us, of
+// Cornell box, outdoor, maps on every material, sphere grid and occluded room:
+// 61x47x2 391/291 552/495 847/781 742/623 1414/1125; 125x93x16 3217/2512
+// 5417/5245 10442/9320 5721/5029 13465/13063; 200x150x4 1048/1046 1902/2374
+// 3649/3773 2172/2300 5511/6709; 256x256x16 6094/7533 12013/11750 23853/20806
+// 11152/13700 35934/43885.
 static MegaShape mega_shape(int n, int sms) {
-  constexpr int warps = kMegaThreads / 32;
+  constexpr int kFewLanes = 12;
   MegaShape s;
+  s.threads = n <= sms * (kMegaFewThreads / 32) * kFewLanes ? kMegaFewThreads : kMegaThreads;
+  const int warps = s.threads / 32;
   s.lanes = std::min(32, (n + sms * warps - 1) / (sms * warps));
   s.grid = std::min(sms, (n + warps * s.lanes - 1) / (warps * s.lanes));
   return s;
@@ -1704,7 +1710,7 @@ static tr_status render_persistent(tr_ctx* ctx, const JobSpec* jobs, int njobs, 
   TR_CUDA(ctx, rb->mega_state.reserve(kCtrBytes + kStatBytes));
   TR_CUDA(ctx, rb->jobs.reserve((size_t)njobs * sizeof(JobDev)));
   if (!jobs[0].film) TR_CUDA(ctx, rb->acc.reserve((size_t)n * 32));
-  if (ctx->dsc.has_textures) TR_CUDA(ctx, rb->MT.reserve((size_t)shape.grid * kMegaThreads * sizeof(DMat)));
+  if (ctx->dsc.has_textures) TR_CUDA(ctx, rb->MT.reserve((size_t)shape.grid * shape.threads * sizeof(DMat)));
   if (!rb->h_mega) TR_CUDA(ctx, cudaHostAlloc((void**)&rb->h_mega, kCtrBytes + kStatBytes, cudaHostAllocDefault));
   for (cudaEvent_t* e : {&rb->mega_e0, &rb->mega_e1})
     if (!*e) TR_CUDA(ctx, cudaEventCreate(e));
@@ -1728,7 +1734,7 @@ static tr_status render_persistent(tr_ctx* ctx, const JobSpec* jobs, int njobs, 
   for (int k = 0; k < njobs && le == cudaSuccess; ++k)
     le = cudaMemsetAsync(jd[k].film, 0, (size_t)jd[k].W * jd[k].H * (jd[k].fp64 ? 32 : 16), st);
   if (le == cudaSuccess) le = cudaMemsetAsync(ctr, 0, kCtrBytes + kStatBytes, st);
-  if (le == cudaSuccess) le = launch_mega(M, mask, shape.grid, st);
+  if (le == cudaSuccess) le = launch_mega(M, mask, shape, st);
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
   if (use_graph) {
@@ -2482,7 +2488,7 @@ tr_status render_noalloc_impl(tr_ctx* ctx, const tr_camera* cam, const tr_filter
     NCHK(cudaMemsetAsync(P.ctr, 0, kCtrWords * 4, st));
     NCHK(cudaMemsetAsync(P.stats, 0, kStatWords * 8, st));
     ctx->cancel.store(0);
-    const cudaError_t le = launch_mega(M, mega_mask(ctx), shape.grid, st);
+    const cudaError_t le = launch_mega(M, mega_mask(ctx), shape, st);
     if (le == cudaSuccess) {
       unsigned long long hs[kStatWords];
       unsigned int ctrs[kCtrWords];
