@@ -263,7 +263,7 @@ tr_status tr_synchronize(tr_ctx* ctx);
  *  - trav_blocks_per_sm: resident 128-thread blocks per SM of the
  *    persistent traversal kernels (0: as many as fit);
  *  - shade_blocks_per_sm: 128-thread blocks per SM of the shading kernels
- *    (grid-stride loops);
+ *    (grid-stride loops; in graphs at most 8 of the light-sample kernels);
  *  - graph_iterations: wavefront iterations captured into one CUDA graph
  *    and replayed as one launch (at most two, one per queue parity; 0: no
  *    graph, one launch after another);

@@ -99,6 +99,14 @@ constexpr int kStatWords = 16;
 // every material 11580/14500, 12960/21440, 15610/31680 (2 samples 2370/1990,
 // 2510/2780, 3560/4060).
 constexpr long long kMegaAutoSlots = 1 << 16;
+// Most blocks per SM of k_nee and k_remembered in graphs, whose queues hold an
+// item per vertex and light: about what is resident (6 and 12). With 32 the
+// blocks of one kernel held the SMs' slots against the other branches' kernels
+// (alone, without branches, k_nee is a fifth slower with 8). 32 / 16 / 8 and 12, ms: room
+// 1024x768x16 147.5 / 144.4 / 144.1, 900x700x8 63.4 / 61.9 / 61.4, 640x480x8
+// 38.3 / 38.1 / 37.5; guided 90.2 / 88.7 / 89.0; sphere grid 47.5 / 47.3 /
+// 47.2; batch of 12 scenes 58.1 / 58.1 / 58.1. (Materials and k_logic: no gain.)
+constexpr int kNeeBlocks = 8, kRememberedBlocks = 12;
 // Material code in the shading context: the material index, or with this bit
 // set the slot's own set-up in Launch::MT (a Phong material with maps).
 constexpr int kMatScratch = 1 << 30;
@@ -1947,6 +1955,7 @@ tr_status render_jobs(tr_ctx* ctx, const JobSpec* jobs, int njobs, uint32_t flag
   cudaGraphExec_t gexec[3] = {};
   const bool timed = (flags & TR_RENDER_TIME_STAGES) != 0;
   const bool count = (flags & TR_RENDER_COUNT_VISITS) != 0;
+  const bool graphs = !timed && !count && ctx->tune.graph_iterations > 0;
   std::vector<cudaEvent_t>& ev = rb->ev_pool;
   size_t nev = 0;
   auto cleanup = [&]() {
@@ -2026,24 +2035,25 @@ tr_status render_jobs(tr_ctx* ctx, const JobSpec* jobs, int njobs, uint32_t flag
     }
   };
   auto nee = [&](int kind, int cur, cudaStream_t t) {
+    const int grid_nee = graphs ? std::min(grid, sms * kNeeBlocks) : grid;
     // (MAPS instantiations: hits of materials with image maps read the slot's set-up)
     if (!kinds[kind]) return;
     switch (kind) {
       case MAT_PHONG:
-        if (P.MT) k_nee<MAT_PHONG, true><<<grid, 128, 0, t>>>(P, cur);
-        else k_nee<MAT_PHONG><<<grid, 128, 0, t>>>(P, cur);
+        if (P.MT) k_nee<MAT_PHONG, true><<<grid_nee, 128, 0, t>>>(P, cur);
+        else k_nee<MAT_PHONG><<<grid_nee, 128, 0, t>>>(P, cur);
         break;
       case MAT_DISNEY12:
-        if (P.MT) k_nee<MAT_DISNEY12, true><<<grid, 128, 0, t>>>(P, cur);
-        else k_nee<MAT_DISNEY12><<<grid, 128, 0, t>>>(P, cur);
+        if (P.MT) k_nee<MAT_DISNEY12, true><<<grid_nee, 128, 0, t>>>(P, cur);
+        else k_nee<MAT_DISNEY12><<<grid_nee, 128, 0, t>>>(P, cur);
         break;
       case MAT_METAL:
-        if (P.MT) k_nee<MAT_METAL, true><<<grid, 128, 0, t>>>(P, cur);
-        else k_nee<MAT_METAL><<<grid, 128, 0, t>>>(P, cur);
+        if (P.MT) k_nee<MAT_METAL, true><<<grid_nee, 128, 0, t>>>(P, cur);
+        else k_nee<MAT_METAL><<<grid_nee, 128, 0, t>>>(P, cur);
         break;
       case MAT_DISNEY15:
-        if (P.MT) k_nee<MAT_DISNEY15, true><<<grid, 128, 0, t>>>(P, cur);
-        else k_nee<MAT_DISNEY15><<<grid, 128, 0, t>>>(P, cur);
+        if (P.MT) k_nee<MAT_DISNEY15, true><<<grid_nee, 128, 0, t>>>(P, cur);
+        else k_nee<MAT_DISNEY15><<<grid_nee, 128, 0, t>>>(P, cur);
         break;
     }
   };
@@ -2052,7 +2062,8 @@ tr_status render_jobs(tr_ctx* ctx, const JobSpec* jobs, int njobs, uint32_t flag
     if (count && wide) k_shadow<true, true><<<grid_sh, 128, 0, t>>>(P, cur);
     else if (count) k_shadow<true><<<grid_sh, 128, sh_smem, t>>>(P, cur);
     else if (remembered) {
-      k_remembered<<<grid, 128, 0, t>>>(P, cur);
+      const int grid_rem = std::min(grid, sms * kRememberedBlocks);
+      k_remembered<<<grid_rem, 128, 0, t>>>(P, cur);
       if (wide) k_shadow<false, true, true><<<grid_sh, 128, 0, t>>>(P, cur);
       else k_shadow<false, false, true><<<grid_sh, 128, sh_smem, t>>>(P, cur);
     } else if (wide) k_shadow<false, true><<<grid_sh, 128, 0, t>>>(P, cur);
@@ -2140,7 +2151,6 @@ tr_status render_jobs(tr_ctx* ctx, const JobSpec* jobs, int njobs, uint32_t flag
     branch(sh_st, st, 5);
     return launched();
   };
-  const bool graphs = !timed && !count && ctx->tune.graph_iterations > 0;
   if (graphs) {
     for (cudaStream_t& t : rb->side)
       if (!t) RCHK(cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking));
