@@ -88,7 +88,9 @@ bool build_env_tables(const tr_scene_desc* d, EnvHost& env, std::string& err) {
       for (int sy = yb; sy <= ye; ++sy)
         for (int sx = xb; sx <= xe; ++sx) {
           const float su = (float)(sx + 0.5) / w, sv = (float)(sy + 0.5) / h;
-          const f3 c = ldr ? env_tex_eval8(tex8, w, h, su, sv) : env_tex_eval(tex, w, h, su, sv);
+          float uw, vw;
+          tex_wrap(su, sv, uw, vw);  // (the host's doubles are fast: the expressions as written)
+          const f3 c = ldr ? env_tex_eval8_d(tex8, w, h, uw, vw) : env_tex_eval_d(tex, w, h, uw, vw);
           lum += 0.2126f * c.x + 0.7152f * c.y + 0.0722f * c.z;
         }
       // d_omega = sin(theta) d_theta d_phi over the cell, the sine in double
