@@ -412,11 +412,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_mega(MegaLaunch P) {
         if (!more) __syncthreads();
         // ---- trace (k_extend, k_shadow)
         n_hits += pool_trace(sc, pool, traced, n, P.occluder_cache && sc.slot_leaf, P.err);
+        // (a pixel's last vertex is gathered after the lane has claimed its
+        // next pixel, which may be another scene's: oc is that pixel's by then)
+        const bool remember = !due || due_slot == p.slot;
         for (int e = mine; e < mine + n_mine; ++e) {
           const float4 c = pc[e];
           const int w = __float_as_int(c.w);
-          if (w >= 0 && (w & kBlocked)) oc[(__float_as_int(pb[e].w) >> 7) & 31] = w & ~kBlocked;
-          else direct = direct + mk3(c.x, c.y, c.z);
+          if (w < 0 || !(w & kBlocked)) direct = direct + mk3(c.x, c.y, c.z);
+          else if (remember) oc[(__float_as_int(pb[e].w) >> 7) & 31] = w & ~kBlocked;
         }
         __syncwarp();
         n = traced = front;
