@@ -429,9 +429,7 @@ __device__ __forceinline__ uint32_t h2_where(uint32_t u, uint32_t h) {
   return u & ((h & 0x7fffu ? 0xffffu : 0u) | (h & 0x7fff0000u ? 0xffff0000u : 0u));
 }
 // Meets the other threads of one group of k_train.
-__device__ __forceinline__ void group_sync(int g) {
-  asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(256) : "memory");
-}
+__device__ __forceinline__ void group_sync(int g) { tc05::bar_sync(g + 1, kGroupThreads); }
 
 // A row whose lobes are split between two threads of a k_train group: the
 // second half's sum goes on from the first half's, in lobe order.
@@ -582,11 +580,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
           }
         first = false;
       }
-      if (!ok) {
-        *failed = 1;
-        tc05::commit(drain);
-        tc05::mbar_wait(drain, 0u);  // bounded: let the MMAs in flight finish
-      }
+      if (!ok) *failed = 1;
     }
     __syncwarp();
   } else {
@@ -702,6 +696,10 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
         tc05::fence_proxy_async();
         tc05::mbar_arrive(ready + grp);
       }
+      // A thread whose wait ran out has gone on without waiting, and arrived
+      // like the others, to the end of the tile. The group leaves together: a
+      // thread that left alone would be missing at the next tile's group_sync.
+      ok = tc05::bar_all(grp + 1, kGroupThreads, ok);
     }
     if (!ok) *failed = 1;
   }
@@ -709,7 +707,17 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
   __syncthreads();
   tc05::fence_after();
   const bool ok = *failed == 0;
-  if (!ok && tid == 0) atomicOr(err, 1);
+  if (!ok) {
+    // whoever gave up did not see the MMAs issued so far end: wait for them
+    // (bounded) before tensor memory is read and freed
+    if (tid == 2 * kGroupThreads) {
+      tc05::commit(drain);
+      tc05::mbar_wait(drain, 0u);
+    }
+    if (tid == 0) atomicOr(err, 1);
+    __syncthreads();
+    tc05::fence_after();
+  }
   // this CTA's partial: weight gradients from TMEM lanes 0..63 (one output
   // unit per lane), the layers split between the warps that read those lanes
   float* mine = part + (size_t)blockIdx.x * kPartStride;

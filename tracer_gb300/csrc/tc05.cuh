@@ -118,6 +118,23 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity, uint3
   return false;
 }
 
+// Meets the other threads that use named barrier `id`, `threads` in all (whole
+// warps). Unbounded: every one of them has to come.
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+// The same, and whether `mine` holds for all of them.
+__device__ __forceinline__ bool bar_all(int id, int threads, bool mine) {
+  uint32_t all;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\tbar.red.and.pred p, %1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(all)
+      : "r"(id), "r"(threads), "r"(mine ? 1u : 0u)
+      : "memory");
+  return all != 0u;
+}
+
 // 32 lanes x 32 consecutive 32-bit columns; the values are there after
 // tmem_wait.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
