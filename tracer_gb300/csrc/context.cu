@@ -1010,6 +1010,7 @@ tr_status tr_scene_set_upload(tr_ctx* ctx, const tr_scene_desc* descs, uint32_t 
   if (!ctx || !descs || n == 0 || n > 65536) return TR_ERR_ARG;
   TR_DEVICE_SCOPE(ctx);
   ctx->has_scene = false;
+  ctx->noalloc_ready = false;
   const bool device_bvh = ctx->bvh_builder == TR_BVH_DEVICE;
   // each scene's tables and tree on its own host thread
   std::vector<HostScene> parts(n);

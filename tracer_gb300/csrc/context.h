@@ -86,6 +86,9 @@ struct tr_ctx {
   cudaStream_t stream = nullptr;
   std::string err;
   bool has_scene = false;
+  // tr_render_dev_noalloc's kernels loaded, and whether the driver has the
+  // local memory of the persistent ones (both since the scene's upload)
+  bool noalloc_ready = false, noalloc_mega = false;
   trg::HostScene hs;
   trg::DScene dsc{};
   trg::DevBuf d_nodes, d_nodes4, d_slots, d_spheres, d_prims, d_tshade, d_mats, d_lights, d_roots;

@@ -2368,6 +2368,41 @@ struct NoAllocLayout {
   }
 };
 
+// What the driver allocates for a kernel it does when the kernel is loaded (its
+// code) or first launched (the local memory of as many threads as can be
+// resident, when that is more than any kernel before it needed): 86 MiB for a
+// process's wavefront kernels, 140 for the persistent kernel in blocks of 256
+// threads and 122 more in blocks of 512 (Cornell box). A context's first call
+// after an upload has all of it allocated at once, by launches over no pixels,
+// so that no later call takes any, whatever its film and path lengths.
+// M.err, M.fetch and M.stats need not be initialised: no lane owns a pixel.
+tr_status noalloc_prepare(tr_ctx* ctx, MegaLaunch M, bool persistent, cudaStream_t st) {
+  for (const void* k :
+       {(const void*)k_init, (const void*)k_extend<false>, (const void*)k_act_order, (const void*)k_logic<false>,
+        (const void*)k_material<MAT_PHONG>, (const void*)k_material<MAT_DISNEY12>, (const void*)k_glass,
+        (const void*)k_material<MAT_METAL>, (const void*)k_material<MAT_DISNEY15>, (const void*)k_nee<MAT_PHONG>,
+        (const void*)k_nee<MAT_DISNEY12>, (const void*)k_nee<MAT_METAL>, (const void*)k_nee<MAT_DISNEY15>,
+        (const void*)k_shadow<false>, (const void*)k_shadow<false, true>}) {
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, k);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaFuncGetAttributes");
+  }
+  M.nslots = 0;
+  ctx->noalloc_mega = persistent;
+  for (int threads : {kMegaFewThreads, kMegaThreads})
+    if (ctx->noalloc_mega) {
+      const cudaError_t e = launch_mega(M, mega_mask(ctx), MegaShape{threads, 32, 1}, st);
+      if (e == cudaErrorMemoryAllocation || e == cudaErrorLaunchOutOfResources) {
+        ctx->noalloc_mega = false;
+        cudaGetLastError();
+      } else if (e != cudaSuccess) {
+        return cuda_fail(ctx, e, "persistent kernel");
+      }
+    }
+  ctx->noalloc_ready = true;
+  return TR_OK;
+}
+
 }  // namespace
 
 tr_status render_noalloc_impl(tr_ctx* ctx, const tr_camera* cam, const tr_filter* filter,
@@ -2484,16 +2519,20 @@ tr_status render_noalloc_impl(tr_ctx* ctx, const tr_camera* cam, const tr_filter
   // delta samples that do not count toward the depth).
   const long long iters =
       (long long)prm->spp * ((long long)prm->max_depth + 2 + (ctx->dsc.has_glass ? kMaxSpecularDepth : 0)) + 4;
+  const MegaShape shape = mega_shape(n, sms);
+  const MegaLaunch M = mega_launch(ctx, P.jobs, 1, n, nl, shape, P.ctr, P.stats);
+  if (!ctx->noalloc_ready) {
+    const tr_status ps = noalloc_prepare(ctx, M, nl <= kMegaLights, st);
+    if (ps != TR_OK) return ps;
+  }
   // Short renders by the persistent kernel, whose state is in registers (two
   // counters and a job record of the array are all it needs): Cornell 125x93x2
-  // 1550 -> 458 us. It cannot stop early, so renders whose longest path chain
+  // 1550 -> 360 us. It cannot stop early, so renders whose longest path chain
   // is more than kNoAllocOneLaunch vertices (tens of milliseconds) keep the
   // wavefront, which looks for tr_cancel between its iterations; so do devices
-  // without the memory to launch it (its local memory per thread is larger).
+  // without the memory to launch it (noalloc_prepare).
   constexpr long long kNoAllocOneLaunch = 256;
-  if (iters <= kNoAllocOneLaunch && nl <= kMegaLights && ctx->tune.render_mode != TR_RENDER_MODE_WAVEFRONT) {
-    const MegaShape shape = mega_shape(n, sms);
-    const MegaLaunch M = mega_launch(ctx, P.jobs, 1, n, nl, shape, P.ctr, P.stats);
+  if (iters <= kNoAllocOneLaunch && ctx->noalloc_mega && ctx->tune.render_mode != TR_RENDER_MODE_WAVEFRONT) {
     NCHK(cudaMemsetAsync(d_rgbw, 0, (size_t)n * 16, st));
     NCHK(cudaMemsetAsync(P.ctr, 0, kCtrWords * 4, st));
     NCHK(cudaMemsetAsync(P.stats, 0, kStatWords * 8, st));
