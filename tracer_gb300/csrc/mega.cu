@@ -271,6 +271,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_mega(MegaLaunch P) {
   bool done = lane >= P.lanes;
   long long steps = 0, max_steps = 0;  // vertex bound of the current pixel
   int oc[kMegaLights];                 // the slot that last blocked each light's shadow ray (-1: none)
+  bool claimed = false;                // a pixel claimed in this iteration: oc is to be cleared
   unsigned long long n_ext = 0, n_sh = 0, n_vert = 0, n_hits = 0;
   // the vertex whose light is being gathered: what its light samples need,
   // its MIS ray, and the sample that ends with it (its film update is due
@@ -307,7 +308,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_mega(MegaLaunch P) {
           const int x = pix % p.J->W, y = pix / p.J->W;
           p.st = Pcg::seed((int)(p.J->seed_base + (unsigned)y * (unsigned)p.J->W + (unsigned)x));
           p.sample = 0;
-          for (int l = 0; l < kMegaLights; ++l) oc[l] = -1;
+          claimed = true;
           steps = 0;
           max_steps = (long long)p.J->spp * ((long long)p.J->max_depth + 2 + ((MASK & MK_GLASS) ? kMaxSpecularDepth : 0));
           p.has_ray = start_sample(p);
@@ -412,20 +413,24 @@ __global__ void __launch_bounds__(THREADS, 1) k_mega(MegaLaunch P) {
         if (!more) __syncthreads();
         // ---- trace (k_extend, k_shadow)
         n_hits += pool_trace(sc, pool, traced, n, P.occluder_cache && sc.slot_leaf, P.err);
-        // (a pixel's last vertex is gathered after the lane has claimed its
-        // next pixel, which may be another scene's: oc is that pixel's by then)
-        const bool remember = !due || due_slot == p.slot;
         for (int e = mine; e < mine + n_mine; ++e) {
           const float4 c = pc[e];
           const int w = __float_as_int(c.w);
-          if (w < 0 || !(w & kBlocked)) direct = direct + mk3(c.x, c.y, c.z);
-          else if (remember) oc[(__float_as_int(pb[e].w) >> 7) & 31] = w & ~kBlocked;
+          if (w >= 0 && (w & kBlocked)) oc[(__float_as_int(pb[e].w) >> 7) & 31] = w & ~kBlocked;
+          else direct = direct + mk3(c.x, c.y, c.z);
         }
         __syncwarp();
         n = traced = front;
         n_mine = 0;
       }
       if (!more) break;
+    }
+
+    // a new pixel, which may be another scene's, starts without occluders; until
+    // here they were those of the pixel before, whose last vertex was gathered
+    if (claimed) {
+      for (int l = 0; l < kMegaLights; ++l) oc[l] = -1;
+      claimed = false;
     }
 
     // ---- finish: the MIS ray's emission, weighted against the light
