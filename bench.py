@@ -763,7 +763,10 @@ def traversal_config(gpus) -> dict:
 
 def launches_of(st) -> int:
     """Kernels one render launched: the persistent kernel's single launch
-    (iterations 1), else k_init and 7 kernels per wavefront iteration."""
+    (iterations 1), else at least k_init and 7 kernels per wavefront iteration
+    (logic, live-slot order, extend, shadow, and a material and a light-sample
+    kernel of each kind, of which these scenes have two in all but one; full
+    iterations also bin the rays, three more)."""
     return 1 if st.iterations == 1 else 1 + 7 * st.iterations
 
 

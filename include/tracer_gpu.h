@@ -456,11 +456,12 @@ typedef struct tr_batch_job {
 tr_status tr_render_batch_dev(tr_ctx* ctx, const tr_batch_job* jobs, uint32_t n, tr_stats* stats);
 /* Launch autotuner. No reference counterpart. Times the batch (each job
  * capped at probe_spp samples per pixel; the jobs' films are overwritten)
- * under candidate tr_tuning settings -- resident traversal blocks per SM,
- * lane-refill threshold, shading grid, CUDA-graph chunk length, any-hit BVH
- * node width -- by coordinate descent (median of three timed renders each, a
- * change kept only if 2% faster), sets the best on the context and returns
- * it with its time. */
+ * under candidate tr_tuning settings -- execution model, resident traversal
+ * blocks per SM, lane-refill threshold, shading grid, CUDA graphs or none,
+ * any-hit BVH node width, ray binning, treelet, occluder cache, any-hit order
+ * -- by coordinate descent (median of three timed renders each, a change kept
+ * only if 2% faster), sets the best on the context and returns it with its
+ * time. */
 tr_status tr_autotune(tr_ctx* ctx, const tr_batch_job* jobs, uint32_t n, int32_t probe_spp,
                       tr_tuning* best, double* best_ms);
 

@@ -26,7 +26,6 @@ struct MegaLaunch {
   DScene sc;
   const JobDev* jobs;
   int njobs, nslots;
-  int nl_max;            // most lights of one job's scene (<= kMegaLights)
   int lanes;             // lanes of a warp that own pixels (1 .. 32)
   DMat* mt;              // sets with image maps: one material set-up per thread of the launch
   int occluder_cache;    // remember each (slot, light)'s last occluder (tr_tuning.occluder_cache)

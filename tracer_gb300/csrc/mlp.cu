@@ -928,7 +928,8 @@ tr_status guide_forward_rows_on_device(tr_ctx* ctx, const float* d_in, const uns
   return e == cudaSuccess ? TR_OK : cuda_fail(ctx, e, "k_forward");
 }
 
-// The row scale of a training pass or step (scal[2]) from the weights w[0..n).
+// The partial sums (scal[16..]) of the weights w[0..n) of a training pass or
+// step, from which its kernels take the row scale (row_scale).
 static tr_status guide_scale(tr_ctx* ctx, const float* w, unsigned int n) {
   float* scal = ctx->guide->scal.as<float>();
   mlp::k_wsum<<<mlp::kWsumParts, 256, 0, ctx->stream>>>(w, n, scal + 16);

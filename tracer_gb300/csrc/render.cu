@@ -24,7 +24,8 @@
 // one code path. All random draws of a vertex happen in `material`, before
 // any of its rays is traced, in the reference's order (its draws never depend
 // on ray results); the contributions are summed back in the reference's
-// order in `logic`. Queues are appended with warp-aggregated atomics.
+// order in `logic`. A block reserves its queue entries with one atomic add per
+// queue (`reserve`).
 
 #include <cuda_runtime.h>
 
@@ -92,7 +93,10 @@ constexpr int kCtrWords = C_BANK + 2 * kBankWords;  // the counter array
 constexpr int kStatWords = 16;
 // render_mode auto: renders of at most this many pixels use the persistent
 // kernel, of scenes with image maps half as many (their set-ups at a hit
-// diverge most). Wavefront / persistent us, 16 samples, at 30,000, 66,000 and
+// diverge most). One line for all scenes, samples and lights, which the
+// crossovers scatter around: at 66,000 pixels the Cornell box would still gain
+// with the persistent kernel, at 30,000 the mapped scene would with the
+// wavefront when it has many samples. Wavefront / persistent us, 16 samples, at 30,000, 66,000 and
 // 128,000 pixels: Cornell box 6640/4010, 7370/5930, 10130/10020; outdoor
 // 9280/7680, 10660/11310, 12170/16430; sphere grid 10250/7470, 12140/11400,
 // 14250/18630; occluded room 30490/20930, 37220/39900, 47870/67860; maps on
@@ -1662,14 +1666,13 @@ static MegaShape mega_shape(int n, int sms) {
   return s;
 }
 
-static MegaLaunch mega_launch(tr_ctx* ctx, const JobDev* jobs, int njobs, int n, int nl, const MegaShape& shape,
+static MegaLaunch mega_launch(tr_ctx* ctx, const JobDev* jobs, int njobs, int n, const MegaShape& shape,
                               unsigned int* ctr, unsigned long long* st) {
   MegaLaunch M;
   M.sc = ctx->dsc;
   M.jobs = jobs;
   M.njobs = njobs;
   M.nslots = n;
-  M.nl_max = nl;
   M.lanes = shape.lanes;
   M.mt = nullptr;
   M.occluder_cache = ctx->tune.occluder_cache;
@@ -1708,7 +1711,7 @@ static tr_status mega_result(tr_ctx* ctx, unsigned int err, const unsigned long 
 // CUDA graph (with graphs enabled); one job's three operations are issued
 // directly. Capturing and instantiating those, creating events and two
 // blocking copies took 65 of a 61x47x1 frame's 796 us.
-static tr_status render_persistent(tr_ctx* ctx, const JobSpec* jobs, int njobs, int n, int nl, int sms,
+static tr_status render_persistent(tr_ctx* ctx, const JobSpec* jobs, int njobs, int n, int sms,
                                    tr_stats* stats) {
   if (!ctx->rb) ctx->rb = new RenderBuffers();
   RenderBuffers* rb = ctx->rb;
@@ -1730,7 +1733,7 @@ static tr_status render_persistent(tr_ctx* ctx, const JobSpec* jobs, int njobs, 
   }
   TR_CUDA(ctx, cudaMemcpyAsync(rb->jobs.p, jd.data(), jd.size() * sizeof(JobDev), cudaMemcpyHostToDevice, st));
   unsigned int* ctr = rb->mega_state.as<unsigned int>();
-  MegaLaunch M = mega_launch(ctx, rb->jobs.as<JobDev>(), njobs, n, nl, shape, ctr,
+  MegaLaunch M = mega_launch(ctx, rb->jobs.as<JobDev>(), njobs, n, shape, ctr,
                              reinterpret_cast<unsigned long long*>(rb->mega_state.as<char>() + kCtrBytes));
   if (ctx->dsc.has_textures) M.mt = rb->MT.as<DMat>();
   ctx->cancel.store(0);
@@ -1797,7 +1800,7 @@ tr_status render_jobs(tr_ctx* ctx, const JobSpec* jobs, int njobs, uint32_t flag
   if (!gp && !(flags & (TR_RENDER_TIME_STAGES | TR_RENDER_COUNT_VISITS)) && nl <= kMegaLights &&
       (ctx->tune.render_mode == TR_RENDER_MODE_PERSISTENT ||
        (ctx->tune.render_mode == TR_RENDER_MODE_AUTO && (long long)n <= kMegaAutoSlots >> (ctx->dsc.has_textures ? 1 : 0))))
-    return render_persistent(ctx, jobs, njobs, n, nl, sms, stats);
+    return render_persistent(ctx, jobs, njobs, n, sms, stats);
   tr_status s = reserve_render(ctx, n, nl);
   if (s != TR_OK) return s;
   RenderBuffers* rb = ctx->rb;
@@ -2520,7 +2523,7 @@ tr_status render_noalloc_impl(tr_ctx* ctx, const tr_camera* cam, const tr_filter
   const long long iters =
       (long long)prm->spp * ((long long)prm->max_depth + 2 + (ctx->dsc.has_glass ? kMaxSpecularDepth : 0)) + 4;
   const MegaShape shape = mega_shape(n, sms);
-  const MegaLaunch M = mega_launch(ctx, P.jobs, 1, n, nl, shape, P.ctr, P.stats);
+  const MegaLaunch M = mega_launch(ctx, P.jobs, 1, n, shape, P.ctr, P.stats);
   if (!ctx->noalloc_ready) {
     const tr_status ps = noalloc_prepare(ctx, M, nl <= kMegaLights, st);
     if (ps != TR_OK) return ps;
@@ -2659,7 +2662,7 @@ extern "C" tr_status tr_autotune(tr_ctx* ctx, const tr_batch_job* jobs, uint32_t
   };
   // coordinate descent over the discrete settings, the execution model first
   static const int kMode[] = {TR_RENDER_MODE_WAVEFRONT, TR_RENDER_MODE_PERSISTENT}, kBlocks[] = {0, 4, 6, 8},
-                   kRefill[] = {12, 20, 28}, kShade[] = {8, 16, 32}, kGraph[] = {0, 4, 8, 16}, kWidth[] = {2, 4},
+                   kRefill[] = {12, 20, 28}, kShade[] = {8, 16, 32}, kGraph[] = {0, 2}, kWidth[] = {2, 4},
                    kBins[] = {0, 3, 4}, kTreelet[] = {0, 64, 256}, kCache[] = {0, 1}, kOrder[] = {0, 1, 2};
   struct Dim {
     int32_t tr_tuning::*field;
@@ -2668,7 +2671,7 @@ extern "C" tr_status tr_autotune(tr_ctx* ctx, const tr_batch_job* jobs, uint32_t
   };
   static const Dim kDims[] = {{&tr_tuning::render_mode, kMode, 2},        {&tr_tuning::trav_blocks_per_sm, kBlocks, 4},
                               {&tr_tuning::trav_refill_lanes, kRefill, 3}, {&tr_tuning::shade_blocks_per_sm, kShade, 3},
-                              {&tr_tuning::graph_iterations, kGraph, 4},   {&tr_tuning::any_node_width, kWidth, 2},
+                              {&tr_tuning::graph_iterations, kGraph, 2},   {&tr_tuning::any_node_width, kWidth, 2},
                               {&tr_tuning::ray_bin_bits, kBins, 3},        {&tr_tuning::treelet_nodes, kTreelet, 3},
                               {&tr_tuning::occluder_cache, kCache, 2},    {&tr_tuning::any_hit_order, kOrder, 3}};
   tr_tuning cur = ctx->tune;
@@ -2681,6 +2684,8 @@ extern "C" tr_status tr_autotune(tr_ctx* ctx, const tr_batch_job* jobs, uint32_t
       for (int k = 0; k < dim.nv; ++k) {
         tr_tuning t = cur;
         if (t.*dim.field == dim.vals[k]) continue;
+        // (any number of graph iterations above zero is the same program)
+        if (dim.field == &tr_tuning::graph_iterations && t.graph_iterations && dim.vals[k]) continue;
         t.*dim.field = dim.vals[k];
         double ms = 0.0;
         s = time_once(t, ms);

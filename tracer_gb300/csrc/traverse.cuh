@@ -326,10 +326,10 @@ __device__ __forceinline__ bool occluded_by_slot(const DScene& sc, int scene, in
 
 // ---------------------------------------------------------------------------
 // Persistent traversal with dynamic fetch. Each lane runs the same per-ray
-// algorithm as Traversal::run (same order, same culling, same tests), cut
+// algorithm as BVHAccel's loops (same order, same culling, same tests), cut
 // into steps so that a warp can keep its lanes busy: interior steps repeat
-// while any lane of the warp is at an interior node, then the lanes at
-// leaves test their primitives; when fewer than `refill` lanes still hold a
+// until fewer than kWalkLanes lanes are without a leaf, then the lanes that
+// have one test its primitives; when fewer than `refill` lanes still hold a
 // ray, the finished lanes take new rays from the work queue (one atomic per
 // warp). Every loop decision is warp-uniform; all 32 lanes stay in the loop
 // until the queue is exhausted, so the kernel must be launched with whole
