@@ -95,7 +95,8 @@ def dram_bound(traffic_per_launch: float, launch_ms: float, peak_gbs: float) -> 
 
 
 def traffic_per_unit(stage: str):
-    """DRAM bytes per work item of a kernel from a committed ncu summary, or None."""
+    """DRAM bytes per work item of a kernel from a committed ncu summary (under
+    "present" those of the kernel as it is now, where it has been captured again), or None."""
     try:
         with open(os.path.join(ROOT, "profiles", "dram_traffic.json")) as f:
             return json.load(f).get(stage)
@@ -886,6 +887,7 @@ def run_ours(args):
                      "units_per_launch": dom_items / max(iters, 1)})
         tr = traffic_per_unit(dom)
         if tr is not None:
+            tr = tr.get("present", tr)  # the capture of the present kernels
             roof["traffic"] = tr["bytes_per_unit"] * dom_items / max(iters, 1)
             roof["traffic_source"] = tr["source"]
             roof.update(dram_bound(roof["traffic"], roof["avg_launch_ms"], peak))
